@@ -6,8 +6,8 @@
 // serving loop cannot spend per request.  Here the levels are related as the tree is: dt halves
 // from one level to the next, so U_l = U_{l+1}^2.  The finest level is a Taylor series of the
 // scaled generator X = K dt / 2^s with ||X||_1 <= 1/4 (degree 14: remainder below 1e-19 of ||e^X||),
-// squared s times; every coarser level is one squaring.  All products are FP64 complex GEMMs in a
-// plain shared-memory tiled kernel (setup work, not the hot path).
+// squared s times; every coarser level is one squaring.  All products are FP64 complex GEMMs on the
+// FP64 tensor core.
 #include <algorithm>
 #include <cmath>
 #include <utility>
@@ -17,67 +17,95 @@
 
 namespace tree {
 
-constexpr int BM = 64, BN = 64, BK = 8, TX = 16;  // 256 threads, 4 x 4 complex outputs each
+constexpr int BM = 32, BN = 32, BK = 8, kStages = 4;   // 256 threads
+constexpr int kAStride = BK + 2, kBStride = BN + 2;    // components; both 32 bytes modulo the banks
 
-// C = A B for n x n complex row-major matrices.
-__global__ void __launch_bounds__(256) zgemm_kernel(int n, const double2 *A, const double2 *B, double2 *C)
+__device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b)
 {
-    __shared__ double2 As[BK][BM];
-    __shared__ double2 Bs[BK][BN];
-    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
+}
+
+// 16 bytes global -> shared, zeros where !valid (the address is not read then).
+__device__ __forceinline__ void cp16(double2 *dst, const double2 *src, bool valid)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+// C = A B for n x n complex row-major matrices, or with div != 0 a Horner step of the Taylor
+// series, C = I + (A B) / div.  FP64 tensor-core MMA, per output the k-ascending chain
+// c.x += a.x b.x; c.x -= a.y b.y; c.y += a.x b.y; c.y += a.y b.x (A = [ar, ai] of two k against
+// B = [br; -bi] and [bi; br]: the MMA's accumulation is that chain, see qjx_kernels.cu), so the
+// results are those of a plain fma loop bit for bit.
+// Bound: the FP64 tensor pipe (8 n^3 flop).  32 x 32 tiles, because n = 256 .. 512 has too few
+// 64 x 64 tiles for 148 SMs (64 at n = 512); a warp owns one 8-row block and two 8-column blocks
+// (four independent chains), and a four-stage cp.async ring of 8 k feeds the CTA.
+__global__ void __launch_bounds__(256) zgemm_kernel(int n, const double2 *A, const double2 *B, double2 *C, double div)
+{
+    __shared__ __align__(16) double2 As[kStages][BM * kAStride];
+    __shared__ __align__(16) double2 Bs[kStages][BK * kBStride];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3, th = t >> 1, todd = t & 1;
     const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
-    double2 acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = make_double2(0.0, 0.0);
-    for (int k0 = 0; k0 < n; k0 += BK) {
-        for (int e = tid; e < BM * BK; e += 256) {
-            const int m = e / BK, k = e % BK, r = row0 + m, kk = k0 + k;
-            As[k][m] = (r < n && kk < n) ? A[(size_t)r * n + kk] : make_double2(0.0, 0.0);
+    const int rb = warp & 3, cb = 2 * (warp >> 2);
+    const int nk = (n + BK - 1) / BK;
+    auto load = [&](int it) {
+        if (it < nk) {
+            double2 *as = As[it % kStages], *bs = Bs[it % kStages];
+            for (int e = tid; e < BM * BK; e += 256) {
+                const int m = e / BK, k = e % BK, r = row0 + m, kk = it * BK + k;
+                const bool v = r < n && kk < n;
+                cp16(as + m * kAStride + k, A + (v ? (size_t)r * n + kk : 0), v);
+            }
+            for (int e = tid; e < BK * BN; e += 256) {
+                const int k = e / BN, c = e % BN, kk = it * BK + k, cc = col0 + c;
+                const bool v = kk < n && cc < n;
+                cp16(bs + k * kBStride + c, B + (v ? (size_t)kk * n + cc : 0), v);
+            }
         }
-        for (int e = tid; e < BK * BN; e += 256) {
-            const int k = e / BN, c = e % BN, kk = k0 + k, cc = col0 + c;
-            Bs[k][c] = (kk < n && cc < n) ? B[(size_t)kk * n + cc] : make_double2(0.0, 0.0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double re[2][2], im[2][2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) re[j][0] = re[j][1] = im[j][0] = im[j][1] = 0.0;
+    for (int i = 0; i < kStages - 1; i++) load(i);
+    for (int it = 0; it < nk; it++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();  // stage `it` has landed for every thread, and nobody reads the one refilled next
+        load(it + kStages - 1);
+        const double *as = reinterpret_cast<const double *>(As[it % kStages] + (8 * rb + g) * kAStride) + t;
+        const double2 *bs = Bs[it % kStages] + th * kBStride + 8 * cb + g;
+#pragma unroll
+        for (int k = 0; k < BK; k += 2) {
+            const double a = as[2 * k];
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const double2 b = bs[k * kBStride + 8 * j];
+                dmma(re[j][0], re[j][1], a, todd ? -b.y : b.x);
+                dmma(im[j][0], im[j][1], a, todd ? b.x : b.y);
+            }
         }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < BK; k++) {
-            double2 a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[k][ty + TX * i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[k][tx + TX * j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    double2 &c = acc[i][j];
-                    c.x = __fma_rn(a[i].x, b[j].x, c.x);
-                    c.x = __fma_rn(-a[i].y, b[j].y, c.x);
-                    c.y = __fma_rn(a[i].x, b[j].y, c.y);
-                    c.y = __fma_rn(a[i].y, b[j].x, c.y);
-                }
-        }
-        __syncthreads();
     }
+    const int r = row0 + 8 * rb + g;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int j = 0; j < 2; j++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int r = row0 + ty + TX * i, c = col0 + tx + TX * j;
-            if (r < n && c < n) C[(size_t)r * n + c] = acc[i][j];
+        for (int i = 0; i < 2; i++) {
+            const int c = col0 + 8 * (cb + j) + 2 * t + i;
+            if (r >= n || c >= n) continue;
+            double2 v = make_double2(re[j][i], im[j][i]);
+            if (div != 0.0) v = make_double2(__dadd_rn(r == c ? 1.0 : 0.0, __ddiv_rn(v.x, div)), __ddiv_rn(v.y, div));
+            C[(size_t)r * n + c] = v;
         }
 }
 
-// T = I + P / k (a Horner step of the Taylor series; P may be T)
-__global__ void horner_kernel(int n, const double2 *P, double k, double2 *T)
+// T = I
+__global__ void identity_kernel(int n, double2 *T)
 {
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)n * n) return;
-    const double2 p = P[e];
-    const bool diag = (e / n) == (e % n);
-    T[e] = make_double2(__dadd_rn(diag ? 1.0 : 0.0, __ddiv_rn(p.x, k)), __ddiv_rn(p.y, k));
+    if (e < (size_t)n * n) T[e] = make_double2((e / n) == (e % n) ? 1.0 : 0.0, 0.0);
 }
 
 // X = s K (complex K, real s)
@@ -88,10 +116,10 @@ __global__ void scale_kernel(int n, const double2 *K, double s, double2 *X)
     X[e] = make_double2(__dmul_rn(K[e].x, s), __dmul_rn(K[e].y, s));
 }
 
-static cudaError_t gemm(int n, const double2 *A, const double2 *B, double2 *C, cudaStream_t st)
+static cudaError_t gemm(int n, const double2 *A, const double2 *B, double2 *C, double div, cudaStream_t st)
 {
     const dim3 grid((n + BN - 1) / BN, (n + BM - 1) / BM);
-    zgemm_kernel<<<grid, 256, 0, st>>>(n, A, B, C);
+    zgemm_kernel<<<grid, 256, 0, st>>>(n, A, B, C, div);
     return cudaGetLastError();
 }
 
@@ -135,20 +163,19 @@ extern "C" qjx_status qjx_expm_tree(int d, int nb, const double *K, const double
         }
         scale_kernel<<<eg, eb, 0, st>>>(d, dK, std::ldexp(dt, -sq), X);
         // Horner: T = I; T = I + X T / k for k = 14 .. 1
-        cudaMemsetAsync(T, 0, bytes, st);
-        horner_kernel<<<eg, eb, 0, st>>>(d, T, 1.0, T);  // T = I
+        identity_kernel<<<eg, eb, 0, st>>>(d, T);
         for (int k = 14; k >= 1; k--) {
-            if (gemm(d, X, T, P, st) != cudaSuccess) status = QJX_ERR_CUDA;
-            horner_kernel<<<eg, eb, 0, st>>>(d, P, (double)k, T);
+            if (gemm(d, X, T, P, (double)k, st) != cudaSuccess) status = QJX_ERR_CUDA;
+            std::swap(T, P);
         }
         for (int i = 0; i < sq; i++) {  // (e^X)^(2^sq)
-            if (gemm(d, T, T, P, st) != cudaSuccess) status = QJX_ERR_CUDA;
+            if (gemm(d, T, T, P, 0.0, st) != cudaSuccess) status = QJX_ERR_CUDA;
             std::swap(T, P);
         }
         // levels deep-1 .. 0: each the square of the next finer one
         for (int l = deep - 1; l >= 0 && status == QJX_OK; l--) {
             if (l < deep - 1) {
-                if (gemm(d, T, T, P, st) != cudaSuccess) status = QJX_ERR_CUDA;
+                if (gemm(d, T, T, P, 0.0, st) != cudaSuccess) status = QJX_ERR_CUDA;
                 std::swap(T, P);
             }
             if (cudaMemcpyAsync(Utree + 2 * dd * ((size_t)b * deep + l), T, bytes, cudaMemcpyDeviceToHost, st) !=
