@@ -2,9 +2,9 @@
 //
 // The reference integrates dx/dt = Gs x + E(t) Qs_drv x - Ks with classic RK4
 // (source/cpp/CQdiss_os_dimer/CQdiss/calcODE.cpp:75-118 calcVectValue_real, :249-389
-// calcODE_trans/std), two mkl_dcsrgemv per stage.  Two GPU paths:
-//   * rk4_cluster: one thread-block cluster holds the whole system in distributed shared memory
-//     and integrates a period per launch (systems that fit <= 16 CTAs);
+// calcODE_trans/std), two mkl_dcsrgemv per stage.  GPU paths:
+//   * resident forms, one launch per period: rk4_cluster holds the whole system in the shared memory
+//     of one thread-block cluster, rk4_grid spreads a larger one over every SM;
 //   * rk_stage: one launch per RK stage (four per step) computes both CSR row products, the
 //     stage vector k = (Gs x + drv Qs x - Ks) h and the next stage argument, or in stage 4 the
 //     RK4 update of x.  The stage arguments are double-buffered (stage s reads one buffer and
@@ -16,9 +16,11 @@
 // combined by an xor butterfly (offsets 16, 8, 4, 2, 1).  All other arithmetic is literal
 // (-fmad=false).  The drive uses sin() of the stage time (CUDA libdevice), so drv_type 1
 // matches the CPU within rounding, not bit-for-bit.
-#include <cooperative_groups.h>
+#include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -114,148 +116,350 @@ static cudaError_t queue_rk_stages(const FbParams &P, double T, int num_steps, i
     return cudaSuccess;
 }
 
-// ---------------------------------------------------------------- cluster-resident RK4
-// One thread-block cluster integrates the whole system: CTA r owns rows [row_lo[r], row_lo[r+1])
-// and keeps their CSR slices of Gs and Qs_drv in shared memory (the cluster's distributed shared
-// memory holds the whole Liouvillian), plus full copies of x and of the two stage arguments.
-// Each stage computes the owned rows and stores the next stage argument into every CTA of the
-// cluster (DSMEM); a hardware cluster barrier separates the stages, four per RK4 step, and no
-// kernel launch happens inside a period.  Rows are computed thread-per-row with the canonical
-// 32-lane order (lane partial sums over nonzeros l, l+32, ..., then the butterfly tree), so the
-// results equal the warp-per-row kernel bit for bit.
-struct FbClusterParams {
+// ---------------------------------------------------------------- resident RK4
+// Both resident forms keep each CTA's rows in shared memory for a whole launch (a period).  Short rows
+// (at most kW nonzeros and one of the drive, all but about N of the dimer's N^2) are held thread-per-row, nonzero l of
+// consecutive rows side by side (no bank conflicts), padded with a zero value and a column that holds
+// zero; long rows are done by a warp each.  Thread-per-row keeps the canonical order (lane partial
+// sums over nonzeros l, l + 32, ..., then the butterfly tree): with at most kW <= 32 nonzeros each
+// lane holds one product, and a level of the tree that pairs a product with an absent lane's +0.0
+// changes nothing but a -0 into +0, which one addition at the end does for all.
+constexpr int kW = 20;
+constexpr long long kFbWait = 1ll << 24;  // polls of a wait before it gives up
+
+// Rows of one CTA: S short rows, then L long ones; row i of the CTA is entry base + i of the vectors.
+struct FbRows {
+    int base, S, L, ln;  // first entry, short rows, long rows, their nonzeros
+};
+
+struct FbResParams {
     int n;
-    const int *row_lo;  // [cluster size + 1]
-    const int *gr, *gc;
-    const double *gv;
-    const int *qr, *qc;
-    const double *qv;
-    const double *Ks;
+    const FbRows *rows;                      // [CTAs]
+    const double *ev;                        // short rows: [kW][RS] values per CTA (RS = maxS)
+    const unsigned short *ec16;              // and columns (entry numbers; n: the zero)
+    const int *ec32;                         // the same for the grid form
+    const double *lv;                        // long rows: nonzeros, each row's of Gs, then of Qs
+    const int *lc, *lp;                      // columns, starts [CTA][2 maxL + 1]: Gs of row j at 2 j, Qs at 2 j + 1
+    const double *ks, *qv;                   // per entry: constant term; short rows: drive value (0: none)
+    const int *qc;                           // and column (n: none)
+    const int *perm;                         // entry -> row of the caller's vectors
     double *x;
+    double *buf;                             // grid form: two arguments [2][n + 1]
+    unsigned *arrived;                       // grid form: CTAs that have passed a stage
+    int *fail;                               // a wait that gave up
+    int maxS, maxL, maxN;                    // strides of the per-CTA arrays
     double drv_ampl, drv_freq, drv_phase;
     int drv_type;
     double T, h;
-    int num_steps, period0, n_periods;
-    int max_rows, max_gnz, max_qnz;
+    int num_steps, period;
 };
 
-__device__ __forceinline__ double row_sum_lanes(const int *rp, const int *col, const double *val, const double *arg,
-                                                int r)
+__device__ __forceinline__ double short_row(const double *val, int stride, const double (&x)[kW])
 {
-    const int b = rp[r], e = rp[r + 1];
-    // A row with at most one nonzero (every row of the drive matrix Qs, so warps do not diverge
-    // here): lane 0 holds fma(v, a, 0) and the tree adds only +0.0 to it, which leaves every value
-    // but -0 unchanged and turns -0 into +0, i.e. the result is p0 + 0.0.
-    if (e - b <= 1) return e > b ? __dadd_rn(__fma_rn(val[b], arg[col[b]], 0.0), 0.0) : 0.0;
-    double p[32];
+    double p[kW];
 #pragma unroll
-    for (int l = 0; l < 32; l++) p[l] = 0.0;
-    for (int base = b; base < e; base += 32) {
-#pragma unroll
-        for (int l = 0; l < 32; l++) {
-            const int j = base + l;
-            if (j < e) p[l] = __fma_rn(val[j], arg[col[j]], p[l]);
-        }
-    }
+    for (int l = 0; l < kW; l++) p[l] = __fma_rn(val[l * stride], x[l], 0.0);
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1)
 #pragma unroll
-        for (int l = 0; l < off; l++) p[l] = __dadd_rn(p[l], p[l + off]);
-    return p[0];
+        for (int l = 0; l < off; l++)
+            if (l + off < kW && (off == 16 || l + off < 2 * off)) p[l] = __dadd_rn(p[l], p[l + off]);
+    return __dadd_rn(p[0], 0.0);
 }
 
-constexpr int kMaxCluster = 16;
-
-__global__ void __launch_bounds__(512, 1) rk4_cluster(const FbClusterParams P)
+// Row sum of a long row by a warp (the canonical order itself).
+template <class Load>
+__device__ __forceinline__ double long_row(const double *v, const int *c, int b, int e, int lane, const Load &arg)
 {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank(), cs = (int)cl.num_blocks();
+    double s = 0.0;
+    for (int j = b + lane; j < e; j += 32) s = __fma_rn(v[j], arg(c[j]), s);
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
+    return s;
+}
+
+// drv of stage 1 (j = 0), 2 and 3 (j = 1) or 4 (j = 2) of step s (calcODE.cpp:84-94, 278-302)
+__device__ __forceinline__ double stage_drive(const FbResParams &P, int s, int j)
+{
+    const double t = __dadd_rn(__dmul_rn((double)P.period, P.T), __dmul_rn((double)s, P.h));
+    const double tt = j == 0 ? t : (j == 2 ? __dadd_rn(t, P.h) : __dadd_rn(t, __ddiv_rn(P.h, 2.0)));
+    const double sn = sin(__dadd_rn(__dmul_rn(P.drv_freq, tt), P.drv_phase));
+    return P.drv_type == 1 ? __dmul_rn(P.drv_ampl, sn) : __dmul_rn(P.drv_ampl, (sn < 0.0) ? -1.0 : 1.0);
+}
+
+// Shared memory of a CTA's rows (both forms): per-row vectors, short-row values, long-row values, then
+// the integers.
+struct FbSmem {
+    double *x, *k1, *k2, *k3, *ks, *qv, *ev, *lv, *drv;
+    int *qc, *lc, *lp;
+};
+
+__host__ __device__ inline size_t fb_rows_bytes(int maxS, int maxL, int maxN)
+{
+    return sizeof(double) * (6 * (size_t)(maxS + maxL) + (size_t)kW * maxS + maxN + 6) +
+           sizeof(int) * ((size_t)(maxS + maxL) + maxN + 2 * (size_t)maxL + 2);
+}
+
+__device__ __forceinline__ FbSmem fb_carve(const FbResParams &P, unsigned char *smem)
+{
+    FbSmem m;
+    const int R = P.maxS + P.maxL;
+    m.x = reinterpret_cast<double *>(smem);
+    m.k1 = m.x + R;
+    m.k2 = m.k1 + R;
+    m.k3 = m.k2 + R;
+    m.ks = m.k3 + R;
+    m.qv = m.ks + R;
+    m.ev = m.qv + R;
+    m.lv = m.ev + (size_t)kW * P.maxS;
+    m.drv = m.lv + P.maxN;  // [2][3]
+    m.qc = reinterpret_cast<int *>(m.drv + 6);
+    m.lc = m.qc + R;
+    m.lp = m.lc + P.maxN;
+    return m;
+}
+
+// Loads a CTA's rows and the first step's drive (CTA-wide; the caller synchronises).
+__device__ __forceinline__ void fb_load_rows(const FbResParams &P, int cta, const FbRows &r, const FbSmem &m)
+{
+    const int tid = threadIdx.x, nt = blockDim.x;
+    for (int i = tid; i < r.S + r.L; i += nt) {
+        m.x[i] = P.x[P.perm[r.base + i]];
+        m.ks[i] = P.ks[r.base + i];
+        m.qv[i] = P.qv[r.base + i];
+        m.qc[i] = P.qc[r.base + i];
+    }
+    for (int i = tid; i < kW * P.maxS; i += nt) m.ev[i] = P.ev[(size_t)cta * kW * P.maxS + i];
+    for (int i = tid; i < r.ln; i += nt) {
+        m.lv[i] = P.lv[(size_t)cta * P.maxN + i];
+        m.lc[i] = P.lc[(size_t)cta * P.maxN + i];
+    }
+    for (int i = tid; i <= 2 * r.L; i += nt) m.lp[i] = P.lp[(size_t)cta * (2 * P.maxL + 1) + i];
+    if (tid < 3) m.drv[tid] = stage_drive(P, 0, tid);
+}
+
+// Row i of a stage from its two row sums: k = (Gs x + drv Qs x - Ks) h and the entry of the next
+// stage's argument, or in stage 4 of the new x (calcODE.cpp:95-117, 278-302).
+__device__ __forceinline__ double fb_finish(const FbResParams &P, const FbSmem &m, int stage, int i, double t1, double t2,
+                                            double drv)
+{
+    const double k = __dmul_rn(__dsub_rn(__dadd_rn(t1, __dmul_rn(drv, t2)), m.ks[i]), P.h);
+    const double x = m.x[i];
+    if (stage == 1) {
+        m.k1[i] = k;
+        return __dadd_rn(x, __ddiv_rn(k, 2.0));
+    }
+    if (stage == 2) {
+        m.k2[i] = k;
+        return __dadd_rn(x, __ddiv_rn(k, 2.0));
+    }
+    if (stage == 3) {
+        m.k3[i] = k;
+        return __dadd_rn(x, k);
+    }
+    const double sum = __dadd_rn(__dadd_rn(__dadd_rn(m.k1[i], __dmul_rn(2.0, m.k2[i])), __dmul_rn(2.0, m.k3[i])), k);
+    const double v = __dadd_rn(x, __ddiv_rn(sum, 6.0));
+    m.x[i] = v;
+    return v;
+}
+
+// ---- cluster form: the whole system in the shared memory of one cluster of at most 16 CTAs
+constexpr int kMaxCluster = 16, kClusterThreads = 512, kClusterRows = 192;
+
+__device__ __forceinline__ uint32_t fb_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ uint32_t fb_map(uint32_t addr, int rank)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
+
+__device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity)
+{
+    for (long long i = 0; i < kFbWait; i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// Every CTA holds full copies of two arguments, used in turn; a stage's entries are stored into every
+// CTA with st.async, whose bytes complete the receiver's mbarrier of that stage: a CTA goes on when
+// all n entries have arrived, with no cluster barrier (two round trips) and no wait for stores to be
+// acknowledged.  Two mbarriers and two arguments are enough: a CTA can send entries of stage s + 1
+// only after it has all of stage s, so after every CTA has finished reading the argument of stage s
+// (the one that stage s + 1 overwrites is that of stage s - 1).  One warp works out the next step's
+// drive values meanwhile.  Bound: the latency of a stage (gather, row sum, st.async, mbarrier), about
+// 0.5 us.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread its own
+// sine): 2.9 us a stage at N = 50.
+__global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResParams P, int cs)
+{
     extern __shared__ __align__(16) unsigned char fsm[];
-    const int n = P.n, tid = threadIdx.x, nt = blockDim.x;
-    double *xf = reinterpret_cast<double *>(fsm);
-    double *va = xf + n;
-    double *vb = va + n;
-    double *k1 = vb + n;
-    double *k2 = k1 + P.max_rows;
-    double *k3 = k2 + P.max_rows;
-    double *ks = k3 + P.max_rows;
-    double *gval = ks + P.max_rows;
-    double *qval = gval + P.max_gnz;
-    int *grp = reinterpret_cast<int *>(qval + P.max_qnz);
-    int *qrp = grp + P.max_rows + 1;
-    int *gcol = qrp + P.max_rows + 1;
-    int *qcol = gcol + P.max_gnz;
-    const int r0 = P.row_lo[rank], nr = P.row_lo[rank + 1] - r0;
-    const int gb = P.gr[r0], qb = P.qr[r0];
-    for (int i = tid; i < n; i += nt) xf[i] = P.x[i];
-    for (int i = tid; i <= nr; i += nt) {
-        grp[i] = P.gr[r0 + i] - gb;
-        qrp[i] = P.qr[r0 + i] - qb;
+    __shared__ __align__(8) uint64_t bar[2];
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const int n = P.n;
+    int rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    double *buf = reinterpret_cast<double *>(fsm);  // [2][n + 1]
+    const FbSmem m = fb_carve(P, fsm + sizeof(double) * 2 * (size_t)(n + 1));
+    unsigned short *ec = reinterpret_cast<unsigned short *>(m.lp + 2 * P.maxL + 2);  // [kW][maxS]
+    const FbRows r = P.rows[rank];
+    fb_load_rows(P, rank, r, m);
+    for (int i = tid; i < kW * P.maxS; i += nt) ec[i] = P.ec16[(size_t)rank * kW * P.maxS + i];
+    for (int i = tid; i <= n; i += nt) {
+        buf[i] = i < n ? P.x[P.perm[i]] : 0.0;
+        if (i == n) buf[n + 1 + n] = 0.0;
     }
-    for (int j = tid; j < P.gr[r0 + nr] - gb; j += nt) {
-        gval[j] = P.gv[gb + j];
-        gcol[j] = P.gc[gb + j];
+    const uint32_t bar0 = fb_smem_u32(bar);
+    if (tid == 0) {
+        for (int q = 0; q < 2; q++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(bar0 + 8 * q) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int j = tid; j < P.qr[r0 + nr] - qb; j += nt) {
-        qval[j] = P.qv[qb + j];
-        qcol[j] = P.qc[qb + j];
-    }
-    for (int i = tid; i < nr; i += nt) ks[i] = P.Ks[r0 + i];
-    cl.sync();
-    const double h = P.h;
-    for (int p = P.period0; p < P.period0 + P.n_periods; p++) {
-        for (int s = 0; s < P.num_steps; s++) {
-            const double t = __dadd_rn(__dmul_rn((double)p, P.T), __dmul_rn((double)s, h));
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    bool ok = true;
+    uint32_t it = 0;  // stages done
+    for (int s = 0; s < P.num_steps; s++) {
 #pragma unroll 1
-            for (int stage = 1; stage <= 4; stage++) {
-                const double *arg = (stage == 1) ? xf : ((stage == 3) ? vb : va);
-                const double tt =
-                    (stage == 1) ? t : ((stage == 4) ? __dadd_rn(t, h) : __dadd_rn(t, __ddiv_rn(h, 2.0)));
-                const double sn = sin(__dadd_rn(__dmul_rn(P.drv_freq, tt), P.drv_phase));
-                const double drv = (P.drv_type == 1) ? __dmul_rn(P.drv_ampl, sn)
-                                                     : __dmul_rn(P.drv_ampl, (sn < 0.0) ? -1.0 : 1.0);
-                for (int i = tid; i < nr; i += nt) {
-                    const double t1 = row_sum_lanes(grp, gcol, gval, arg, i);
-                    const double t2 = row_sum_lanes(qrp, qcol, qval, arg, i);
-                    const double k = __dmul_rn(__dsub_rn(__dadd_rn(t1, __dmul_rn(drv, t2)), ks[i]), h);
-                    const int row = r0 + i;
-                    const double x = xf[row];
-                    if (stage == 1) {
-                        k1[i] = k;
-                        const double v = __dadd_rn(x, __ddiv_rn(k, 2.0));
-                        for (int r = 0; r < cs; r++) *cl.map_shared_rank(va + row, r) = v;
-                    } else if (stage == 2) {
-                        k2[i] = k;
-                        const double v = __dadd_rn(x, __ddiv_rn(k, 2.0));
-                        for (int r = 0; r < cs; r++) *cl.map_shared_rank(vb + row, r) = v;
-                    } else if (stage == 3) {
-                        k3[i] = k;
-                        const double v = __dadd_rn(x, k);
-                        for (int r = 0; r < cs; r++) *cl.map_shared_rank(va + row, r) = v;
-                    } else {
-                        const double sum =
-                            __dadd_rn(__dadd_rn(__dadd_rn(k1[i], __dmul_rn(2.0, k2[i])), __dmul_rn(2.0, k3[i])), k);
-                        const double xn = __dadd_rn(x, __ddiv_rn(sum, 6.0));
-                        for (int r = 0; r < cs; r++) *cl.map_shared_rank(xf + row, r) = xn;
-                    }
-                }
-                cl.sync();
+        for (int stage = 1; stage <= 4; stage++, it++) {
+            const double *arg = buf + (it & 1) * (size_t)(n + 1);
+            const uint32_t out = fb_smem_u32(buf + ((it & 1) ^ 1) * (size_t)(n + 1) + r.base);
+            const uint32_t mb = bar0 + 8 * (it & 1);
+            const double drv = m.drv[3 * (s & 1) + (stage == 1 ? 0 : (stage == 4 ? 2 : 1))];
+            auto send = [&](int i, double v) {
+                for (int c = 0; c < cs; c++)
+                    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                                     fb_map(out + 8 * i, c)),
+                                 "l"(__double_as_longlong(v)), "r"(fb_map(mb, c))
+                                 : "memory");
+            };
+            auto drive_sum = [&](int i) { return __dadd_rn(__fma_rn(m.qv[i], arg[m.qc[i]], 0.0), 0.0); };
+            for (int i = tid; i < r.S; i += nt) {
+                double x[kW];
+#pragma unroll
+                for (int l = 0; l < kW; l++) x[l] = arg[ec[l * P.maxS + i]];
+                const double t1 = short_row(m.ev + i, P.maxS, x);
+                send(i, fb_finish(P, m, stage, i, t1, drive_sum(i), drv));
+            }
+            for (int j = nw - 1 - warp; j < r.L; j += nw) {
+                const int i = r.S + j;
+                const auto load = [&](int c) { return arg[c]; };
+                const double t1 = long_row(m.lv, m.lc, m.lp[2 * j], m.lp[2 * j + 1], lane, load);
+                const double t2 = long_row(m.lv, m.lc, m.lp[2 * j + 1], m.lp[2 * j + 2], lane, load);
+                if (lane == 0) send(i, fb_finish(P, m, stage, i, t1, t2, drv));
+            }
+            if (warp == nw - 1) {
+                if (stage == 1 && lane < 3) m.drv[3 * ((s + 1) & 1) + lane] = stage_drive(P, s + 1, lane);
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mb) : "memory");
+            }
+            if (tid == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(8 * n) : "memory");
+            if (ok && !fb_wait(mb, (it >> 1) & 1)) {  // (every CTA then runs on without waiting, to the end)
+                ok = false;
+                atomicExch(P.fail, 1);
             }
         }
     }
-    for (int i = tid; i < nr; i += nt) P.x[r0 + i] = xf[r0 + i];
+    for (int i = tid; i < r.S + r.L; i += nt) P.x[P.perm[r.base + i]] = m.x[i];
+    // no CTA leaves while another's stores into it may be on their way
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// ---- grid form: systems too large for a cluster, on every SM
+// The rows of the system over all CTAs of one cooperative launch, the two arguments in global memory
+// (L2), a bounded grid barrier per stage.  Bound: the latency of a stage (L2 gather, row sum, barrier),
+// about 1.5 us; one launch per stage before this took 8 us.
+constexpr int kGridThreads = 256;
+
+__global__ void __launch_bounds__(kGridThreads, 1) rk4_grid(const FbResParams P)
+{
+    extern __shared__ __align__(16) unsigned char fsm[];
+    __shared__ int s_ok;
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const int n = P.n, cta = blockIdx.x;
+    const FbSmem m = fb_carve(P, fsm);
+    int *ec = m.lp + 2 * P.maxL + 2;  // [kW][maxS]
+    const FbRows r = P.rows[cta];
+    fb_load_rows(P, cta, r, m);
+    for (int i = tid; i < kW * P.maxS; i += nt) ec[i] = P.ec32[(size_t)cta * kW * P.maxS + i];
+    if (tid == 0) s_ok = 1;
+    __syncthreads();
+    uint32_t it = 0;  // barriers passed
+    auto sync = [&] {
+        __syncthreads();
+        it++;
+        if (tid == 0) {
+            __threadfence();
+            atomicAdd(P.arrived, 1u);
+            const unsigned want = it * gridDim.x;
+            long long i = 0;
+            unsigned v;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.arrived) : "memory");
+            } while ((int)(v - want) < 0 && ++i < kFbWait);
+            if ((int)(v - want) < 0) {
+                s_ok = 0;
+                atomicExch(P.fail, 1);
+            }
+            __threadfence();
+        }
+        __syncthreads();
+        return s_ok != 0;
+    };
+    for (int i = tid; i < r.S + r.L; i += nt) __stcg(P.buf + r.base + i, m.x[i]);
+    if (cta == 0 && tid < 2) __stcg(P.buf + tid * (size_t)(n + 1) + n, 0.0);
+    bool ok = sync();
+    uint32_t q = 0;  // argument in use
+    for (int s = 0; s < P.num_steps && ok; s++) {
+#pragma unroll 1
+        for (int stage = 1; stage <= 4 && ok; stage++) {
+            const double *arg = P.buf + q * (size_t)(n + 1);
+            double *out = P.buf + (q ^ 1) * (size_t)(n + 1) + r.base;
+            const double drv = m.drv[3 * (s & 1) + (stage == 1 ? 0 : (stage == 4 ? 2 : 1))];
+            auto drive_sum = [&](int i) { return __dadd_rn(__fma_rn(m.qv[i], __ldcg(arg + m.qc[i]), 0.0), 0.0); };
+            for (int i = tid; i < r.S; i += nt) {
+                double x[kW];
+#pragma unroll
+                for (int l = 0; l < kW; l++) x[l] = __ldcg(arg + ec[l * P.maxS + i]);
+                const double t2 = drive_sum(i);
+                const double t1 = short_row(m.ev + i, P.maxS, x);
+                __stcg(out + i, fb_finish(P, m, stage, i, t1, t2, drv));
+            }
+            for (int j = nw - 1 - warp; j < r.L; j += nw) {
+                const int i = r.S + j;
+                const auto load = [&](int c) { return __ldcg(arg + c); };
+                const double t1 = long_row(m.lv, m.lc, m.lp[2 * j], m.lp[2 * j + 1], lane, load);
+                const double t2 = long_row(m.lv, m.lc, m.lp[2 * j + 1], m.lp[2 * j + 2], lane, load);
+                if (lane == 0) __stcg(out + i, fb_finish(P, m, stage, i, t1, t2, drv));
+            }
+            if (stage == 1 && warp == nw - 1 && lane < 3) m.drv[3 * ((s + 1) & 1) + lane] = stage_drive(P, s + 1, lane);
+            q ^= 1;
+            ok = sync();
+        }
+    }
+    if (ok)
+        for (int i = tid; i < r.S + r.L; i += nt) P.x[P.perm[r.base + i]] = m.x[i];
 }
 
 }  // namespace fb
 
 struct qjx_fb {
     fb::FbParams P{};
-    // cluster-resident path (used when the system fits the shared memory of <= 16 CTAs)
-    bool cluster = false;
-    int cs = 0;
-    size_t csmem = 0;
-    fb::FbClusterParams CP{};
+    // resident forms: cs CTAs of one cluster, or `grid` CTAs of a cooperative launch (neither: stage kernels)
+    int cs = 0, grid = 0;
+    size_t smem = 0;
+    fb::FbResParams R{};
+    int *h_fail = nullptr;  // pinned
     int device = 0;
     double T = 0.0;
     int num_steps = 0;
@@ -271,6 +475,214 @@ static void *fb_alloc(qjx_fb *h, size_t bytes)
     if (cudaMalloc(&p, bytes ? bytes : 16) != cudaSuccess) return nullptr;
     h->allocs.push_back(p);
     return p;
+}
+
+// The caller's system (host CSR).
+struct FbSystem {
+    int n;
+    const int *gr, *gc;
+    const double *gv;
+    const int *qr, *qc;
+    const double *qv;
+    const double *ks;
+};
+
+template <class V>
+static V *fb_upload(qjx_fb *h, const std::vector<V> &v)
+{
+    V *p = (V *)fb_alloc(h, v.size() * sizeof(V));
+    if (p && !v.empty() && cudaMemcpy(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
+    return p;
+}
+
+// The rows dealt to `nc` CTAs and their shared-memory form: the rows of each nonzero count, in their
+// natural order (neighbours read neighbouring columns), cut into nc equal runs, so every CTA gets the
+// same mix.  Entries of the vectors are numbered CTA after CTA, short rows first.
+struct FbDeal {
+    std::vector<fb::FbRows> rows;
+    std::vector<int> perm, pos;  // entry -> row, row -> entry
+    int maxS = 0, maxL = 0, maxN = 0;
+};
+
+static void fb_deal(const FbSystem &y, int nc, FbDeal &d)
+{
+    const int n = y.n;
+    std::vector<int> order(n);
+    for (int i = 0; i < n; i++) order[i] = i;
+    // a row's nonzeros; past kW (long) also when its drive has several
+    auto nnz = [&](int i) {
+        const int g = y.gr[i + 1] - y.gr[i], q = y.qr[i + 1] - y.qr[i];
+        return q > 1 ? fb::kW + 1 + g + q : g;
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return nnz(a) < nnz(b); });
+    std::vector<std::vector<int>> mine(nc);
+    int turn = 0;  // where the remainders of a count go next
+    for (int i = 0; i < n;) {
+        int j = i;
+        while (j < n && nnz(order[j]) == nnz(order[i])) j++;
+        const int per = (j - i) / nc;
+        for (int c = 0; c < nc; c++) mine[c].insert(mine[c].end(), order.begin() + i + c * per, order.begin() + i + (c + 1) * per);
+        for (int k = i + nc * per; k < j; k++, turn++) mine[turn % nc].push_back(order[k]);
+        i = j;
+    }
+    d = FbDeal();
+    d.perm.reserve(n);
+    d.pos.assign(n, 0);
+    for (int c = 0; c < nc; c++) {
+        fb::FbRows r{(int)d.perm.size(), 0, 0, 0};
+        for (int i : mine[c]) {  // ascending counts: the long rows are last
+            if (nnz(i) <= fb::kW) {
+                r.S++;
+            } else {
+                r.L++;
+                r.ln += y.gr[i + 1] - y.gr[i] + y.qr[i + 1] - y.qr[i];
+            }
+            d.pos[i] = (int)d.perm.size();
+            d.perm.push_back(i);
+        }
+        d.rows.push_back(r);
+        d.maxS = std::max(d.maxS, r.S);
+        d.maxL = std::max(d.maxL, r.L);
+        d.maxN = std::max(d.maxN, r.ln);
+    }
+    d.maxS = std::max(32, (d.maxS + 31) & ~31);
+}
+
+static bool fb_upload_deal(qjx_fb *h, const FbSystem &y, const FbDeal &d, bool cluster)
+{
+    const int n = y.n, nc = (int)d.rows.size();
+    std::vector<double> ev((size_t)nc * fb::kW * d.maxS, 0.0), lv((size_t)nc * std::max(1, d.maxN), 0.0), ks(n), qv(n, 0.0);
+    std::vector<int> ec(ev.size(), n), lc(lv.size(), 0), lp((size_t)nc * (2 * d.maxL + 1), 0), qc(n, n);
+    for (int c = 0; c < nc; c++) {
+        const fb::FbRows &r = d.rows[c];
+        int at = 0;
+        for (int i = 0; i < r.S + r.L; i++) {
+            const int row = d.perm[r.base + i], b = y.gr[row], len = y.gr[row + 1] - b;
+            ks[r.base + i] = y.ks[row];
+            if (i < r.S) {
+                for (int l = 0; l < len; l++) {
+                    const size_t e = ((size_t)c * fb::kW + l) * d.maxS + i;
+                    ev[e] = y.gv[b + l];
+                    ec[e] = d.pos[y.gc[b + l]];
+                }
+                if (y.qr[row + 1] > y.qr[row]) {
+                    qv[r.base + i] = y.qv[y.qr[row]];
+                    qc[r.base + i] = d.pos[y.qc[y.qr[row]]];
+                }
+            } else {
+                auto put = [&](double v, int col) {
+                    lv[(size_t)c * d.maxN + at] = v;
+                    lc[(size_t)c * d.maxN + at++] = d.pos[col];
+                };
+                int *start = lp.data() + (size_t)c * (2 * d.maxL + 1) + 2 * (i - r.S);
+                for (int l = 0; l < len; l++) put(y.gv[b + l], y.gc[b + l]);
+                start[1] = at;
+                for (int l = y.qr[row]; l < y.qr[row + 1]; l++) put(y.qv[l], y.qc[l]);
+                start[2] = at;
+            }
+        }
+    }
+    fb::FbResParams &R = h->R;
+    R.n = n;
+    R.rows = fb_upload(h, d.rows);
+    R.ev = fb_upload(h, ev);
+    if (cluster) R.ec16 = fb_upload(h, std::vector<unsigned short>(ec.begin(), ec.end()));
+    else R.ec32 = fb_upload(h, ec);
+    R.lv = fb_upload(h, lv);
+    R.lc = fb_upload(h, lc);
+    R.lp = fb_upload(h, lp);
+    R.ks = fb_upload(h, ks);
+    R.qv = fb_upload(h, qv);
+    R.qc = fb_upload(h, qc);
+    R.perm = fb_upload(h, d.perm);
+    R.x = h->P.x;
+    R.fail = (int *)fb_alloc(h, sizeof(int));
+    if (!R.rows || !R.ev || !(cluster ? (const void *)R.ec16 : R.ec32) || !R.lv || !R.lc || !R.lp || !R.ks || !R.qv || !R.qc ||
+        !R.perm || !R.fail || cudaMemset(R.fail, 0, sizeof(int)) != cudaSuccess ||
+        (!h->h_fail && cudaMallocHost(&h->h_fail, sizeof(int)) != cudaSuccess))
+        return false;
+    *h->h_fail = 0;
+    R.maxS = d.maxS;
+    R.maxL = d.maxL;
+    R.maxN = d.maxN;
+    R.drv_ampl = h->P.drv_ampl;
+    R.drv_freq = h->P.drv_freq;
+    R.drv_phase = h->P.drv_phase;
+    R.drv_type = h->P.drv_type;
+    R.T = h->T;
+    R.h = h->T / double(h->num_steps);
+    R.num_steps = h->num_steps;
+    return true;
+}
+
+// The cluster form: the smallest cluster (a power of two up to 16) with at most kClusterRows rows a
+// CTA, or 16, when its shared memory holds the system.
+static bool fb_setup_cluster(qjx_fb *h, const FbSystem &y)
+{
+    if (y.n >= 65535) return false;  // 16-bit columns
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
+    int cs = 1;
+    while (cs < fb::kMaxCluster && (y.n + cs - 1) / cs > fb::kClusterRows) cs *= 2;
+    for (; cs <= fb::kMaxCluster; cs *= 2) {
+        FbDeal d;
+        fb_deal(y, cs, d);
+        const size_t bytes = sizeof(double) * 2 * ((size_t)y.n + 1) + fb::fb_rows_bytes(d.maxS, d.maxL, d.maxN) +
+                             sizeof(unsigned short) * fb::kW * d.maxS + 16;
+        if (bytes + 1024 > (size_t)optin) continue;
+        if (cudaFuncSetAttribute(fb::rk4_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+            (cs > 8 && cudaFuncSetAttribute(fb::rk4_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+            cudaGetLastError();
+            continue;
+        }
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3(cs);
+        lc.blockDim = dim3(fb::kClusterThreads);
+        lc.dynamicSmemBytes = bytes;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cs;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        lc.attrs = at;
+        lc.numAttrs = 1;
+        int nclusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&nclusters, fb::rk4_cluster, &lc) != cudaSuccess || nclusters < 1) {
+            cudaGetLastError();
+            continue;
+        }
+        if (!fb_upload_deal(h, y, d, true)) return false;
+        h->cs = cs;
+        h->smem = bytes;
+        return true;
+    }
+    return false;
+}
+
+// The grid form: one CTA on every SM, when the shared memory holds each CTA's rows.
+static bool fb_setup_grid(qjx_fb *h, const FbSystem &y)
+{
+    int optin = 0, sms = 0, coop = 0, per = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
+    if (!coop || sms < 1) return false;
+    FbDeal d;
+    fb_deal(y, sms, d);
+    const size_t bytes = fb::fb_rows_bytes(d.maxS, d.maxL, d.maxN) + sizeof(int) * fb::kW * d.maxS + 16;
+    if (bytes + 1024 > (size_t)optin ||
+        cudaFuncSetAttribute(fb::rk4_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fb::rk4_grid, fb::kGridThreads, bytes) != cudaSuccess || per < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    if (!fb_upload_deal(h, y, d, false)) return false;
+    h->R.buf = (double *)fb_alloc(h, sizeof(double) * 2 * ((size_t)y.n + 1));
+    h->R.arrived = (unsigned *)fb_alloc(h, sizeof(unsigned));
+    if (!h->R.buf || !h->R.arrived) return false;
+    h->grid = sms;
+    h->smem = bytes;
+    return true;
 }
 
 extern "C" qjx_status qjx_fb_create(int n, const int *gs_rowptr, const int *gs_col, const double *gs_val,
@@ -334,84 +746,11 @@ extern "C" qjx_status qjx_fb_create(int n, const int *gs_rowptr, const int *gs_c
         qjx_fb_destroy(h);
         return QJX_ERR_CUDA;
     }
-    // cluster-resident path: smallest cluster (power of two <= 16) whose CTAs hold their rows'
-    // CSR slices plus three full vectors in shared memory; QJX_FB_PATH=stages forces the
-    // per-stage kernels.
+    // resident forms; QJX_FB_PATH=stages forces the per-stage kernels
     const char *path = std::getenv("QJX_FB_PATH");
-    const bool stages_only = path && std::string(path) == "stages";
-    int smem_optin = 0;
-    cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    for (int cs = 1; cs <= fb::kMaxCluster && !stages_only && !h->cluster; cs *= 2) {
-        // balanced contiguous row split by nonzeros + a fixed cost per row
-        std::vector<int> lo(cs + 1, n);
-        lo[0] = 0;
-        const long long total = (long long)gnz + qnz + 8LL * n;
-        int r = 0;
-        long long acc = 0;
-        for (int c = 1; c < cs; c++) {
-            const long long target = total * c / cs;
-            while (r < n && acc + (gs_rowptr[r + 1] - gs_rowptr[r]) + (qs_rowptr[r + 1] - qs_rowptr[r]) + 8 <= target) {
-                acc += (gs_rowptr[r + 1] - gs_rowptr[r]) + (qs_rowptr[r + 1] - qs_rowptr[r]) + 8;
-                r++;
-            }
-            lo[c] = r;
-        }
-        int mr = 0, mg = 0, mq = 0;
-        for (int c = 0; c < cs; c++) {
-            mr = std::max(mr, lo[c + 1] - lo[c]);
-            mg = std::max(mg, gs_rowptr[lo[c + 1]] - gs_rowptr[lo[c]]);
-            mq = std::max(mq, qs_rowptr[lo[c + 1]] - qs_rowptr[lo[c]]);
-        }
-        const size_t bytes = sizeof(double) * (3 * (size_t)n + 4 * (size_t)mr + mg + mq) +
-                             sizeof(int) * (2 * (size_t)(mr + 1) + mg + mq);
-        if (bytes + 1024 > (size_t)smem_optin) continue;
-        if (cudaFuncSetAttribute(fb::rk4_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-            continue;
-        if (cs > 8 && cudaFuncSetAttribute(fb::rk4_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-            continue;
-        cudaLaunchConfig_t lc = {};
-        lc.gridDim = dim3(cs);
-        lc.blockDim = dim3(512);
-        lc.dynamicSmemBytes = bytes;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cs;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        lc.attrs = at;
-        lc.numAttrs = 1;
-        int nclusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&nclusters, fb::rk4_cluster, &lc) != cudaSuccess || nclusters < 1) {
-            cudaGetLastError();
-            continue;
-        }
-        int *d_lo = (int *)fb_alloc(h, sizeof(int) * (cs + 1));
-        if (!d_lo) break;
-        cudaMemcpy(d_lo, lo.data(), sizeof(int) * (cs + 1), cudaMemcpyHostToDevice);
-        fb::FbClusterParams &C = h->CP;
-        C.n = n;
-        C.row_lo = d_lo;
-        C.gr = P.gr;
-        C.gc = P.gc;
-        C.gv = P.gv;
-        C.qr = P.qr;
-        C.qc = P.qc;
-        C.qv = P.qv;
-        C.Ks = P.Ks;
-        C.x = P.x;
-        C.drv_ampl = P.drv_ampl;
-        C.drv_freq = P.drv_freq;
-        C.drv_phase = P.drv_phase;
-        C.drv_type = P.drv_type;
-        C.T = T;
-        C.h = T / double(num_steps);
-        C.num_steps = num_steps;
-        C.max_rows = mr;
-        C.max_gnz = mg;
-        C.max_qnz = mq;
-        h->cluster = true;
-        h->cs = cs;
-        h->csmem = bytes;
+    if (!(path && std::string(path) == "stages")) {
+        const FbSystem sys{n, gs_rowptr, gs_col, gs_val, qs_rowptr, qs_col, qs_val, Ks};
+        if (!fb_setup_cluster(h, sys)) fb_setup_grid(h, sys);
     }
     cudaGetLastError();
     *out = h;
@@ -424,25 +763,41 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
     if (cudaSetDevice(h->device) != cudaSuccess) return QJX_ERR_CUDA;
     const fb::FbParams &P = h->P;
     cudaEventRecord(h->e0, h->stream);
-    if (h->cluster) {  // one cluster launch per period
+    if (h->cs || h->grid) {  // one launch per period
         cudaLaunchConfig_t lc = {};
-        lc.gridDim = dim3(h->cs);
-        lc.blockDim = dim3(512);
-        lc.dynamicSmemBytes = h->csmem;
+        lc.gridDim = dim3(h->cs ? h->cs : h->grid);
+        lc.blockDim = dim3(h->cs ? fb::kClusterThreads : fb::kGridThreads);
+        lc.dynamicSmemBytes = h->smem;
         lc.stream = h->stream;
         cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = h->cs;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
+        if (h->cs) {
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = h->cs;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+        } else {
+            at[0].id = cudaLaunchAttributeCooperative;
+            at[0].val.cooperative = 1;
+        }
         lc.attrs = at;
         lc.numAttrs = 1;
         for (int p = period0; p < period0 + n_periods; p++) {
-            fb::FbClusterParams C = h->CP;
-            C.period0 = p;
-            C.n_periods = 1;
-            if (cudaLaunchKernelEx(&lc, fb::rk4_cluster, C) != cudaSuccess) return QJX_ERR_CUDA;
+            fb::FbResParams C = h->R;
+            C.period = p;
+            if (!h->cs) cudaMemsetAsync(C.arrived, 0, sizeof(unsigned), h->stream);
+            const cudaError_t e = h->cs ? cudaLaunchKernelEx(&lc, fb::rk4_cluster, C, h->cs)
+                                        : cudaLaunchKernelEx(&lc, fb::rk4_grid, C);
+            if (e == cudaErrorCooperativeLaunchTooLarge && !h->cs) {
+                // not every CTA can be resident (another context holds SMs): the stage kernels
+                cudaGetLastError();
+                h->grid = 0;
+                if (fb::queue_rk_stages(P, h->T, h->num_steps, p, period0 + n_periods - p, h->stream) != cudaSuccess)
+                    return QJX_ERR_CUDA;
+                break;
+            }
+            if (e != cudaSuccess) return QJX_ERR_CUDA;
         }
+        cudaMemcpyAsync(h->h_fail, h->R.fail, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
     } else if (fb::queue_rk_stages(P, h->T, h->num_steps, period0, n_periods, h->stream) != cudaSuccess) {
         return QJX_ERR_CUDA;
     }
@@ -451,13 +806,14 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, h->e0, h->e1);
     h->last_ms = ms;
+    if (h->h_fail && *h->h_fail) return QJX_ERR_TIMEOUT;
     return QJX_OK;
 }
 
 extern "C" qjx_status qjx_fb_info(qjx_fb *h, int *cluster_size)
 {
     if (!h || !cluster_size) return QJX_ERR_INVALID_ARG;
-    *cluster_size = h->cluster ? h->cs : 0;
+    *cluster_size = h->cs;
     return QJX_OK;
 }
 
@@ -537,6 +893,7 @@ extern "C" void qjx_fb_destroy(qjx_fb *h)
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void *p : h->allocs) cudaFree(p);
+    if (h->h_fail) cudaFreeHost(h->h_fail);
     if (h->e0) cudaEventDestroy(h->e0);
     if (h->e1) cudaEventDestroy(h->e1);
     if (h->stream) cudaStreamDestroy(h->stream);
