@@ -112,10 +112,10 @@ def bench_config(world, n, d, P, W):
 
 
 def kernel_name(d):
-    """Instantiation qjx::step_kernel<NRB, CBMAX> the library picks for dimension d <= 208
-    (32-column sub-tiles: CBMAX 4, NRB row blocks per warp at 4 warps per column block)."""
+    """The plain form's sub-tile kernel as the library instantiates it for 128 < d <= 232 (256 threads,
+    16-column sub-tiles: row blocks per warp at 4 and at 8 warps per column block)."""
     rb = (d + 7) // 8
-    return f"qjx::step_kernel<{(rb + 3) // 4}, 4>"
+    return f"qjx::flow_kernel<256, {(rb + 3) // 4}, {(rb + 7) // 8}, 0>"
 
 
 def start_states(n, d):
@@ -224,7 +224,7 @@ def fbasis_bench(args, local):
     out = {"workload": f"f-basis Lindblad RK4, dimer N={FB_N} (f-vector {n}), dt={FB_DT} ({steps} steps/period), "
                        f"Gs nnz {Gs.nnz}, Qs nnz {Qs.nnz}",
            "metric": "periods/s", "value": 1e3 / per, "ms_per_period": per, "us_per_rk4_step": 1e3 * per / steps,
-           "kernel": "fb::rk4_cluster" if cs else "fb::rk_stage + fb::rk_update", "cluster_size": cs,
+           "kernel": "fb::rk4_cluster" if cs else "fb::rk4_grid", "cluster_size": cs,
            "roofline": {"bound": "shared memory / cluster barrier latency (operands resident in the cluster's shared "
                                  "memory, no HBM traffic after the first load)",
                         "achieved": achieved, "unit": "GB/s", "peak": smem_peak,
@@ -260,7 +260,7 @@ def batch_draw(count):
 
 def batched_bench(args, local):
     """Chosen form 2: ensembles of uneven dimension advanced together by one engine (one set of
-    persistent micro-step launches, CUDA graphs of 6 micro-steps), one period per step, against
+    persistent launches and queues), one period per step, against
     the same ensembles solved one after another by single-ensemble engines (serial plain FP64)."""
     import torch
 
@@ -341,7 +341,7 @@ def batched_bench(args, local):
         "serial_single_ensemble_engines": {"value": n_tot * args.steps / (ms_serial * 1e-3),
                                            "ms_per_step": ms_serial / args.steps},
         "speedup_vs_serial": ms_serial / ms,
-        "roofline": {"bound": "tensor", "kernel": "qjx::step_kernel (per-(ensemble, matrix) buckets)",
+        "roofline": {"bound": "tensor", "kernel": "qjx::flow_kernel and qjx::solo_kernel (per-(ensemble, matrix) queues)",
                      "achieved": flops / kern_s / 1e12, "peak": peak, "unit": "TFLOP/s",
                      "frac": flops / kern_s / 1e12 / peak,
                      "flops": "8 d_e^2 per executed matvec, summed over the ensembles (matvecs counted by the "
@@ -831,9 +831,9 @@ def run_ours(args):
     ms_per_step = dev_ms_max / args.steps
     ens_sum = ens_plain[-1]
 
-    # roofline of the dominant kernel (step_kernel, grouped FP64 complex GEMM + fused epilogue)
+    # roofline of the dominant kernel (flow_kernel, grouped FP64 complex GEMM + fused epilogue)
     matvecs = st1["matvecs"] - st0["matvecs"]
-    launches_step = st1["micro_steps"] - st0["micro_steps"]
+    launches_step = st1["launches"] - st0["launches"]
     kern_ms = st1["step_kernel_ms"] - st0["step_kernel_ms"]
     flops = 8.0 * d * d * matvecs
     achieved = flops / (kern_ms * 1e-3) / 1e12

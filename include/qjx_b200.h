@@ -60,7 +60,7 @@ typedef struct qjx_engine qjx_engine;
  * output keeps its own summation order whatever the tiling. */
 typedef struct {
     int nc;      /* plain form: trajectory columns per sub-tile (32, 16 or 8) */
-    int kb;      /* plain form: k rows per propagator slab (even, 2..16) */
+    int kb;      /* plain form: most k rows per propagator slab (even, 2..16) */
     int stages;  /* split form: depth of the operand ring (2..8) */
     int rows;    /* split form: fewest trajectories per tcgen05 tile (multiple of 8, 8..128) */
 } qjx_tiles;
@@ -111,7 +111,8 @@ typedef struct {
 } qjx_config;
 
 typedef struct {
-    int64_t micro_steps;     /* lock-step micro-steps launched */
+    int64_t micro_steps;     /* split form: lock-step micro-steps; plain form: sub-tiles (one matrix on 1 to 32
+                                trajectories) */
     int64_t matvecs;         /* complex d x d matvecs executed (trajectory-steps) */
     int64_t jumps;           /* jumps recorded */
     double kernel_ms;        /* device time of run/observe calls, first to last launch (CUDA events) */

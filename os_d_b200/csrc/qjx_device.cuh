@@ -14,18 +14,26 @@
 namespace qjx {
 
 // ---- launch geometry of the micro-step kernel ----
-constexpr int kThreads = 512;          // 16 warps (micro-step kernel)
-constexpr int kNC = 32;                // trajectory columns per sub-tile (max)
-constexpr int kKB = 16;                // k rows per propagator slab (8 k pairs)
-constexpr int kStages = 2;             // slab pipeline depth
+constexpr int kThreads = 512;          // 16 warps (split-form kernel)
+constexpr int kKB = 16;                // most k rows per propagator slab
+constexpr int kMaxDt = 64;             // split-level steps [nb][deep] a CTA keeps in shared memory
+constexpr int kColPad = 2;             // components between staged columns past the padded rows
 constexpr int kMaxGroups = 256;        // distinct matrices in one engine
 constexpr int kMaxMD = 1024;           // d <= 1024 (plain form; the split form takes d <= 256)
 constexpr double kSplitNormSlack = 1e-4;  // split precision: tolerated norm excess over 1
 constexpr int kMaxSplitStages = 8;        // split precision: deepest operand ring
-// Thread layouts of a sub-tile (rows ty + TY i, columns tx + TX j, TY * TX = 256):
-//   TY = 32: MD = 32 * MT padded rows, TX = 8 column threads, up to 4 columns each
-//   TY = 16: MD = 16 * MT padded rows, TX = 16 column threads, up to 2 columns each
-// The host picks the layout with fewer padded rows.
+// plain kernel: a launch hands the device back after kSliceNs (engines of other streams get
+// their turn; the host launches again), and a CTA that finds no work for kIdleNs leaves
+constexpr unsigned long long kSliceNs = 4000000, kIdleNs = 200000;
+constexpr unsigned kFree = 0xffffffffu;  // an empty queue entry
+constexpr int kSoloThreads = 256;      // most threads (rows) per CTA of the one-trajectory kernel
+constexpr int kLive = 6;               // ctrl[6]: trajectories the plain kernel has not finished in this call
+
+// Position of M[row][k] in a matrix of MD padded rows: mats[g][k / 2][row][k % 2].
+__host__ __device__ inline size_t mat_at(int k, int row, int MD)
+{
+    return 2 * ((size_t)(k >> 1) * MD + row) + (k & 1);
+}
 
 // ---- trajectory phases ----
 enum Phase : int {
@@ -72,17 +80,51 @@ struct __align__(16) TrajState {
 };
 static_assert(sizeof(TrajState) == 144, "TrajState layout");
 
+// What the plain kernel needs of a group (one matrix of one ensemble).
+struct __align__(16) GroupDesc {
+    long long roff;                 // its queue's ring in Params::ring
+    long long moff;                 // its matrix in Params::mats (double2 units)
+    unsigned char rlog, nc, kb, _;  // log2 of the ring length (>= the ensemble's trajectories), columns per
+                                    // sub-tile (32, 16 or 8), k rows per propagator slab
+    int d, ens, group;              // dimension, ensemble, the group itself
+    __host__ __device__ unsigned rmask() const { return (1u << rlog) - 1u; }
+};
+static_assert(sizeof(GroupDesc) == 32, "two 16-byte loads");
+
+// A group's queue: entries waiting, counts of the entries taken and reserved so far, and the widest
+// sub-tile of its ensemble.
+struct __align__(16) Queue {
+    int avail;
+    unsigned head, tail;
+    int nc;
+};
+
+__device__ __forceinline__ GroupDesc load_desc(const GroupDesc *p)
+{
+    GroupDesc g;
+    uint4 *t = reinterpret_cast<uint4 *>(&g);
+    t[0] = __ldg(reinterpret_cast<const uint4 *>(p));
+    t[1] = __ldg(reinterpret_cast<const uint4 *>(p) + 1);
+    return g;
+}
+
 struct Params {
     int d, MD, n, deep, nb, nd, nr, G;
     int gL0, gHE, gR0;
-    const double2 *mats;     // [G][d][MD]  transposed matrices: mats[g][k][row]
+    int Ge;                  // groups per ensemble (ensemble e's first group is e Ge)
+    const double2 *mats;     // [G][kp / 2][MD][2]  matrices by k pair: mats[g][k / 2][row][k % 2]
     double2 *psi;            // [2][n][MD]
     TrajState *st;           // [n]
     double *gn;              // [n][nd] channel weights
     const double *g;         // [nd]
     const double *dt;        // [deep]
-    int *cnt;                // [3][G]
-    int *lists;              // [2][G][n]
+    int *cnt;                // [3][G]  split form: bucket sizes of three micro-steps
+    int *lists;              // [2][ltot] split form: bucket lists of two
+    // plain form: one queue per group, a ring of entries (trajectory and input slot; kFree: empty)
+    // with counts of the entries taken and reserved so far
+    Queue *q;                // [G]
+    unsigned int *ring;
+    const GroupDesc *gd;     // [G]
     // rng
     int rng_kind;
     unsigned long long seed;
@@ -107,9 +149,9 @@ struct Params {
     double *r_time, *r_norm, *r_eta;
     int *r_type;
     // control: [0] error count, [1] first error trajectory, [2] paused count, [3] first error code,
-    //          [4] timeouts
+    //          [4] timeouts, [kLive] trajectories left (plain form)
     int *ctrl;
-    long long *work;         // [0] trajectory-matvecs executed
+    long long *work;         // trajectory-matvecs; split form: tiles, rechecks; [3] plain form: sub-tiles
     // optional per-CTA trace, accumulated over micro-steps: [grid][kTraceFields] clock64 cycles
     // and counts (null: tracing off)
     long long *trace;
@@ -147,11 +189,7 @@ struct Params {
     // (the ensemble slots of a serving engine)
     int n_active;
     const unsigned char *active;
-    // plain step kernel tiling, per ensemble (chosen from its padded rows and the shared memory):
-    // columns per sub-tile (32, 16 or 8) and k rows per propagator slab; step_smem is the
-    // kernel's dynamic shared memory (the largest ensemble layout)
-    const int *e_nc, *e_kb;
-    int step_smem;
+    int step_smem;                // plain kernel: dynamic shared memory (the largest ensemble layout)
     // ensembles (a batched engine holds E ensembles of their own dimension, operators, seed and
     // period; an ordinary engine is the batch of one).  Trajectories [e_tr0[e], e_tr0[e+1]) form
     // ensemble e; its groups are e_g0[e] + the local group (branch * deep + level, gL0 + channel,
@@ -169,24 +207,10 @@ struct Params {
     const long long *g_loff;          // [G] start of the group's bucket list (capacity: the
                                       // ensemble's trajectories); lists hold 2 x ltot entries
     long long ltot;
-    // plain step kernel plan of the next micro-step: [0, G] bucket starts, [G + 1, 2G + 1] cost
-    // prefix; written by the last CTA of a micro-step (or plan_kernel after a host call)
-    int *plan;
     unsigned int *plan_sync;          // [1] CTAs finished in the current micro-step
     unsigned int *gen;                // [1] split form: plans made (the grid barrier of a multi-step launch)
     int *sdone;                       // [1] split form: micro-steps run since the host last cleared it
 };
-
-// Dimension, split-level steps and jump rates of a trajectory's ensemble.
-__device__ __forceinline__ int dim_of(const Params &P, const TrajState &s) { return P.e_d[s.ens]; }
-__device__ __forceinline__ const double *dt_of(const Params &P, const TrajState &s)
-{
-    return P.e_dt + ((size_t)s.ens * P.nb + s.b) * P.deep;
-}
-__device__ __forceinline__ double rate_of(const Params &P, const TrajState &s, int i)
-{
-    return P.e_rate[(size_t)s.ens * P.nd + i];
-}
 
 // Lyapunov paired trajectories (task_id 7, LpnMult): [0, n/2) bases, n/2 + b the variation of b.
 struct LpnParams {

@@ -1,6 +1,6 @@
-// qjx_engine.cu -- host side of the QJ trajectory engine: device memory, the micro-step
-// loop (CUDA graphs of 6 micro-steps, bounded host polling), jump-record draining, and the
-// C ABI declared in include/qjx_b200.h.
+// qjx_engine.cu -- host side of the QJ trajectory engine: device memory, the loops over time slices
+// (plain form) and micro-step batches (split form), jump-record draining, and the C ABI declared in
+// include/qjx_b200.h.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -17,13 +17,15 @@
 #include "qjx_device.cuh"
 
 namespace qjx {
-cudaError_t launch_step(const Params &P, int s, int grid, cudaStream_t st);
+cudaError_t launch_flow(const Params &P, int nt, int stop_live, int grid, cudaStream_t st);
+cudaError_t launch_solo(const Params &P, int C, int workers, cudaStream_t st);
+cudaError_t launch_split_step(const Params &P, int s, int grid, cudaStream_t st);
 cudaError_t launch_split_steps(const Params &P, int s0, int nsteps, int grid, cudaStream_t st);
 int pick_layout(int d, int *rows_per_block);
 cudaError_t launch_dmma_peak(double *out, int blocks, int iters, cudaStream_t st);
 size_t step_smem_bytes(int MD, int nc, int kb);
-bool pick_step_tiles(int MD, size_t budget, int *nc, int *kb);
-size_t step_static_smem();
+bool pick_step_tiles(int MD, size_t budget, int nt, int nc_max, int *nc, int *kb);
+size_t step_static_smem(int nt);
 cudaError_t launch_schedule(const Params &P, int mode, cudaStream_t st);
 cudaError_t launch_observe(const Params &P, int dump, int is_start, cudaStream_t st);
 cudaError_t launch_init_state(const Params &P, cudaStream_t st, int tr0 = 0, int tr1 = -1);
@@ -53,6 +55,9 @@ struct qjx_engine {
     Params P{};
     int MD = 0;
     int grid = 0;
+    size_t ring_len = 0;               // plain form: entries of all queues
+    int flow_nt = 512, flow_grid = 0;  // plain kernel: threads per CTA, most CTAs
+    int solo_max = 0;                  // plain form: most trajectories that run one to a CTA
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, eb0 = nullptr, eb1 = nullptr;
     std::string err;
@@ -139,16 +144,23 @@ static thread_local std::string g_create_err;
 
 extern "C" const char *qjx_last_error(const qjx_engine *h) { return h ? h->err.c_str() : g_create_err.c_str(); }
 
-// Transposes row-major complex d x d matrices into the device layout mats[g][k][row]
-// (rows padded to MD and k to an even count with zeros), so one K-slab is one contiguous
-// TMA bulk copy and the last k pair of the FP64 MMA multiplies exact zeros.
+// Puts row-major complex d x d matrices into the device layout mats[g][k / 2][row][k % 2]
+// (rows padded to MD and k to an even count with zeros): a K-slab of even height is one
+// contiguous TMA bulk copy, a k pair's 8-row block is the A operand of the FP64 MMA in lane order,
+// and the last k pair multiplies exact zeros.
 static void pack_transposed(const double *M, int d, int MD, double *out)
 {
-    for (int i = 0; i < d; i++)
-        for (int k = 0; k < d; k++) {
-            out[2 * ((size_t)k * MD + i)] = M[2 * ((size_t)i * d + k)];
-            out[2 * ((size_t)k * MD + i) + 1] = M[2 * ((size_t)i * d + k) + 1];
-        }
+    // blocks of 8 rows x 8 k: whole cache lines on both sides
+    for (int i0 = 0; i0 < d; i0 += 8)
+        for (int k0 = 0; k0 < d; k0 += 8)
+            for (int k = k0; k < std::min(d, k0 + 8); k++) {
+                double *o = out + 2 * mat_at(k, i0, MD);
+                const double *m = M + 2 * ((size_t)i0 * d + k);
+                for (int i = i0; i < std::min(d, i0 + 8); i++, o += 4, m += 2 * (size_t)d) {
+                    o[0] = m[0];
+                    o[1] = m[1];
+                }
+            }
 }
 
 // bf16 nearest (ties to even) of x with 8 significant bits; *val receives the rounded value.
@@ -230,15 +242,29 @@ static T *upload(qjx_engine *h, const std::vector<T> &v)
 }
 
 // ---------------------------------------------------------------- tile shapes
-// Whether the plain kernel can run sub-tiles of nc columns and slabs of kb k rows for padded rows
-// MD within `budget` bytes of dynamic shared memory (the constraints pick_step_tiles applies).
-static bool tiles_fit(int MD, size_t budget, int nc, int kb)
+// Whether a plain-form shape (columns per sub-tile, k rows per slab) is valid for padded rows MD: at
+// most 8 row blocks per warp of a 512-thread CTA, and columns and two slabs within kTileSmem bytes.
+constexpr size_t kTileSmem = 225920;
+static bool tiles_valid(int MD, int nc, int kb)
 {
     if (nc != 8 && nc != 16 && nc != 32) return false;
     if (kb < 2 || kb > kKB || (kb & 1)) return false;
     const int RB = MD / 8, W1 = 16 / (nc / 8);
     if ((RB + W1 - 1) / W1 > 8) return false;
-    return step_smem_bytes(MD, nc, kb) <= budget;
+    return (size_t)(nc * (MD + 1) + 2 * kb * MD) * sizeof(double2) <= kTileSmem;
+}
+
+// Whether the plain kernel with nt threads can run the shape within `budget` bytes of dynamic shared
+// memory; lowers *kb where that makes it fit (the slab height never changes results).
+static int max_columns(int MD, int nt) { return nt == 512 || MD <= 128 ? 32 : 16; }
+
+static bool tiles_fit(int MD, size_t budget, int nt, int nc, int *kb)
+{
+    if (nc > max_columns(MD, nt)) return false;
+    const int RB = MD / 8, W1 = nt / 32 / (nc / 8);
+    if ((RB + W1 - 1) / W1 > 8) return false;
+    while (*kb > 2 && step_smem_bytes(MD, nc, *kb) > budget) *kb -= 2;
+    return step_smem_bytes(MD, nc, *kb) <= budget;
 }
 
 // The autotuner's cache: text lines "precision d nc kb stages rows us" (later lines win), in
@@ -364,29 +390,45 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     h->MD = MD;
     Params &P = h->P;
     std::vector<int> e_nc(E), e_kb(E);
-    {  // plain step kernel tiling of every ensemble within the shared memory
-        int optin = 0;
+    {  // plain kernel tiling of every ensemble within the shared memory
+        int optin = 0, per_sm = 0, reserved = 0;
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device);
-        const size_t fixed = step_static_smem() + 1024;
-        if ((size_t)optin <= fixed) return bail(QJX_ERR_UNSUPPORTED);
-        size_t smem = 0;
-        const size_t budget = (size_t)optin - fixed;
-        for (int e = 0; e < E; e++) {
-            const int MDe = 8 * ((ens[e].d + 7) / 8);
-            qjx_tiles ct{};
-            if (c.tiles.nc > 0 || c.tiles.kb > 0) {  // explicit shapes must fit
-                if (!tiles_fit(MDe, budget, c.tiles.nc, c.tiles.kb)) return bail(QJX_ERR_UNSUPPORTED);
-                e_nc[e] = c.tiles.nc;
-                e_kb[e] = c.tiles.kb;
-            } else if (tile_cache_get(0, ens[e].d, &ct) && tiles_fit(MDe, budget, ct.nc, ct.kb)) {
-                e_nc[e] = ct.nc;  // the autotuner's choice for this dimension
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c.device);
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, c.device);
+        // two CTAs of 256 threads per SM when every ensemble's sub-tiles fit half of the SM's shared
+        // memory (16 columns and slabs of at least 6 k rows, d <= 232, or explicit or autotuned shapes
+        // of at most 16 columns), so that one CTA's scan, staging and epilogue overlap the other's
+        // products; else one CTA of 512
+        const size_t whole = (size_t)std::max(0, optin - (int)step_static_smem(512));
+        for (const int nt : {256, 512}) {
+            const size_t budget =
+                nt == 512 ? whole : (size_t)std::max(0, per_sm / 2 - reserved - (int)step_static_smem(256));
+            size_t smem = 0;
+            bool fits = nt == 512 || MD <= 256;
+            for (int e = 0; e < E && fits; e++) {
+                const int MDe = 8 * ((ens[e].d + 7) / 8);
+                qjx_tiles ct{};
+                if (c.tiles.nc > 0 || c.tiles.kb > 0) {  // an explicit shape must fit
+                    ct = c.tiles;
+                    if (!tiles_valid(MDe, ct.nc, ct.kb)) return bail(QJX_ERR_UNSUPPORTED);
+                    fits = ct.nc <= max_columns(MD, nt) && tiles_fit(MDe, budget, nt, ct.nc, &ct.kb);
+                } else if (tile_cache_get(0, ens[e].d, &ct) && tiles_valid(MDe, ct.nc, ct.kb)) {
+                    fits = ct.nc <= max_columns(MD, nt) && tiles_fit(MDe, budget, nt, ct.nc, &ct.kb);  // the autotuner's choice for this dimension
+                } else {
+                    fits = pick_step_tiles(MDe, budget, nt, std::min(max_columns(MDe, nt), max_columns(MD, nt)), &ct.nc, &ct.kb) &&
+                           (nt == 512 || (ct.nc >= 16 && ct.kb >= 6));
+                }
+                e_nc[e] = ct.nc;
                 e_kb[e] = ct.kb;
-            } else if (!pick_step_tiles(MDe, budget, &e_nc[e], &e_kb[e])) {
-                return bail(QJX_ERR_UNSUPPORTED);
+                if (fits) smem = std::max(smem, step_smem_bytes(MDe, ct.nc, ct.kb));
             }
-            smem = std::max(smem, step_smem_bytes(MDe, e_nc[e], e_kb[e]));
+            if (!fits && nt == 512) return bail(QJX_ERR_UNSUPPORTED);
+            if (!fits) continue;
+            h->flow_nt = nt;
+            h->flow_grid = h->grid * (nt == 256 ? 2 : 1);
+            P.step_smem = (int)smem;
+            break;
         }
-        P.step_smem = (int)smem;
     }
     P.d = d;
     P.MD = MD;
@@ -398,6 +440,7 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     P.G = G;
     P.E = E;
     P.gL0 = c.num_branches * c.deep;  // local group offsets, the same in every ensemble
+    P.Ge = Ge;
     P.gHE = P.gL0 + c.num_diss;
     P.gR0 = P.gHE + 1;
     P.rng_kind = c.rng_kind;
@@ -453,8 +496,6 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     h->e_tr0 = e_tr0;
     h->e_d_host = e_d;
     P.e_d = upload(h, e_d);
-    P.e_nc = upload(h, e_nc);
-    P.e_kb = upload(h, e_kb);
     P.e_tr0 = upload(h, e_tr0);
     P.e_g0 = upload(h, e_g0);
     P.e_dt = upload(h, e_dt);
@@ -465,14 +506,21 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     P.g_ens = upload(h, g_ens);
     P.g_loff = upload(h, g_loff);
     P.ltot = loff;
+    // Where one trajectory per CTA beats shared sub-tiles: it reads a whole matrix (16 d^2 bytes, from L2)
+    // per trajectory and step, but has no queue and a short step.  Measured best switch-over on ensembles of
+    // one dimension (ms a period there / one trajectory per CTA throughout / sub-tiles to the last 100): d = 31:
+    // 10^4 (10.2 / 10.2 / 11.1), d = 51: 3000 (14.5 / 18.1 / 16.3), d = 101: 500 to 1300 (21.3 / 33.9 /
+    // 24.3), d = 201: 350 to 600 (68.5 / 78.3 / 74.7), d = 401: all of 300 (236 / 236 / 269); d^2 is the
+    // trajectories' mean in a batch.
+    double d2 = 0.0;
+    for (const EnsDesc &x : ens) d2 += (double)x.n * x.d * x.d;
+    h->solo_max = 250 + (int)(6.5e6 / (d2 / n));
     P.dt = P.e_dt;
     P.g = P.e_rate;
-    P.plan = (int *)dalloc(h, (size_t)(2 * G + 2) * sizeof(int));
     P.plan_sync = (unsigned int *)dalloc(h, sizeof(unsigned int));
-    if (!P.e_d || !P.e_nc || !P.e_kb || !P.e_tr0 || !P.e_g0 || !P.e_dt || !P.e_rate || !P.e_seed || !P.e_sbase || !P.g_off || !P.g_ens ||
-        !P.g_loff || !P.plan || !P.plan_sync)
+    if (!P.e_d || !P.e_tr0 || !P.e_g0 || !P.e_dt || !P.e_rate || !P.e_seed || !P.e_sbase || !P.g_off || !P.g_ens ||
+        !P.g_loff || !P.plan_sync)
         return bail(QJX_ERR_OOM);
-    cudaMemset(P.plan, 0, (size_t)(2 * G + 2) * sizeof(int));
     cudaMemset(P.plan_sync, 0, sizeof(unsigned int));
 
     P.grid = h->grid;
@@ -552,8 +600,27 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     P.psi = (double2 *)dalloc(h, (size_t)psi_slots * n * MD * sizeof(double2));
     P.st = (TrajState *)dalloc(h, (size_t)n * sizeof(TrajState));
     P.gn = (double *)dalloc(h, (size_t)n * c.num_diss * sizeof(double));
-    P.cnt = (int *)dalloc(h, (size_t)3 * G * sizeof(int));
-    P.lists = (int *)dalloc(h, (size_t)2 * P.ltot * sizeof(int));
+    if (c.precision == 1) {  // lock-step bucket lists
+        P.cnt = (int *)dalloc(h, (size_t)3 * G * sizeof(int));
+        P.lists = (int *)dalloc(h, (size_t)2 * P.ltot * sizeof(int));
+    } else {  // queues: a ring per group, a power of two long so that the positions may wrap
+        std::vector<GroupDesc> gd(G);
+        std::vector<Queue> q(G);
+        long long roff = 0;
+        for (int e = 0; e < E; e++) {
+            int rlog = 0;
+            while ((1ll << rlog) < ens[e].n) rlog++;
+            for (int l = 0; l < Ge; l++, roff += 1ll << rlog) {
+                gd[e * Ge + l] = GroupDesc{roff, g_off[e * Ge + l], (unsigned char)rlog, (unsigned char)e_nc[e],
+                                           (unsigned char)e_kb[e], 0, ens[e].d, e, e * Ge + l};
+                q[e * Ge + l] = Queue{0, 0, 0, e_nc[e]};
+            }
+        }
+        h->ring_len = (size_t)roff;
+        P.q = upload(h, q);
+        P.ring = (unsigned int *)dalloc(h, h->ring_len * sizeof(unsigned int));
+        P.gd = upload(h, gd);
+    }
     const size_t nd_ = (size_t)h->cfg.max_dumps * n;
     P.o_norm = (double *)dalloc(h, nd_ * sizeof(double));
     P.o_mean = (double *)dalloc(h, nd_ * sizeof(double));
@@ -570,7 +637,7 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     P.r_type = (int *)dalloc(h, rc * sizeof(int));
     P.ctrl = (int *)dalloc(h, 16 * sizeof(int));
     P.work = (long long *)dalloc(h, 4 * sizeof(long long));
-    if (!P.psi || !P.st || !P.gn || !P.cnt || !P.lists || !P.o_norm || !P.o_mean || !P.o_disp || !P.o_m2 ||
+    if (!P.psi || !P.st || !P.gn || (P.split ? !P.cnt || !P.lists : !P.q || !P.ring || !P.gd) || !P.o_norm || !P.o_mean || !P.o_disp || !P.o_m2 ||
         !P.o_energy || !P.o_robs || !P.o_adr || !P.mean_start || !P.r_time || !P.r_norm || !P.r_eta || !P.r_type ||
         !P.ctrl || !P.work)
         return bail(QJX_ERR_OOM);
@@ -738,133 +805,149 @@ static qjx_status drain_records(qjx_engine *h)
     return QJX_OK;
 }
 
-// Runs lock-step micro-steps until every trajectory is done for this call.  Step 0 of the
-// call reads buckets written into cnt[0] / lists[0] by the schedule or observe kernel.
-static qjx_status run_until_idle(qjx_engine *h)
+// Empty buckets, queues and control words before a call's schedule or observe kernel fills them.
+static cudaError_t clear_queues(qjx_engine *h)
 {
     Params &P = h->P;
-    // plain form: CUDA graphs of 6 micro-steps; split form: one cooperative launch runs up to
-    // 6 x batch micro-steps with grid barriers between them (the buffers rotate with period 6)
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    if (!P.split) {
-        CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        for (int s = 0; s < 6; s++) {
-            cudaError_t e = launch_step(P, s, h->grid, h->stream);
-            if (e != cudaSuccess) {
-                cudaStreamEndCapture(h->stream, &graph);
-                if (graph) cudaGraphDestroy(graph);
-                return cuda_fail(h, e, "launch_step");
-            }
-        }
-        CK(cudaStreamEndCapture(h->stream, &graph));
-        cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (ie != cudaSuccess) return cuda_fail(h, ie, "cudaGraphInstantiate");
+    cudaError_t e = cudaMemsetAsync(P.ctrl, 0, sizeof(int) * 16, h->stream);
+    if (P.split) {
+        if (e == cudaSuccess) e = cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream);
+    } else {
+        if (e == cudaSuccess) // the counts, not the sub-tile width
+            e = cudaMemset2DAsync(P.q, sizeof(Queue), 0, offsetof(Queue, nc), P.G, h->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(P.ring, 0xff, sizeof(unsigned int) * h->ring_len, h->stream);
     }
-    int s0 = 0;  // split form: index of the next micro-step
-    int64_t nlaunch = 0;
+    return e;
+}
 
-    qjx_status rs = QJX_OK;
-    int batch = 1;
-    // QJX_TRACE_BUCKETS=<file>: append the bucket sizes seen at every host poll (profiling aid)
-    FILE *bucket_log = nullptr;
-    if (const char *fn = getenv("QJX_TRACE_BUCKETS")) bucket_log = fopen(fn, "a");
-    int64_t steps = 0;
-    long long work0[3] = {0, 0, 0};
-    cudaMemcpy(work0, P.work, 3 * sizeof(long long), cudaMemcpyDeviceToHost);
-    cudaEventRecord(h->ev0, h->stream);
+// Trajectories paused on full record buffers: drains the records and queues them again (the split
+// form's lists start over at step 0).
+static qjx_status resume_paused(qjx_engine *h)
+{
+    Params &P = h->P;
+    const qjx_status rs = drain_records(h);
+    if (rs != QJX_OK) return rs;
+    CK(cudaMemsetAsync(P.ctrl + 2, 0, sizeof(int), h->stream));
+    if (P.split) {
+        CK(cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream));
+        CK(cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream));
+    }
+    CK(launch_schedule(P, 1, h->stream));
+    h->stats.launches += 2;
+    return QJX_OK;
+}
+
+// CTAs that share a trajectory in the one-trajectory kernel: as many as d needs at a thread per row,
+// and up to 128 rows each while every CTA has an SM of its own (d = 201, 60 trajectories: 20.4 ms a
+// period with 2, 23.6 with 1, 21.6 with 4; d = 401: 66 ms with 4 against 73 with 2 for 30
+// trajectories, 145 against 136 for 150, where two CTAs share an SM's L2 bandwidth).
+static int solo_ctas(const qjx_engine *h, int live)
+{
+    int C = 1;
+    while (h->P.d > kSoloThreads * C) C *= 2;
+    while (C < 8 && h->P.d > 128 * C && live * 2 * C <= h->grid) C *= 2;
+    return C;
+}
+
+// Plain form: one launch per time slice until no trajectory is left.  Up to solo_max trajectories run
+// one to a CTA or cluster, more share sub-tiles.
+static qjx_status run_flow(qjx_engine *h, FILE *bucket_log, int64_t *nlaunch)
+{
+    Params &P = h->P;
+    int live = P.n;
     while (true) {
-        cudaEventRecord(h->eb0, h->stream);
-        if (P.split) {
-            cudaMemsetAsync(P.sdone, 0, sizeof(int), h->stream);
-            cudaError_t e = h->split_coop ? launch_split_steps(P, s0, 6 * batch, h->grid, h->stream)
-                                          : cudaErrorCooperativeLaunchTooLarge;
-            if (e == cudaErrorCooperativeLaunchTooLarge) {
-                // not every CTA can be resident (another context holds SMs): the same micro-steps
-                // as one launch each (an empty step returns at once)
-                cudaGetLastError();
-                h->split_coop = false;
-                e = cudaSuccess;
-                for (int k = 0; k < 6 * batch && e == cudaSuccess; k++) e = launch_step(P, s0 + k, h->grid, h->stream);
-                nlaunch += 6 * batch;
-            } else {
-                nlaunch += 1;
-            }
-            if (e != cudaSuccess) {
-                rs = cuda_fail(h, e, "launch_split_steps");
-                break;
-            }
-        } else {
-            for (int b = 0; b < batch; b++) {
-                cudaError_t e = cudaGraphLaunch(exec, h->stream);
-                if (e != cudaSuccess) {
-                    rs = cuda_fail(h, e, "cudaGraphLaunch");
-                    break;
-                }
-            }
-            if (rs != QJX_OK) break;
-            steps += 6 * batch;
-            nlaunch += 6 * batch;
-        }
-        cudaEventRecord(h->eb1, h->stream);
-        // plain form: the next micro-step's plan total (or all bucket sizes for the bucket log),
-        // which the last micro-step computed; split form: the micro-steps run, the recheck counts
-        // and the next step's tiles
-        const bool all_counts = !P.split && bucket_log;
-        if (P.split) {
-            cudaMemcpyAsync(h->h_ctrl + 8, P.rcnt, 3 * sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-            cudaMemcpyAsync(h->h_ctrl + 11, P.sdone, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-            cudaMemcpyAsync(h->h_ctrl + 12, P.splan + 1 + P.G, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-        } else if (all_counts) {
-            cudaMemcpyAsync(h->h_cnt, P.cnt, sizeof(int) * P.G, cudaMemcpyDeviceToHost, h->stream);
-        } else {
-            cudaMemcpyAsync(h->h_cnt, P.plan + P.G, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-        }
-        cudaMemcpyAsync(h->h_ctrl, P.ctrl, sizeof(int) * 8, cudaMemcpyDeviceToHost, h->stream);
-        cudaError_t e = cudaStreamSynchronize(h->stream);
-        if (e != cudaSuccess) {
-            rs = cuda_fail(h, e, "micro-step batch");
-            break;
-        }
-        if (P.split) {
-            steps += h->h_ctrl[11];
-            s0 = (s0 + h->h_ctrl[11]) % 6;
-        }
-        float bms = 0.f;
-        cudaEventElapsedTime(&bms, h->eb0, h->eb1);
-        h->stats.step_kernel_ms += bms;
-        rs = check_ctrl(h);
-        if (rs != QJX_OK) break;
-        long long active = all_counts ? 0 : h->h_cnt[0];
-        if (all_counts)
-            for (int g = 0; g < P.G; g++) active += h->h_cnt[g];
-        // split form: tiles of the next step and trajectories waiting for an FP64 recheck
-        if (P.split) active = (long long)h->h_ctrl[12] + h->h_ctrl[8 + s0 % 3];
-        if (bucket_log && all_counts) {
+        CK(cudaEventRecord(h->eb0, h->stream));
+        if (live <= h->solo_max) CK(launch_solo(P, solo_ctas(h, live), live, h->stream));
+        else CK(launch_flow(P, h->flow_nt, h->solo_max, std::min(h->flow_grid, live), h->stream));
+        CK(cudaEventRecord(h->eb1, h->stream));
+        *nlaunch += 1;
+        if (bucket_log)
+            CK(cudaMemcpy2DAsync(h->h_cnt, sizeof(int), P.q, sizeof(Queue), sizeof(int), P.G, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaMemcpyAsync(h->h_ctrl, P.ctrl, sizeof(int) * 8, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, h->eb0, h->eb1);
+        h->stats.step_kernel_ms += ms;
+        qjx_status rs = check_ctrl(h);
+        if (rs != QJX_OK) return rs;
+        if (bucket_log) {
             for (int g = 0; g < P.G; g++) fprintf(bucket_log, g ? " %d" : "%d", h->h_cnt[g]);
             fprintf(bucket_log, "\n");
         }
-        if (active == 0) {
-            if (h->h_ctrl[2] > 0) {  // paused on full record buffers: drain and resume
-                rs = drain_records(h);
-                if (rs != QJX_OK) break;
-                cudaMemsetAsync(P.ctrl + 2, 0, sizeof(int), h->stream);
-                cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream);
-                if (P.rcnt) cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream);
-                cudaError_t le = launch_schedule(P, 1, h->stream);
-                h->stats.launches += 2;
-                if (le != cudaSuccess) {
-                    rs = cuda_fail(h, le, "launch_schedule");
-                    break;
-                }
-                s0 = 0;  // the schedule wrote step 0's buckets
-                continue;
-            }
-            break;
+        live = h->h_ctrl[kLive];
+        if (live > 0) continue;
+        if (h->h_ctrl[2] == 0) return QJX_OK;
+        rs = resume_paused(h);
+        if (rs != QJX_OK) return rs;
+        live = P.n;
+    }
+}
+
+// Split form: one cooperative launch runs up to 6 x batch lock-step micro-steps with grid barriers
+// between them (the buffers rotate with period 6).  Step 0 reads the buckets in cnt[0] / lists[0]
+// that the schedule or observe kernel wrote.
+static qjx_status run_split(qjx_engine *h, int64_t *steps, int64_t *nlaunch)
+{
+    Params &P = h->P;
+    int s0 = 0;  // index of the next micro-step
+    int batch = 1;
+    while (true) {
+        CK(cudaEventRecord(h->eb0, h->stream));
+        CK(cudaMemsetAsync(P.sdone, 0, sizeof(int), h->stream));
+        cudaError_t e = h->split_coop ? launch_split_steps(P, s0, 6 * batch, h->grid, h->stream)
+                                      : cudaErrorCooperativeLaunchTooLarge;
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            // not every CTA can be resident (another context holds SMs): the same micro-steps
+            // as one launch each (an empty step returns at once)
+            cudaGetLastError();
+            h->split_coop = false;
+            e = cudaSuccess;
+            for (int k = 0; k < 6 * batch && e == cudaSuccess; k++) e = launch_split_step(P, s0 + k, h->grid, h->stream);
+            *nlaunch += 6 * batch;
+        } else {
+            *nlaunch += 1;
+        }
+        if (e != cudaSuccess) return cuda_fail(h, e, "launch_split_steps");
+        CK(cudaEventRecord(h->eb1, h->stream));
+        // the micro-steps run, the recheck counts and the next step's tiles
+        CK(cudaMemcpyAsync(h->h_ctrl + 8, P.rcnt, 3 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaMemcpyAsync(h->h_ctrl + 11, P.sdone, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaMemcpyAsync(h->h_ctrl + 12, P.splan + 1 + P.G, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaMemcpyAsync(h->h_ctrl, P.ctrl, sizeof(int) * 8, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        *steps += h->h_ctrl[11];
+        s0 = (s0 + h->h_ctrl[11]) % 6;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, h->eb0, h->eb1);
+        h->stats.step_kernel_ms += ms;
+        qjx_status rs = check_ctrl(h);
+        if (rs != QJX_OK) return rs;
+        // tiles of the next step and trajectories waiting for an FP64 recheck
+        if (h->h_ctrl[12] + h->h_ctrl[8 + s0 % 3] == 0) {
+            if (h->h_ctrl[2] == 0) return QJX_OK;
+            rs = resume_paused(h);
+            if (rs != QJX_OK) return rs;
+            s0 = 0;  // the schedule wrote step 0's buckets
+            continue;
         }
         batch = std::min(batch * 2, 16);
     }
+}
+
+// Runs the trajectories that the schedule or observe kernel queued until every one is done for
+// this call.
+static qjx_status run_until_idle(qjx_engine *h)
+{
+    Params &P = h->P;
+    // QJX_TRACE_BUCKETS=<file>: append the queue sizes seen at every host poll (plain form; profiling aid)
+    FILE *bucket_log = nullptr;
+    if (const char *fn = getenv("QJX_TRACE_BUCKETS")) bucket_log = fopen(fn, "a");
+    int64_t steps = 0, nlaunch = 0;
+    long long work0[4] = {0, 0, 0, 0};
+    cudaMemcpy(work0, P.work, 4 * sizeof(long long), cudaMemcpyDeviceToHost);
+    cudaEventRecord(h->ev0, h->stream);
+    const qjx_status rs = P.split ? run_split(h, &steps, &nlaunch) : run_flow(h, bucket_log, &nlaunch);
     if (bucket_log) fclose(bucket_log);
     cudaEventRecord(h->ev1, h->stream);
     cudaEventSynchronize(h->ev1);
@@ -872,14 +955,13 @@ static qjx_status run_until_idle(qjx_engine *h)
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
     h->stats.kernel_ms += ms;
     h->stats.last_call_ms = ms;
-    h->stats.micro_steps += steps;
     h->stats.launches += nlaunch;
-    long long work1[3] = {0, 0, 0};
-    cudaMemcpy(work1, P.work, 3 * sizeof(long long), cudaMemcpyDeviceToHost);
+    long long work1[4] = {0, 0, 0, 0};
+    cudaMemcpy(work1, P.work, 4 * sizeof(long long), cudaMemcpyDeviceToHost);
+    h->stats.micro_steps += P.split ? steps : work1[3] - work0[3];
     h->stats.matvecs += work1[0] - work0[0];
     h->stats.mma_tiles += work1[1] - work0[1];
     h->stats.rechecks += work1[2] - work0[2];
-    if (exec) cudaGraphExecDestroy(exec);
     return rs;
 }
 
@@ -946,10 +1028,11 @@ extern "C" qjx_status qjx_slot_load(qjx_engine *h, int slot, const qjx_ensemble 
     const int MDe = 8 * ((d + 7) / 8), kpe = (d + 1) & ~1;
     int nc = 0, kb = 0;
     qjx_tiles ct{};
-    if (tile_cache_get(0, d, &ct) && tiles_fit(MDe, (size_t)P.step_smem, ct.nc, ct.kb)) {
+    if (tile_cache_get(0, d, &ct) && tiles_valid(MDe, ct.nc, ct.kb) &&
+        ct.nc <= max_columns(P.MD, h->flow_nt) && tiles_fit(MDe, (size_t)P.step_smem, h->flow_nt, ct.nc, &ct.kb)) {
         nc = ct.nc;  // the autotuner's choice for this dimension
         kb = ct.kb;
-    } else if (!pick_step_tiles(MDe, (size_t)P.step_smem, &nc, &kb)) {
+    } else if (!pick_step_tiles(MDe, (size_t)P.step_smem, h->flow_nt, max_columns(P.MD, h->flow_nt), &nc, &kb)) {
         return fail(h, QJX_ERR_UNSUPPORTED, "no tiling");
     }
     // operators into the slot's resident matrix region
@@ -974,8 +1057,17 @@ extern "C" qjx_status qjx_slot_load(qjx_engine *h, int slot, const qjx_ensemble 
     const long long sbase = e->tr_base;
     CK(cudaMemcpy(const_cast<int *>(P.e_d) + slot, &d, sizeof(int), cudaMemcpyHostToDevice));
     h->e_d_host[slot] = d;
-    CK(cudaMemcpy(const_cast<int *>(P.e_nc) + slot, &nc, sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(const_cast<int *>(P.e_kb) + slot, &kb, sizeof(int), cudaMemcpyHostToDevice));
+    std::vector<GroupDesc> gd(Ge);  // same rings and matrix regions
+    CK(cudaMemcpy(gd.data(), P.gd + (size_t)slot * Ge, Ge * sizeof(GroupDesc), cudaMemcpyDeviceToHost));
+    for (GroupDesc &x : gd) {
+        x.d = d;
+        x.nc = (unsigned char)nc;
+        x.kb = (unsigned char)kb;
+    }
+    std::vector<Queue> q(Ge, Queue{0, 0, 0, nc});
+    CK(cudaMemcpy(P.q + (size_t)slot * Ge, q.data(), Ge * sizeof(Queue), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(const_cast<GroupDesc *>(P.gd) + (size_t)slot * Ge, gd.data(), Ge * sizeof(GroupDesc),
+                  cudaMemcpyHostToDevice));
     CK(cudaMemcpy(const_cast<double *>(P.e_dt) + (size_t)slot * P.nb * P.deep, dts.data(),
                   dts.size() * sizeof(double), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(const_cast<double *>(P.e_rate) + (size_t)slot * P.nd, e->g, P.nd * sizeof(double),
@@ -1079,9 +1171,7 @@ extern "C" qjx_status qjx_run_periods(qjx_engine *h, int n_periods, int is_obs, 
     P.target = n_periods;
     P.subdump = subdump;
     P.record = (is_obs == 1 && h->cfg.record > 0) ? 1 : 0;
-    CK(cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream));
-    if (P.rcnt) CK(cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream));
-    CK(cudaMemsetAsync(P.ctrl, 0, sizeof(int) * 16, h->stream));
+    CK(clear_queues(h));
     P.period0 = h->period_base;
     if (P.prop == 1) CK(launch_rk_schedule(P, h->stream));
     else CK(launch_schedule(P, 0, h->stream));
@@ -1114,9 +1204,7 @@ extern "C" qjx_status qjx_run_sub_periods(qjx_engine *h, int n_sub, int dump_bas
     P.sub_target = n_sub;
     P.subdump = 1;
     P.record = h->cfg.record > 0 ? 1 : 0;
-    CK(cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream));
-    if (P.rcnt) CK(cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream));
-    CK(cudaMemsetAsync(P.ctrl, 0, sizeof(int) * 16, h->stream));
+    CK(clear_queues(h));
     P.period0 = h->period_base;
     cudaError_t e = launch_schedule(P, 2, h->stream);
     h->stats.launches += 1;
@@ -1138,9 +1226,7 @@ extern "C" qjx_status qjx_observe(qjx_engine *h, int dump, int is_start)
     P.dump_base = dump;
     P.record = 0;
     P.subdump = 0;
-    CK(cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream));
-    if (P.rcnt) CK(cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream));
-    CK(cudaMemsetAsync(P.ctrl, 0, sizeof(int) * 16, h->stream));
+    CK(clear_queues(h));
     CK(launch_observe(P, dump, is_start, h->stream));
     h->stats.launches += 1;
     return run_until_idle(h);

@@ -6,24 +6,28 @@
 // trajectory's threshold.  Jumps are frequent (about 50 per period at N = 100 and 110 at
 // N = 200), so the bisection, not the jump-free stroboscopic step, is the hot path.
 //
-// B200 design: all trajectories advance in lock-step micro-steps.  In each micro-step
-// every active trajectory needs exactly one matvec with one of G matrices (2 x ex_deep
-// propagators, the jump operators, the energy operator, the random observables).  The
-// trajectories are bucketed by matrix, and one persistent kernel per micro-step runs a
-// grouped FP64 GEMM over the buckets:
-//   * a tile is one matrix x 32 trajectory columns, full height (all d rows), so the
+// B200 design: every active trajectory needs one matvec at a time, with one of G matrices (2 x
+// ex_deep propagators, the jump operators, the energy operator, the random observables).  The
+// trajectories wait in one queue per matrix, and the CTAs of a persistent kernel are independent
+// workers: a CTA takes up to 32 trajectories from the fullest queue, multiplies them by that
+// queue's matrix, runs the state machine on each, appends each to the queue of its next matrix
+// and takes the next batch.  No CTA waits for another, so there is no lock-step, no grid barrier
+// and no plan:
+//   * a sub-tile is one matrix x 8, 16 or 32 trajectory columns, full height (all d rows), so the
 //     column norm needed by the jump test stays inside the CTA;
-//   * the gathered state columns and the propagator K-slabs are moved by the TMA engine
-//     (cp.async.bulk + mbarrier, 2-stage slab pipeline of 16 k-rows), so the tensor pipe is
-//     fed while the next slab streams from L2;
+//   * the gathered state columns and the propagator K-slabs are copied to shared memory with cp.async
+//     through a ring of stages, so the tensor pipe is fed while the next slabs stream from L2;
 //   * the epilogue is the whole trajectory state machine: norm test, descend / accept,
 //     jump record, renormalisation, channel choice, threshold redraw, time bookkeeping,
-//     period and dump accounting, the observables, and re-bucketing for the next step.
+//     period and dump accounting and the observables.
 // FP64 has no tcgen05 kind, so the plain form's contraction runs on the FP64 tensor core
 // (mma.sync m8n8k4 f64), laid out so that every output keeps the oracle's k-ascending fma
 // chain (bit-identical results).  The split-precision form (qjx_split.cuh, included at the
-// end) runs the same micro-steps with bf16x3 products on the tcgen05 tensor cores.
+// end) runs lock-step micro-steps over the same buckets with bf16x3 products on the tcgen05 tensor
+// cores.
 #include <algorithm>
+#include <atomic>
+#include <type_traits>
 
 #include "qjx_device.cuh"
 
@@ -34,6 +38,30 @@ constexpr long long kWaitLimit = 1ll << 24;  // bounded mbarrier polls before gi
 __device__ __forceinline__ double2 *slot_ptr(const Params &P, int slot, int tr)
 {
     return P.psi + ((size_t)slot * P.n + tr) * P.MD;
+}
+
+// What the state machine needs of a trajectory's ensemble: dimension, first group, split-level steps
+// [nb][deep] and jump rates.
+struct Ens {
+    int d, g0;
+    const double *dt, *rate;
+};
+
+__device__ __forceinline__ Ens global_ens(const Params &P, int e)
+{
+    return Ens{P.e_d[e], e * P.Ge, P.e_dt + (size_t)e * P.nb * P.deep, P.e_rate + (size_t)e * P.nd};
+}
+
+// The state slots of one trajectory: in P.psi, or a copy in shared memory.
+struct Slots {
+    double2 *base;
+    size_t stride;
+    __device__ __forceinline__ double2 *operator()(int slot) const { return base + slot * stride; }
+};
+
+__device__ __forceinline__ Slots global_slots(const Params &P, int tr)
+{
+    return Slots{slot_ptr(P, 0, tr), (size_t)P.n * P.MD};
 }
 
 // Whether run calls advance trajectory tr.
@@ -94,10 +122,26 @@ __device__ __forceinline__ int rk_begin(TrajState &s, double h, double prev, int
     return 0;
 }
 
-__device__ __forceinline__ void enqueue(const Params &P, int *cnt, int *list, int g, int tr)
+// Queue entry of a trajectory: its index and the slot of its next matvec's input, so that the copy
+// of the input need not wait for the trajectory's record.
+__device__ __forceinline__ unsigned entry_of(int tr, const TrajState &s)
 {
-    const int pos = atomicAdd(&cnt[g], 1);
-    list[P.g_loff[g] + pos] = tr;
+    return ((unsigned)tr << 3) | (unsigned)src_slot(s.phase, s.cur, s.rk_stage);
+}
+
+// Appends trajectory tr to bucket g before a run: the split form's lists of step 0, or the plain
+// form's queue (its entries past the tail are free).
+__device__ __forceinline__ void enqueue(const Params &P, int g, int tr)
+{
+    if (P.split) {
+        const int pos = atomicAdd(&P.cnt[g], 1);
+        P.lists[P.g_loff[g] + pos] = tr;
+    } else {
+        const unsigned pos = atomicAdd(&P.q[g].tail, 1u);
+        P.ring[P.gd[g].roff + (pos & P.gd[g].rmask())] = entry_of(tr, P.st[tr]);
+        atomicAdd(&P.q[g].avail, 1);
+        atomicAdd(P.ctrl + kLive, 1);
+    }
 }
 
 __device__ __forceinline__ void report_error(const Params &P, int tr, int code)
@@ -154,14 +198,14 @@ __device__ __forceinline__ double adr_of(double2 v, double inv)
 // the normalised state psi / sqrt(norm) written to the spare slot for the energy and
 // random-observable micro-steps.  Warp-cooperative; every lane computes the sequential
 // sums identically.
-__device__ void obs_prep(const Params &P, const TrajState &s, int tr, const double2 *col, int lane, int dump,
-                         int is_start)
+__device__ void obs_prep(const Params &P, const TrajState &s, int tr, const Ens &sys, const Slots &slots, const double2 *col, int lane,
+                         int dump, int is_start)
 {
-    const int d = dim_of(P, s);
+    const int d = sys.d;
     const double nrm = warp_norm(col, d, lane);
     const double sq = __dsqrt_rn(nrm);
     const double inv = __ddiv_rn(1.0, nrm);
-    double2 *hat = slot_ptr(P, s.cur ^ 1, tr);
+    double2 *hat = slots(s.cur ^ 1);
     double *adr_out = !P.o_adr ? nullptr
                       : (P.keep_adr ? P.o_adr + ((size_t)dump * P.n + tr) * P.d : P.o_adr + (size_t)tr * P.d);
     for (int k = lane; k < d; k += 32) {
@@ -193,18 +237,18 @@ __device__ void obs_prep(const Params &P, const TrajState &s, int tr, const doub
 
 // Continue after a completed split step: period / dump / target bookkeeping.  Returns the
 // next group, or -1 when the trajectory is done for this call.
-__device__ int after_step(const Params &P, TrajState &s, int tr, const double2 *col, int lane)
+__device__ int after_step(const Params &P, TrajState &s, int tr, const Ens &sys, const Slots &slots, const double2 *col, int lane)
 {
-    const int a = advance(s, dt_of(P, s), P.nb, P.brep);
+    const int a = advance(s, (sys.dt + s.b * P.deep), P.nb, P.brep);
     if (a == 2) s.pc += 1;
     if (a >= 1 && P.subdump && (s.rk_sid & 1) == 0) {  // deep task: a sub-period ended
-        obs_prep(P, s, tr, col, lane, P.dump_base + s.di, 0);
+        obs_prep(P, s, tr, sys, slots, col, lane, P.dump_base + s.di, 0);
         s.phase = PH_OBS_E;
         return P.gHE;
     }
     if (a == 2) {
         if (s.di < P.n_dumps && s.pc == P.dump_at[s.di]) {
-            obs_prep(P, s, tr, col, lane, P.dump_base + s.di, 0);
+            obs_prep(P, s, tr, sys, slots, col, lane, P.dump_base + s.di, 0);
             s.phase = PH_OBS_E;
             return P.gHE;
         }
@@ -233,7 +277,7 @@ __device__ int finish_obs(const Params &P, TrajState &s)
 
 // An RK step finished without crossing (rk_period, core.cpp:443-449): next step, period and dump
 // bookkeeping.  `col` holds psi, nrm its norm.
-__device__ int rk_after_step(const Params &P, TrajState &s, int tr, const double2 *col, int lane,
+__device__ int rk_after_step(const Params &P, TrajState &s, int tr, const Ens &sys, const Slots &slots, const double2 *col, int lane,
                              double nrm)
 {
     s.rk_prev = nrm;
@@ -242,7 +286,7 @@ __device__ int rk_after_step(const Params &P, TrajState &s, int tr, const double
         s.rk_sid = 0;
         s.pc += 1;
         if (s.di < P.n_dumps && s.pc == P.dump_at[s.di]) {
-            obs_prep(P, s, tr, col, lane, P.dump_base + s.di, 0);
+            obs_prep(P, s, tr, sys, slots, col, lane, P.dump_base + s.di, 0);
             s.phase = PH_OBS_E;
             return P.gHE;
         }
@@ -258,12 +302,12 @@ __device__ int rk_after_step(const Params &P, TrajState &s, int tr, const double
 // Apply the chosen jump channel: psi = (L_idx psi_hat) / sqrt(w_idx / g_idx)
 // (experiment.cpp:1346-1369), record the channel, redraw eta (qj_proc.cpp:310-314) and
 // count the finest-level step.
-__device__ int apply_jump(const Params &P, TrajState &s, int tr, double2 *col, int lane, int idx,
+__device__ int apply_jump(const Params &P, TrajState &s, int tr, const Ens &sys, const Slots &slots, double2 *col, int lane, int idx,
                           double w_idx, int *err)
 {
-    const int d = dim_of(P, s);
-    const double q = __dsqrt_rn(__ddiv_rn(w_idx, rate_of(P, s, idx)));
-    double2 *dst = slot_ptr(P, s.cur ^ 1, tr);
+    const int d = sys.d;
+    const double q = __dsqrt_rn(__ddiv_rn(w_idx, sys.rate[idx]));
+    double2 *dst = slots(s.cur ^ 1);
     for (int k = lane; k < d; k += 32) {
         const double2 v = col[k];
         const double2 r = make_double2(__ddiv_rn(v.x, q), __ddiv_rn(v.y, q));
@@ -281,16 +325,19 @@ __device__ int apply_jump(const Params &P, TrajState &s, int tr, double2 *col, i
         return rk_begin(s, s.rk_end, nrm, 0);
     }
     s.phase = PH_STEP;
-    s.t = __dadd_rn(s.t, dt_of(P, s)[P.deep - 1]);
-    return after_step(P, s, tr, col, lane);
+    s.t = __dadd_rn(s.t, (sys.dt + s.b * P.deep)[P.deep - 1]);
+    return after_step(P, s, tr, sys, slots, col, lane);
 }
 
 // Warp-cooperative epilogue of one trajectory column: `col` holds M_g * psi in shared memory,
-// `s_in` the trajectory's state record (loaded by the caller).  Returns the bucket of the
-// trajectory's next micro-step, or -1 (done, paused or failed); the caller appends it.
-__device__ int column_epilogue(const Params &P, double2 *col, int tr, const TrajState &s_in, int lane)
+// `s_in` the trajectory's state record (loaded by the caller), `sys` its ensemble, `slots` its states; the new record
+// goes to `out`.  Returns the bucket of the trajectory's next micro-step, or -1 (done, paused or
+// failed), and its queue entry in `entry`; the caller appends it.  `lead` is false in all but one of
+// several CTAs that run the same column.
+__device__ int column_epilogue(const Params &P, double2 *col, int tr, const TrajState &s_in, int lane, unsigned &entry,
+                               const Ens &sys, const Slots &slots, TrajState *out, bool lead)
 {
-    const int d = dim_of(P, s_in);
+    const int d = sys.d;
     TrajState s = s_in;
     int g2 = -1;
     int err = 0;
@@ -314,13 +361,13 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
             g2 = kRecheck;
             break;
         }
-        const double dt = dt_of(P, s)[s.lvl];
+        const double dt = (sys.dt + s.b * P.deep)[s.lvl];
         if (nrm > s.eta) {  // not crossed: accept psi' (qj_proc.cpp:317, 335)
-            double2 *dst = slot_ptr(P, s.cur ^ 1, tr);
+            double2 *dst = slots(s.cur ^ 1);
             for (int k = lane; k < d; k += 32) dst[k] = col[k];
             s.cur ^= 1;
             s.t = __dadd_rn(s.t, dt);
-            g2 = after_step(P, s, tr, col, lane);
+            g2 = after_step(P, s, tr, sys, slots, col, lane);
         } else if (s.lvl < P.deep - 1) {  // crossed on a coarse level: bisect from psi (qj_proc.cpp:328-331)
             s.lvl += 1;
             g2 = s.b * P.deep + s.lvl;
@@ -342,7 +389,7 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
             }
             // recovery: psi' /= sqrt(norm_square(psi'))  (experiment.cpp:1291-1296)
             const double sq = __dsqrt_rn(nrm);
-            double2 *dst = slot_ptr(P, s.cur ^ 1, tr);
+            double2 *dst = slots(s.cur ^ 1);
             for (int k = lane; k < d; k += 32) {
                 const double2 v = col[k];
                 dst[k] = make_double2(__ddiv_rn(v.x, sq), __ddiv_rn(v.y, sq));
@@ -359,7 +406,7 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
 
     case PH_REC_W: {  // gnorms[i] = norm_square(L_i psi_hat) * g[i]  (experiment.cpp:1301-1322)
         double w = warp_norm(col, d, lane);
-        w = __dmul_rn(w, rate_of(P, s, s.sub));
+        w = __dmul_rn(w, sys.rate[s.sub]);
         if (lane == 0) P.gn[(size_t)tr * P.nd + s.sub] = w;
         s.tmpw = __dadd_rn(s.tmpw, w);
         if (s.sub + 1 < P.nd) {
@@ -389,7 +436,7 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
         }
         if (err) break;
         if (P.nd == 1) {
-            g2 = apply_jump(P, s, tr, col, lane, index, w, &err);
+            g2 = apply_jump(P, s, tr, sys, slots, col, lane, index, w, &err);
         } else {
             s.phase = PH_REC_A;
             s.sub = index;
@@ -399,12 +446,12 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
 
     case PH_REC_A: {
         const double w = P.gn[(size_t)tr * P.nd + s.sub];
-        g2 = apply_jump(P, s, tr, col, lane, s.sub, w, &err);
+        g2 = apply_jump(P, s, tr, sys, slots, col, lane, s.sub, w, &err);
     } break;
 
     case PH_RK: {  // one right-hand side of rk_int_dimer (core.cpp:11592-11619), col = M arg
         if (s.rk_part == 0) {  // H_eff arg, kept for the drive part
-            double2 *dst = slot_ptr(P, kSlotND, tr);
+            double2 *dst = slots(kSlotND);
             for (int k = lane; k < d; k += 32) dst[k] = col[k];
             s.rk_part = 1;
             g2 = 1;
@@ -412,14 +459,14 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
         }
         // k = -i (H_eff arg + E H_drv arg)  (core.cpp:11106-11112)
         const double E = rk_drive(P, s.t);
-        const double2 *nd = slot_ptr(P, kSlotND, tr);
-        const double2 *phi = slot_ptr(P, s.cur, tr);
+        const double2 *nd = slots(kSlotND);
+        const double2 *phi = slots(s.cur);
         const double h = s.rk_h;
         if (s.rk_stage < 4) {
             // arg_upd (rk_proc.cpp:146-185) uses the full rk_step, also inside a begin or end part
             const double c = (s.rk_stage == 3) ? __dmul_rn(1.0, P.rk_step) : __dmul_rn(0.5, P.rk_step);
-            double2 *kd = slot_ptr(P, kSlotK1 + s.rk_stage - 1, tr);
-            double2 *args = slot_ptr(P, kSlotArgs, tr);
+            double2 *kd = slots(kSlotK1 + s.rk_stage - 1);
+            double2 *args = slots(kSlotArgs);
             for (int k = lane; k < d; k += 32) {
                 const double2 a = nd[k], b = col[k], x = phi[k];
                 const double kr = __dadd_rn(a.y, __dmul_rn(E, b.y)), ki = -__dadd_rn(a.x, __dmul_rn(E, b.x));
@@ -437,8 +484,8 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
             break;
         }
         // rk_final (rk_proc.cpp:187-196): psi + (k1 + 2 k2 + 2 k3 + k4) h / 6, into col
-        const double2 *k1 = slot_ptr(P, kSlotK1, tr), *k2 = slot_ptr(P, kSlotK1 + 1, tr);
-        const double2 *k3 = slot_ptr(P, kSlotK1 + 2, tr);
+        const double2 *k1 = slots(kSlotK1), *k2 = slots(kSlotK1 + 1);
+        const double2 *k3 = slots(kSlotK1 + 2);
         for (int k = lane; k < d; k += 32) {
             const double2 a = nd[k], b = col[k], x = phi[k], p1 = k1[k], p2 = k2[k], p3 = k3[k];
             const double kr = __dadd_rn(a.y, __dmul_rn(E, b.y)), ki = -__dadd_rn(a.x, __dmul_rn(E, b.x));
@@ -455,9 +502,9 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
                 break;
             }
             if (nrm > s.eta) {  // not crossed: accept psi in place
-                double2 *dst = slot_ptr(P, s.cur, tr);
+                double2 *dst = slots(s.cur);
                 for (int k = lane; k < d; k += 32) dst[k] = col[k];
-                g2 = rk_after_step(P, s, tr, col, lane, nrm);
+                g2 = rk_after_step(P, s, tr, sys, slots, col, lane, nrm);
             } else {  // crossed: integrate the begin part from psi, still in its slot (core.cpp:11913-11922)
                 const double norm_diff = __dsub_rn(s.rk_prev, nrm);
                 const double begin_part = __ddiv_rn(__dsub_rn(s.rk_prev, s.eta), norm_diff);
@@ -479,7 +526,7 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
                 s.jumps += 1;
             }
             const double sq = __dsqrt_rn(nrm);
-            double2 *dst = slot_ptr(P, s.cur ^ 1, tr);
+            double2 *dst = slots(s.cur ^ 1);
             for (int k = lane; k < d; k += 32) {
                 const double2 v = col[k];
                 dst[k] = make_double2(__ddiv_rn(v.x, sq), __ddiv_rn(v.y, sq));
@@ -495,7 +542,7 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
     } break;
 
     case PH_OBS_E: {  // energy <psi_hat| H + E0 Hd |psi_hat>  (experiment.cpp:1423-1469)
-        const double2 *hat = slot_ptr(P, s.cur ^ 1, tr);
+        const double2 *hat = slots(s.cur ^ 1);
         double e = 0.0;
         for (int k = lane; k < d; k += 32) {
             const double2 h = hat[k], m = col[k];
@@ -514,7 +561,7 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
     } break;
 
     case PH_OBS_R: {  // <psi_hat| R |psi_hat>  (experiment.cpp:2037-2068)
-        const double2 *hat = slot_ptr(P, s.cur ^ 1, tr);
+        const double2 *hat = slots(s.cur ^ 1);
         double rr = 0.0, ri = 0.0;
         for (int k = lane; k < d; k += 32) {
             const double2 h = hat[k], m = col[k];
@@ -544,38 +591,20 @@ __device__ int column_epilogue(const Params &P, double2 *col, int tr, const Traj
         if (err) {
             s.err = err;
             s.phase = PH_ERROR;
-            report_error(P, tr, err);
+            if (lead) report_error(P, tr, err);
         } else if (paused) {
             s.paused = 1;
-            atomicAdd(&P.ctrl[2], 1);
+            if (lead) atomicAdd(&P.ctrl[2], 1);
         }
-        P.st[tr] = s;
+        *out = s;
     }
     __syncwarp();
+    entry = entry_of(tr, s);
     if (to_recheck) return kRecheck;
-    return g2 >= 0 ? P.e_g0[s.ens] + g2 : -1;  // local group -> the ensemble's bucket
+    return g2 >= 0 ? sys.g0 + g2 : -1;  // local group -> the ensemble's bucket
 }
 
-// Appends trajectories trs[c] to their next buckets g2s[c] (c < ncol, -1 skips) with one global
-// atomic per distinct bucket of each 32 columns: warp w takes columns 32w .. 32w + 31, lanes
-// with the same bucket find each other with __match_any_sync, the lowest reserves the run and
-// the others take consecutive slots in lane order.  Independent of the number of groups.
-__device__ void enqueue_batch(const Params &P, int *cnt_next, int *list_next, const int *trs, const int *g2s, int ncol)
-{
-    const int lane = threadIdx.x & 31;
-    for (int c0 = (threadIdx.x >> 5) * 32; c0 < ncol; c0 += blockDim.x) {
-        const int c = c0 + lane;
-        const int g = (c < ncol) ? g2s[c] : -1;
-        const unsigned m = __match_any_sync(0xffffffffu, g);
-        const int leader = __ffs(m) - 1;
-        int base = 0;
-        if (g >= 0 && lane == leader) base = atomicAdd(&cnt_next[g], __popc(m));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (g >= 0) list_next[P.g_loff[g] + base + __popc(m & ((1u << lane) - 1u))] = trs[c];
-    }
-}
-
-// Copies a 96-byte trajectory record with 16-byte accesses.
+// Copies a 144-byte trajectory record with 16-byte accesses.
 __device__ __forceinline__ void load_state(TrajState *dst, const TrajState *src)
 {
     const uint4 *s = reinterpret_cast<const uint4 *>(src);
@@ -584,11 +613,6 @@ __device__ __forceinline__ void load_state(TrajState *dst, const TrajState *src)
     for (int i = 0; i < (int)(sizeof(TrajState) / 16); i++) t[i] = s[i];
 }
 
-// Accumulates M_g * B for one sub-tile of NTE x TX columns (all rows), streaming the
-// propagator in K-slabs through the TMA pipeline, then stages the result in Bt.
-// Per output the k-ascending fma chain of the oracle is kept; within one k the four fmas
-// are issued in two passes (re += Mr xr, im += Mr xi for every output, then re -= Mi xi,
-// im += Mi xr), which leaves each chain's order unchanged.
 __device__ __forceinline__ double neg(double x)
 {
     return __longlong_as_double(__double_as_longlong(x) ^ (long long)0x8000000000000000ull);
@@ -600,366 +624,687 @@ __device__ __forceinline__ double neg(double x)
 // oracle's per-output k-ascending order.
 __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b)
 {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(c0), "+d"(c1)
+        : "d"(a), "d"(b));
+}
+
+// 16 bytes global -> shared (past L1), asynchronously; zeros where !valid (the address is not read then).
+__device__ __forceinline__ void cp16(double2 *dst, const double2 *src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void cp_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Starts the copy of slab `sl` (KS k rows from KS sl on; nothing past the last) into its half of the
+// slab buffer, as one group of this thread.
+template <int NT>
+__device__ __forceinline__ void load_slab(const double2 *mat, double2 *Us, int sl, int kp, int KS, int MD)
+{
+    const int n = min(KS, kp - sl * KS) * MD;
+    double2 *dst = Us + (sl & 1) * KS * MD;
+    const double2 *src = mat + (size_t)sl * KS * MD;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += NT) cp16(dst + i, src + i, true);
+    cp_commit();
 }
 
 // Complex sub-tile product on the FP64 tensor core.  Rows are in 8-row blocks (RB of them,
-// MD = 8 RB), columns in 8-column blocks (CB active of 4).  For one pair of complex k the
-// real parts use A = [Mr_k, -Mi_k, Mr_k+1, -Mi_k+1] against B = [xr_k; xi_k; xr_k+1; xi_k+1]
-// and the imaginary parts A = [Mr_k, Mi_k, ...] against B = [xi_k; xr_k; ...]; that is the
-// k-ascending chain re += Mr xr; re -= Mi xi; im += Mr xi; im += Mi xr of the contract.
+// MD = 8 RB), columns in 8-column blocks.  For one pair of complex k the real parts use
+// A = [Mr_k, Mi_k, Mr_k+1, Mi_k+1] against B = [xr_k; -xi_k; xr_k+1; -xi_k+1] and the imaginary
+// parts the same A against B = [xi_k; xr_k; ...]; that is the k-ascending chain re += Mr xr;
+// re -= Mi xi; im += Mr xi; im += Mi xr of the contract (the sign of a product is exact).  With
+// the matrix as [k / 2][row][k % 2], lane l's A operand of row block rb is double 32 rb + l of the
+// k pair: one conflict-free 256-byte read per warp and row block, no sign or select on the A side.
+// (The layout [k][row] before it put the two k of a pair on the same banks: 4 shared-memory
+// wavefronts a read instead of 2, about half of the pipe at d = 201.)
+// The K-slabs (KS rows each, even) come through two buffers by cp.async; the caller has started the
+// first.
 // WPC warps share one column block; warp `sub` of them owns row blocks sub, sub + WPC, ...
-template <int NRB, int WPC>
-__device__ __forceinline__ bool tile_dmma(const double2 *mat, double2 *Bt, double2 *Us, uint64_t *bar,
-                                          int *released, uint32_t &phase, int d, int kp, int KB, int RB, int MD,
-                                          int S16, int warp, int lane, int tid)
+//
+// tile_rows: the share of a warp with exactly N row blocks, two k pairs at a time, their operands read
+// together ahead of the MMAs.  With only two to four warps on a scheduler it is the instructions
+// between the MMAs that cost: a test of the row block around each MMA, a slab of two k pairs with its
+// barrier or mbarrier, a counter of warps per stage.  (A lone 8-column sub-tile of d = 201 took 56k
+// cycles with those, against 21k of tensor pipe.)
+template <int N, int WPC, int NT>
+__device__ __forceinline__ void tile_rows(const double2 *mat, double2 *Bt, double2 *Us, int d, int kp, int KS, int MD,
+                                          int S16, int cb, int sub, int lane)
 {
-    const int g = lane >> 2, t = lane & 3;
-    // warp w runs on scheduler w % 4; rotating the row-block index by column block gives
-    // each scheduler the same number of row blocks
-    const int cb = warp / WPC, sub = (warp % WPC + cb * (WPC / 4)) % WPC;
-    const int th = t >> 1, todd = t & 1;
-    const int nslab = (kp + KB - 1) / KB;
-    bool ok = true;
-    double re[NRB][2], im[NRB][2];
+    constexpr int NA = N > 0 ? N : 1;
+    const int g = lane >> 2, t = lane & 3, todd = t & 1;
+    double re[NA][2], im[NA][2];
 #pragma unroll
-    for (int i = 0; i < NRB; i++) re[i][0] = re[i][1] = im[i][0] = im[i][1] = 0.0;
-
-    if (!mbar_wait_bounded(&bar[kStages], (phase >> kStages) & 1u, kWaitLimit)) ok = false;
-    phase ^= 1u << kStages;
-    const double2 *bcol = Bt + (8 * cb + g) * S16;
+    for (int i = 0; i < NA; i++) re[i][0] = re[i][1] = im[i][0] = im[i][1] = 0.0;
+    auto mma = [&](const double (&v)[NA], const double2 &x) {
+        const double bre = todd ? neg(x.y) : x.x, bim = todd ? x.x : x.y;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            dmma(re[i][0], re[i][1], v[i], bre);
+            dmma(im[i][0], im[i][1], v[i], bim);
+        }
+    };
+    const double2 *b = Bt + (8 * cb + g) * S16 + (t >> 1);
+    const size_t astep = 4 * (size_t)MD;
+    const int nslab = (kp + KS - 1) / KS;
+#pragma unroll 1
     for (int sl = 0; sl < nslab; sl++) {
-        const int q = sl % kStages;
-        if (!mbar_wait_bounded(&bar[q], (phase >> q) & 1u, kWaitLimit)) ok = false;
-        phase ^= 1u << q;
-        const int k0 = sl * KB;
-        const int kc = min(KB, kp - k0);  // even
-        const double *Uq = reinterpret_cast<const double *>(Us + q * KB * MD);
-#pragma unroll 2
-        for (int kk = 0; kk < kc; kk += 2) {
-            const double2 xb = bcol[k0 + kk + th];
-            const double bre = todd ? xb.y : xb.x;
-            const double bim = todd ? xb.x : xb.y;
-            const double *urow = Uq + 2 * (size_t)(kk + th) * MD + todd;
+        cp_wait<0>();
+        __syncthreads();  // slab sl (and the columns) has landed for every thread, and no one reads the other buffer
+        const int nk = min(KS, kp - sl * KS) / 2;
+        const double *a = reinterpret_cast<const double *>(Us + (sl & 1) * KS * MD) + 32 * sub + lane;
+        auto pairs = [&](int k0, int k1) {  // k pairs k0 .. k1 of the slab
+            if constexpr (N > 0) {
+                int k = k0;
+#pragma unroll 1
+                for (; k + 2 <= k1; k += 2, a += 2 * astep, b += 4) {
+                    const double2 x0 = b[0], x1 = b[2];
+                    double v0[NA], v1[NA];
 #pragma unroll
-            for (int i = 0; i < NRB; i++) {
-                const int rb = sub + WPC * i;
-                if (rb < RB) {
-                    const double v = urow[2 * (8 * rb + g)];
-                    dmma(re[i][0], re[i][1], todd ? neg(v) : v, bre);
-                    dmma(im[i][0], im[i][1], v, bim);
+                    for (int i = 0; i < N; i++) v0[i] = a[32 * WPC * i];
+#pragma unroll
+                    for (int i = 0; i < N; i++) v1[i] = a[astep + 32 * WPC * i];
+                    mma(v0, x0);
+                    mma(v1, x1);
+                }
+                if (k < k1) {
+                    const double2 x0 = b[0];
+                    double v0[NA];
+#pragma unroll
+                    for (int i = 0; i < N; i++) v0[i] = a[32 * WPC * i];
+                    mma(v0, x0);
+                    b += 2;
                 }
             }
-        }
-        // release the stage: the last of the 16 warps to finish it issues the refill, so no
-        // warp waits for another's release (no CTA-wide barrier per slab)
-        __syncwarp();
-        if (lane == 0 && sl + kStages < nslab) {
-            __threadfence_block();
-            if (atomicAdd(&released[q], 1) == kThreads / 32 - 1) {
-                released[q] = 0;
-                const int sn = sl + kStages;
-                const int kn = min(KB, kp - sn * KB);
-                fence_proxy_async();
-                mbar_expect_tx(&bar[q], (uint32_t)(kn * MD * 16));
-                bulk_g2s(Us + q * KB * MD, mat + (size_t)sn * KB * MD, (uint32_t)(kn * MD * 16), &bar[q]);
-            }
-        }
-        __syncwarp();  // lanes 1-31 wait here, not spinning on the next slab beside the issuing lane
+        };
+        // the next slab's copies are issued while the first k pair's MMAs run
+        const int first = min(nk, 1);
+        pairs(0, first);
+        a = reinterpret_cast<const double *>(Us + (sl & 1) * KS * MD) + 32 * sub + lane + first * astep;
+        load_slab<NT>(mat, Us, sl + 1, kp, KS, MD);
+        pairs(first, nk);
     }
     __syncthreads();
     // stage: thread (g, t) of row block rb holds rows 8 rb + g, columns 8 cb + 2t, 8 cb + 2t + 1
 #pragma unroll
-    for (int i = 0; i < NRB; i++) {
-        const int rb = sub + WPC * i;
-        const int row = 8 * rb + g;
-        if (rb < RB && row < d) {
+    for (int i = 0; i < N; i++) {
+        const int row = 8 * (sub + WPC * i) + g;
+        if (row < d) {
             Bt[(8 * cb + 2 * t) * S16 + row] = make_double2(re[i][0], im[i][0]);
             Bt[(8 * cb + 2 * t + 1) * S16 + row] = make_double2(re[i][1], im[i][1]);
         }
     }
-    return ok;
 }
 
-// Estimated cost of a bucket of m columns cut into sub-tiles the way the kernel cuts them
-// (32-column chunks; a rest of 17..24 columns as 16 + rest), in units of ~5k cycles: 2 per
-// sub-tile (gather, epilogue), 6 per active 8-column block (MMA loop), and 3 more per
-// sub-tile of the jump-operator and observable buckets, whose epilogues renormalise, draw
-// and reduce.
-// Columns of the next sub-tile of a bucket piece of m columns: with 32-column sub-tiles a rest
-// of 17..24 columns is cut as 16 + rest (no sub-tile of 3 column blocks); narrower sub-tiles
-// (large d) take min(m, NC).
-__device__ __forceinline__ int subtile_cols(int m, int NC)
+template <int NRB, int WPC, int NT>
+__device__ __forceinline__ void tile_dmma(const double2 *mat, double2 *Bt, double2 *Us, int d, int kp, int KS, int RB,
+                                          int S16, int warp, int lane)
 {
-    if (NC == kNC) return (m > 24) ? min(m, kNC) : (m > 16 ? 16 : m);
-    return min(m, NC);
-}
-
-__device__ __forceinline__ int subtile_cost(int m, int NC, int u_sub, int u_blk, int u_col4)
-{
-    int c = 0;
-    while (m > 0) {
-        const int s = subtile_cols(m, NC);
-        const int cb = (s + 7) / 8;
-        c += u_sub + u_blk * ((cb == 3) ? 4 : cb) + (s * u_col4) / 4;
-        m -= s;
+    // warp w runs on scheduler w % 4; rotating the row-block index by column block gives each
+    // scheduler the same number of row blocks (two column blocks of four warps: by half a turn)
+    const int cb = warp / WPC, sub = (warp % WPC + cb * WPC / (NT == 256 && WPC == 4 ? 2 : 4)) % WPC;
+    const int nr = RB > sub ? (RB - sub + WPC - 1) / WPC : 0;  // this warp's row blocks (at most NRB)
+    auto rows = [&](auto count) {
+        constexpr int N = decltype(count)::value;
+        if constexpr (N <= NRB) tile_rows<N, WPC, NT>(mat, Bt, Us, d, kp, KS, 8 * RB, S16, cb, sub, lane);
+    };
+    switch (nr) {
+    case 1: rows(std::integral_constant<int, 1>()); break;
+    case 2: rows(std::integral_constant<int, 2>()); break;
+    case 3: rows(std::integral_constant<int, 3>()); break;
+    case 4: rows(std::integral_constant<int, 4>()); break;
+    case 5: rows(std::integral_constant<int, 5>()); break;
+    case 6: rows(std::integral_constant<int, 6>()); break;
+    case 7: rows(std::integral_constant<int, 7>()); break;
+    case 8: rows(std::integral_constant<int, 8>()); break;
+    default: rows(std::integral_constant<int, 0>()); break;
     }
-    return c;
 }
 
-// Estimated cost of group g's bucket of m columns, in units of 0.25 us at d = 201, fitted to the
-// busy time of every CTA in 512 full micro-steps of the headline ensemble against the work it
-// got (least squares, 1.9 us rms): 7.8 us per sub-tile (gather, slab pipeline fill, epilogue
-// passes), 15.0 us per active 8-column block (MMA loop), 0.06 us per column and 0.15 us more per
-// column of the jump-operator and observable buckets (their epilogues renormalise, draw and
-// reduce); scaled to the group's dimension (epilogue ~ d, MMA ~ row blocks x k rows).
-__device__ __forceinline__ int group_cost(const Params &P, int g, int m)
+// Starts the copies of column c of a sub-tile (trajectory and slot of entry `en`) and its record (one
+// warp; no group is committed).
+__device__ __forceinline__ void stage_column(const Params &P, unsigned en, int kp, double2 *col, TrajState *st, int lane)
 {
-    if (m == 0) return 0;
-    const int e = P.g_ens[g], d = P.e_d[e];
-    const bool heavy = g - P.e_g0[e] >= P.gL0;
-    const int u_sub = max(1, (31 * d + 100) / 201);
-    const int u_blk = max(1, (((d + 7) >> 3) * ((d + 1) & ~1) * 60 + 2626) / 5252);
-    const int u_col4 = max(1, ((heavy ? 7 : 2) * d + 200) / 402);
-    return subtile_cost(m, P.e_nc[e], u_sub, u_blk, u_col4);
+    const int tr = (int)(en >> 3);
+    const double2 *src = slot_ptr(P, (int)(en & 7u), tr);
+    for (int k = lane; k < kp; k += 32) cp16(col + k, src + k, true);
+    if (lane < (int)(sizeof(TrajState) / 16))
+        cp16(reinterpret_cast<double2 *>(st) + lane, reinterpret_cast<const double2 *>(&P.st[tr]) + lane, true);
 }
 
-// Plan of a micro-step from its bucket sizes cnt[G]: bucket starts plan[0..G] and cost prefix
-// plan[G+1..2G+1].  Block-wide (any multiple of 32 threads); reads cnt past L1 (its atomics
-// were made by other CTAs).
-__device__ void plan_scan(const Params &P, const int *cnt)
+__device__ __forceinline__ unsigned long long global_ns()
 {
-    __shared__ int w_c[32], w_k[32];
-    const int G = P.G, nt = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int per = (G + nt - 1) / nt;
-    const int g0 = min(G, tid * per), g1 = min(G, g0 + per);
-    int c = 0, k = 0;
-    for (int g = g0; g < g1; g++) {
-        const int m = __ldcg(cnt + g);
-        c += m;
-        k += group_cost(P, g, m);
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+// What a CTA has done, kept in shared memory by one thread: matvecs, sub-tiles and (for
+// qjx_set_trace) clock64 cycles per part.
+struct Tally {
+    long long begin, work, subtiles, blocks, setup, claim, loop, epi;
+    __device__ void reset()
+    {
+        begin = clock64();
+        work = subtiles = blocks = setup = claim = loop = epi = 0;
     }
-    int ic = c, ik = k;  // inclusive warp scans
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int yc = __shfl_up_sync(0xffffffffu, ic, off), yk = __shfl_up_sync(0xffffffffu, ik, off);
-        if (lane >= off) {
-            ic += yc;
-            ik += yk;
+    // a sub-tile of n columns in nb 8-column blocks: taken at t0, staged at t1, product done at t2,
+    // epilogue at t3
+    __device__ void add(int n, int nb, long long t0, long long t1, long long t2, long long t3)
+    {
+        work += n;
+        subtiles += 1;
+        blocks += nb;
+        setup += t1 - t0;
+        loop += t2 - t1;
+        epi += t3 - t2;
+    }
+    __device__ void flush(const Params &P) const
+    {
+        if (work) {
+            atomicAdd((unsigned long long *)P.work, (unsigned long long)work);
+            atomicAdd((unsigned long long *)(P.work + 3), (unsigned long long)subtiles);
         }
+        if (!P.trace) return;
+        const long long v[kTraceFields] = {clock64() - begin, setup, claim, loop, epi, subtiles, blocks, work};
+        long long *t = P.trace + (size_t)(blockIdx.x % P.grid) * kTraceFields;
+        for (int i = 0; i < kTraceFields; i++) atomicAdd((unsigned long long *)(t + i), (unsigned long long)v[i]);
     }
-    if (lane == 31) {
-        w_c[warp] = ic;
-        w_k[warp] = ik;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = nt >> 5;
-        int vc = lane < nw ? w_c[lane] : 0, vk = lane < nw ? w_k[lane] : 0;
+};
+
+// A queue to take from and how many trajectories: 0 when all are empty, -1 when the call is done
+// (at most stop_live trajectories left).
+struct Pick {
+    int n, g;
+};
+
+// Looks the queues over (one warp, converged): a claim is at most NCM trajectories and an equal share
+// of the unfinished ones in whole 8-column blocks (NCM = 1: one trajectory).  Any queue that has the
+// share waiting will do (a different one for each CTA and attempt, so that claims spread), else the
+// fullest.  Queues are scanned 256 at a time from a place that differs by CTA, up to the first 256
+// with a share waiting.
+template <int NCM>
+__device__ __forceinline__ Pick scan(const Params &P, int stop_live, unsigned &turn, int lane)
+{
+    const int G = P.G, chunks = (G + 255) / 256;
+    turn += 7u;
+    const int live = __ldcg(P.ctrl + kLive);
+    int share = NCM;
+    Pick pick{0, 0};
+    for (int c = 0; c < chunks && pick.n < share; c++) {
+        const int base = 256 * (int)((c + turn) % (unsigned)chunks);
+        int av[8], cap[8];
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int yc = __shfl_up_sync(0xffffffffu, vc, off), yk = __shfl_up_sync(0xffffffffu, vk, off);
-            if (lane >= off) {
-                vc += yc;
-                vk += yk;
+        for (int i = 0; i < 8; i++) {
+            const int gi = base + 32 * i + lane;
+            av[i] = cap[i] = 0;
+            if (gi < G) {
+                const int4 v = __ldcg(reinterpret_cast<const int4 *>(P.q) + gi);
+                av[i] = v.x;
+                cap[i] = v.w;
             }
         }
-        if (lane < nw) {
-            w_c[lane] = vc;  // inclusive totals through warp `lane`
-            w_k[lane] = vk;
+        share = min(NCM, 8 * ((live + 8 * (int)gridDim.x - 1) / (8 * (int)gridDim.x)));
+        int b = 0, bi = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int a = min(av[i], min(share, cap[i]));
+            if (a > b) {
+                b = a;
+                bi = base + 32 * i + lane;
+            }
+        }
+        const int m = __reduce_max_sync(0xffffffffu, b);
+        if (m > pick.n) {
+            const unsigned who = __ballot_sync(0xffffffffu, b == m);
+            const int r = turn & 31;
+            pick.n = m;
+            pick.g = __shfl_sync(0xffffffffu, bi, (__ffs(__funnelshift_r(who, who, r)) - 1 + r) & 31);
         }
     }
-    __syncthreads();
-    int cs = ic - c + (warp ? w_c[warp - 1] : 0), ks = ik - k + (warp ? w_k[warp - 1] : 0);
-    for (int g = g0; g < g1; g++) {
-        const int m = __ldcg(cnt + g);
-        P.plan[g] = cs;
-        P.plan[G + 1 + g] = ks;
-        cs += m;
-        ks += group_cost(P, g, m);
-    }
-    if (tid == nt - 1) {
-        P.plan[G] = cs;
-        P.plan[2 * G + 1] = ks;
-    }
-    __syncthreads();
+    if (live <= stop_live) pick.n = -1;
+    return pick;
 }
 
-// Column position of cost offset k (monotone in k) in a plan.
-__device__ __forceinline__ int cost_to_column(const int *cstart, const int *kc, int G, long long k)
+// Takes trajectories from a queue (one warp, converged), from `pick` first if that has any: lane
+// i < n gets the i-th entry in `en`, gd the queue's descriptor.  Returns n, or 0: the call's work is
+// done, the slice is over, or nothing turned up for kIdleNs.  A claim is two atomics that cannot
+// fail (a claim by compare-and-swap of the head, before, was lost to another CTA four times in five
+// at d = 51): what the count of available entries grants, then as many positions.  What was written
+// about the trajectories before their entries is visible to this SM afterwards.
+template <int NCM>
+__device__ __forceinline__ int take(const Params &P, unsigned long long t_end, int stop_live, Pick pick, unsigned &turn,
+                                    int lane, GroupDesc &gd, unsigned &en)
 {
-    if (k >= kc[G]) return cstart[G];
-    int lo = 0, hi = G;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (kc[mid] <= k) lo = mid;
-        else hi = mid;
+    // a queue that others have nearly emptied since it was looked at is passed over this many times:
+    // a sub-tile of a few columns costs as much tensor time as a full block of eight
+    constexpr int kTries = 2;
+    unsigned long long t_idle = 0;
+    int n = 0, tries = 0;
+    unsigned pos = 0;
+    en = kFree;
+    while (true) {
+        if (pick.n == 0) pick = scan<NCM>(P, stop_live, turn, lane);
+        const unsigned long long now = global_ns();
+        if (pick.n < 0 || now >= t_end) return 0;
+        if (pick.n > 0) {
+            gd = load_desc(P.gd + pick.g);
+            if (lane == 0) {
+                Queue *q = P.q + pick.g;
+                const int want = (pick.n > 16 && pick.n <= 24) ? 16 : pick.n;  // no sub-tile of 3 column blocks
+                n = max(0, min(want, atomicSub(&q->avail, want)));
+                if (n > 16 && n <= 24) n = 16;
+                if (4 * n < 3 * want && tries < kTries) n = 0;
+                if (n < want) atomicAdd(&q->avail, want - n);
+                if (n > 0) pos = atomicAdd(&q->head, (unsigned)n);
+            }
+            n = __shfl_sync(0xffffffffu, n, 0);
+            if (n > 0) break;
+            pick.n = 0;  // other CTAs took them: look again
+            tries++;
+            continue;
+        }
+        if (t_idle == 0) t_idle = now + kIdleNs;
+        else if (now >= t_idle) return 0;
+        __nanosleep(50);
     }
-    const int cnt = cstart[lo + 1] - cstart[lo];
-    const int cost = kc[lo + 1] - kc[lo];
-    if (cost <= 0) return cstart[lo];
-    const long long off = (k - kc[lo]) * (long long)cnt / cost;
-    const int col = (int)min((long long)cnt, ((off + 4) / 8) * 8);
-    return cstart[lo] + col;
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    if (lane < n) {
+        unsigned *entry = P.ring + gd.roff + ((pos + (unsigned)lane) & gd.rmask());
+        for (long long i = 0; i < kWaitLimit && en == kFree; i++) en = atomicExch(entry, kFree);
+    }
+    __threadfence();  // acquire
+    if (__any_sync(0xffffffffu, lane < n && en == kFree)) {  // never published: report and stop
+        if (lane == 0) {
+            atomicAdd(&P.ctrl[4], 1);
+            report_error(P, -1, ERR_TIMEOUT);
+        }
+        return 0;
+    }
+    return n;
 }
 
-// One lock-step micro-step: grouped complex GEMM over the buckets of step `s` on the FP64
-// tensor core, with the fused epilogue.  The concatenated bucket lists (C columns) are split
-// into equal column ranges, one per persistent CTA; each range is processed as sub-tiles of
-// at most 32 columns of one matrix, and a sub-tile costs in proportion to its active 8-column
-// blocks (1, 2 or 4): the warps are spread over the row blocks of the active column blocks.
-// Each ensemble has its own sub-tile width (32, 16 or 8 columns) and slab height; the shared
-// memory holds the staged columns (stride MD + 1, odd: conflict-free column reads) followed by
-// the propagator slabs, laid out per sub-tile.  R4, R2, R1: row blocks per warp of the sub-tiles
-// with 4, 2 and 1 column blocks (4, 8 and 16 warps per column block), large enough for every
-// ensemble that uses them.
-template <int R4, int R2, int R1>
-__global__ void __launch_bounds__(kThreads, 1) step_kernel(const Params P, int s)
+// Appends trajectories to their next queues (one warp, converged): lane i < n has the bucket g2 and
+// the entry `en` of one, -1 when it is finished, paused or failed.  Lanes with the same bucket find
+// each other, the lowest reserves the run.
+__device__ void append(const Params &P, int g2, unsigned en, int n, int lane)
 {
+    __threadfence();  // release: what the CTA wrote, before the entries
+    const unsigned m = __match_any_sync(0xffffffffu, g2);
+    const int leader = __ffs(m) - 1;
+    GroupDesc gd{};
+    if (g2 >= 0) gd = load_desc(P.gd + g2);
+    unsigned base = 0;
+    if (lane == leader) {
+        if (g2 >= 0) {
+            base = atomicAdd(&P.q[g2].tail, (unsigned)__popc(m));
+            atomicAdd(&P.q[g2].avail, __popc(m));
+        } else {
+            const int gone = __popc(m) - (32 - n);  // lanes past n are in this set too
+            if (gone > 0) atomicSub(P.ctrl + kLive, gone);
+        }
+    }
+    base = __shfl_sync(0xffffffffu, base, leader);
+    bool put = g2 < 0;
+    unsigned *entry = P.ring + gd.roff + ((base + (unsigned)__popc(m & ((1u << lane) - 1u))) & gd.rmask());
+    for (long long i = 0; i < kWaitLimit && !put; i++) put = atomicCAS(entry, kFree, en) == kFree;
+    if (!put) {
+        atomicAdd(&P.ctrl[4], 1);
+        report_error(P, -1, ERR_TIMEOUT);
+    }
+    __syncwarp();
+}
+
+// The plain form's persistent kernel: every CTA takes sub-tiles from the queues until the call's
+// trajectories are done, its time slice ends or it finds nothing to do for a while.  A CTA never
+// waits for work of another (a trajectory that is neither queued nor finished is in a running
+// CTA's sub-tile, and that CTA scans the queues again after appending it), so CTAs need not be
+// co-resident and may leave at any time; the host launches again while trajectories are left.
+// The only waits are for an entry that a running CTA has reserved and is about to write or take
+// (bounded).  A queue is a ring of entries with a head and a tail count; it never holds
+// more than the ensemble's trajectories, and a trajectory is in one place at a time.
+// Results do not depend on which trajectories share a sub-tile: a column's arithmetic involves
+// that column only.
+//
+// What bounds it: the FP64 tensor pipe (8 d^2 flop per column).  Two CTAs of 256 threads per SM
+// while both fit the shared memory (16-column sub-tiles, d <= ~240), so one CTA's scan, gather and
+// epilogue overlap the other's products; one CTA of 512 threads (32, 16 or 8 columns) above that.
+// R4, R2, R1: row blocks per warp of the sub-tiles whose column blocks are shared by 4 warps, by
+// 8 and by 16 (512 threads) or 2 (256 threads, 32-column sub-tiles; 0: none wider than 16).
+template <int NT, int R4, int R2, int R1>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) flow_kernel(const Params P, int stop_live)
+{
+    constexpr int NW = NT / 32, NCM = (NT == 512 || R1 > 0) ? 32 : 16;
     extern __shared__ __align__(128) unsigned char smem[];
     double2 *Bt = reinterpret_cast<double2 *>(smem);
-    __shared__ __align__(8) uint64_t bar[kStages + 1];
-    __shared__ int released[kStages];
-    __shared__ int s_tr[kNC];
-    __shared__ long long s_src[kNC];
-    __shared__ __align__(16) TrajState s_st[kNC];
-    __shared__ int s_g2[kNC];
-    __shared__ int s_last;
+    __shared__ __align__(16) TrajState s_st[NCM];
+    __shared__ int s_g2[NCM];
+    __shared__ unsigned s_in[NCM], s_entry[NCM];
+    __shared__ __align__(16) GroupDesc s_gd;
+    __shared__ int s_n;
+    __shared__ double s_dt[kMaxDt];
+    __shared__ Tally tally;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int G = P.G, n = P.n;
-    int *cnt_next = P.cnt + ((s + 1) % 3) * G;
-    const int *list_cur = P.lists + (size_t)(s & 1) * P.ltot;
-    int *list_next = P.lists + (size_t)((s + 1) & 1) * P.ltot;
-    const int *cstart = P.plan, *kc = P.plan + G + 1;  // this step's plan
-
-    if (blockIdx.x == 0)
-        for (int i = tid; i < G; i += kThreads) P.cnt[((s + 2) % 3) * G + i] = 0;
-    if (tid == 0) {
-        for (int q = 0; q <= kStages; q++) mbar_init(&bar[q], 1);
-        for (int q = 0; q < kStages; q++) released[q] = 0;
-    }
-    __syncthreads();
-    // equal shares of the estimated cost, mapped back to column positions (8-column aligned
-    // inside each bucket): buckets that split into many narrow sub-tiles get shorter ranges
-    const long long K = kc[G];
-    const int c_lo = cost_to_column(cstart, kc, G, K * blockIdx.x / gridDim.x);
-    const int c_hi = cost_to_column(cstart, kc, G, K * (blockIdx.x + 1) / gridDim.x);
-    uint32_t phase = 0;
-    long long work = 0;
-    long long tr_setup = 0, tr_loop = 0, tr_epi = 0, tr_sub = 0, tr_cb = 0;
-    const long long t_begin = clock64();
-
-    for (int pos = c_lo; pos < c_hi;) {
+    if (tid == 0) tally.reset();
+    const unsigned long long t_end = global_ns() + kSliceNs;
+    unsigned turn = blockIdx.x;
+    Pick hint{0, 0};  // (warp 0) the next claim, looked for while the sub-tile before was being staged
+    while (true) {
         const long long t0 = clock64();
-        int lo = 0, hi = G;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (cstart[mid] <= pos) lo = mid;
-            else hi = mid;
+        if (warp == 0) {
+            GroupDesc gd{};
+            unsigned en = kFree;
+            const int n = take<NCM>(P, t_end, stop_live, hint, turn, lane, gd, en);
+            if (lane < NCM) s_in[lane] = en;
+            if (lane == 0) {
+                tally.claim += clock64() - t0;
+                s_gd = gd;
+                s_n = n;
+            }
         }
-        const int g = lo;
-        const int idx = pos - cstart[g];
+        __syncthreads();
+        const int ncol = s_n;
+        if (ncol <= 0) break;
         // the group's matrix: its ensemble's dimension, padded rows, k rows and tiling
-        const int eg = P.g_ens[g];
-        const int dg = P.e_d[eg];
-        const int MD = 8 * ((dg + 7) / 8), RB = MD / 8, kp = (dg + 1) & ~1;
-        const int S16 = MD + 1, KB = P.e_kb[eg], NC = P.e_nc[eg];
-        double2 *Us = Bt + NC * S16;
-        const int nslab = (kp + KB - 1) / KB;
-        // piece of this group left in the range, cut so that no sub-tile has 3 column blocks
-        const int m = min(c_hi - pos, cstart[g + 1] - pos);
-        const int ncol = subtile_cols(m, NC);
+        const int dg = s_gd.d, MD = 8 * ((dg + 7) / 8), RB = MD / 8, kp = (dg + 1) & ~1, S16 = MD + kColPad;
+        const int KS = s_gd.kb;
+        double2 *Us = Bt + s_gd.nc * S16;
+        const double2 *mat = P.mats + s_gd.moff;
         const int ncb = (ncol + 7) / 8;
-        if (tid < kNC) {
-            if (tid < ncol) {
-                const int tr = list_cur[P.g_loff[g] + idx + tid];
-                load_state(&s_st[tid], &P.st[tr]);
-                const int slot = src_slot(s_st[tid].phase, s_st[tid].cur, s_st[tid].rk_stage);
-                s_tr[tid] = tr;
-                s_src[tid] = ((long long)slot * n + tr) * P.MD;
-            } else {
-                s_tr[tid] = -1;
-            }
-        }
-        __syncthreads();
-        const double2 *mat = P.mats + P.g_off[g];
-        if (tid == 0) {
-            fence_proxy_async();
-            mbar_expect_tx(&bar[kStages], (uint32_t)(ncol * kp * 16));
-            for (int c = 0; c < ncol; c++) bulk_g2s(Bt + c * S16, P.psi + s_src[c], (uint32_t)(kp * 16), &bar[kStages]);
-            for (int q = 0; q < kStages && q < nslab; q++) {
-                const int kcq = min(KB, kp - q * KB);
-                mbar_expect_tx(&bar[q], (uint32_t)(kcq * MD * 16));
-                bulk_g2s(Us + q * KB * MD, mat + (size_t)q * KB * MD, (uint32_t)(kcq * MD * 16), &bar[q]);
-            }
-        }
-        __syncwarp();  // warp 0's other lanes wait for the copies to be issued instead of spinning on them
+        for (int c = warp; c < ncol; c += NW) stage_column(P, s_in[c], kp, Bt + c * S16, &s_st[c], lane);
+        load_slab<NT>(mat, Us, 0, kp, KS, MD);
+        const int nbd = P.nb * P.deep;
+        const Ens sys{dg, s_gd.ens * P.Ge, nbd <= kMaxDt ? s_dt : P.e_dt + (size_t)s_gd.ens * nbd,
+                    P.e_rate + (size_t)s_gd.ens * P.nd};
+        if (warp == 0) hint = scan<NCM>(P, stop_live, turn, lane);
+        else if (nbd <= kMaxDt && tid >= 32 && tid < 32 + nbd) s_dt[tid - 32] = __ldg(P.e_dt + (size_t)s_gd.ens * nbd + tid - 32);
         const long long t1 = clock64();
-        bool ok;
-        if (ncb == 1)
-            ok = tile_dmma<R1, 16>(mat, Bt, Us, bar, released, phase, dg, kp, KB, RB, MD, S16, warp, lane, tid);
-        else if (ncb == 2)
-            ok = tile_dmma<R2, 8>(mat, Bt, Us, bar, released, phase, dg, kp, KB, RB, MD, S16, warp, lane, tid);
-        else
-            ok = tile_dmma<R4, 4>(mat, Bt, Us, bar, released, phase, dg, kp, KB, RB, MD, S16, warp, lane, tid);
-        if (!__syncthreads_and(ok ? 1 : 0)) {  // a bounded wait gave up: report and stop
-            if (tid == 0) {
-                atomicAdd(&P.ctrl[4], 1);
-                report_error(P, -1, ERR_TIMEOUT);
-            }
-            break;
+        if constexpr (NT == 256) {
+            if (ncb == 1) tile_dmma<R2, 8, NT>(mat, Bt, Us, dg, kp, KS, RB, S16, warp, lane);
+            else if (R1 == 0 || ncb == 2) tile_dmma<R4, 4, NT>(mat, Bt, Us, dg, kp, KS, RB, S16, warp, lane);
+            else tile_dmma<R1, 2, NT>(mat, Bt, Us, dg, kp, KS, RB, S16, warp, lane);
+        } else {
+            if (ncb == 1) tile_dmma<R1, 16, NT>(mat, Bt, Us, dg, kp, KS, RB, S16, warp, lane);
+            else if (ncb == 2) tile_dmma<R2, 8, NT>(mat, Bt, Us, dg, kp, KS, RB, S16, warp, lane);
+            else tile_dmma<R4, 4, NT>(mat, Bt, Us, dg, kp, KS, RB, S16, warp, lane);
         }
+        __syncthreads();
         const long long t2 = clock64();
-        for (int c = warp; c < ncol; c += kThreads / 32) {
-            const int g2 = column_epilogue(P, Bt + c * S16, s_tr[c], s_st[c], lane);
-            if (lane == 0) s_g2[c] = g2;
+        for (int c = warp; c < ncol; c += NW) {
+            unsigned entry;
+            const int tr = (int)(s_in[c] >> 3);
+            const int g2 = column_epilogue(P, Bt + c * S16, tr, s_st[c], lane, entry, sys, global_slots(P, tr), &P.st[tr],
+                                           true);
+            if (lane == 0) {
+                s_g2[c] = g2;
+                s_entry[c] = entry;
+            }
         }
         __syncthreads();
-        enqueue_batch(P, cnt_next, list_next, s_tr, s_g2, ncol);
-        work += ncol;
-        pos += ncol;
-        fence_proxy_async();
-        __syncthreads();
-        const long long t3 = clock64();
-        tr_setup += t1 - t0;
-        tr_loop += t2 - t1;
-        tr_epi += t3 - t2;
-        tr_sub += 1;
-        tr_cb += (ncb == 3) ? 4 : ncb;
+        // warp 1 appends while warp 0 takes the next sub-tile (s_g2 and s_entry are rewritten after that
+        // sub-tile's products)
+        if (warp == 1) append(P, lane < ncol ? s_g2[lane] : -1, lane < ncol ? s_entry[lane] : kFree, ncol, lane);
+        if (tid == 0) tally.add(ncol, (ncb == 3) ? 4 : ncb, t0, t1, t2, clock64());
     }
-    if (tid == 0 && work) atomicAdd((unsigned long long *)P.work, (unsigned long long)work);
-    if (P.trace && tid == 0) {
-        long long *t = P.trace + (size_t)blockIdx.x * kTraceFields;
-        t[0] += clock64() - t_begin;
-        t[1] += tr_setup;
-        t[2] += 0;
-        t[3] += tr_loop;
-        t[4] += tr_epi;
-        t[5] += tr_sub;
-        t[6] += tr_cb;
-        t[7] += work;
-    }
-    // the last CTA to finish plans the next micro-step from the buckets all CTAs filled
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        s_last = atomicAdd(P.plan_sync, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (s_last) {
-        __threadfence();
-        plan_scan(P, cnt_next);
-        if (tid == 0) *P.plan_sync = 0u;
-    }
+    if (tid == 0) tally.flush(P);
 }
 
-// Plan of step 0 after a host-side enqueue (schedule, observe, resume): one block.
-__global__ void __launch_bounds__(1024) plan_kernel(const Params P)
+// ---------------------------------------------------------------- few trajectories: one per CTA or cluster
+__device__ __forceinline__ void cluster_sync()
 {
-    plan_scan(P, P.cnt);
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ unsigned cluster_rank()
+{
+    unsigned r;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+// Address of `p` (this CTA's shared memory) in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_rank(const void *p, unsigned rank)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+
+__device__ __forceinline__ void st_cluster(uint32_t addr, double2 v)
+{
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y) : "memory");
+}
+
+__device__ __forceinline__ void st_cluster(uint32_t addr, int v)
+{
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+// Row `row` of two complex matrix columns k, k + 1 (32 bytes).
+__device__ __forceinline__ void ld_kpair(const double2 *p, double2 &a, double2 &b)
+{
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y) : "l"(p));
+}
+
+// y[row] = sum_k M[row][k] x[k] with the contract's k-ascending fma chain: `m` points at the row in
+// k pair 0, a k pair is `step` components further.  Blocks of kPre k pairs, the next block's loads
+// in flight behind the current one's fmas; no branch stands between the loads of a block (a test
+// per load made the compiler wait for each: 390 cycles per k pair instead of 110 at d = 201, where
+// one SM's L2 bandwidth, 64 bytes a cycle, gives 104).
+template <int kPre>
+__device__ __forceinline__ double2 row_matvec(const double2 *m, const double2 *x, int kp2, size_t step)
+{
+    double re = 0.0, im = 0.0;
+    auto fmas = [&](const double2 &u, const double2 &v, const double2 &x0, const double2 &x1) {
+        re = __fma_rn(u.x, x0.x, re);
+        im = __fma_rn(u.x, x0.y, im);
+        re = __fma_rn(-u.y, x0.y, re);
+        im = __fma_rn(u.y, x0.x, im);
+        re = __fma_rn(v.x, x1.x, re);
+        im = __fma_rn(v.x, x1.y, im);
+        re = __fma_rn(-v.y, x1.y, re);
+        im = __fma_rn(v.y, x1.x, im);
+    };
+    // block k0 .. (past the end it reads the last pair again)
+    auto load = [&](double2 (&u)[kPre], double2 (&v)[kPre], int k0) {
+        if (k0 + kPre <= kp2) {
+            const double2 *p = m + k0 * step;
+#pragma unroll
+            for (int j = 0; j < kPre; j++) ld_kpair(p + j * step, u[j], v[j]);
+        } else if (k0 < kp2) {
+#pragma unroll
+            for (int j = 0; j < kPre; j++) ld_kpair(m + min(k0 + j, kp2 - 1) * step, u[j], v[j]);
+        }
+    };
+    auto block = [&](const double2 (&u)[kPre], const double2 (&v)[kPre], int k0) {
+        if (k0 + kPre <= kp2) {
+#pragma unroll
+            for (int j = 0; j < kPre; j++) fmas(u[j], v[j], x[2 * (k0 + j)], x[2 * (k0 + j) + 1]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < kPre; j++)
+                if (k0 + j < kp2) fmas(u[j], v[j], x[2 * (k0 + j)], x[2 * (k0 + j) + 1]);
+        }
+    };
+    double2 a[kPre], b[kPre], c[kPre], d[kPre];
+    load(a, b, 0);
+#pragma unroll 1
+    for (int k = 0; k < kp2; k += 2 * kPre) {
+        load(c, d, k + kPre);
+        block(a, b, k);
+        load(a, b, k + 2 * kPre);
+        block(c, d, k + kPre);
+    }
+    return make_double2(re, im);
+}
+
+constexpr int kStint = 128;  // matvecs between two looks at the clock
+
+// The plain form for few trajectories: a cluster of C CTAs takes one trajectory from the queues and
+// runs its whole chain of matvecs (split tree, jumps, observables) until its work of this call is
+// done or the slice is over, with the states and the record in shared memory.  Each CTA computes
+// its share of the rows, a thread per row with the matrix straight from L2 (or L1, for small d),
+// and stores them into every CTA's copy of the product; after one cluster barrier all CTAs run the
+// same epilogue on their own copies, so a step has no global round trip, no queue and no second
+// barrier (the product is double-buffered).
+// What bounds it: the chain of 2 d dependent FP64 fmas per row and the epilogue's latency, or the
+// L2 reads of a whole matrix per trajectory and step (16 d^2 bytes; the sub-tiles of flow_kernel
+// share them over up to 32 trajectories), which is why it takes few trajectories only.
+template <int C, int kPre>
+__global__ void __launch_bounds__(kSoloThreads, kPre > 4 ? 1 : 2) solo_kernel(const Params P, int rows)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(16) TrajState s_st;
+    __shared__ int s_go, s_tr, s_group, s_next;
+    __shared__ unsigned s_entry;
+    __shared__ double s_dt[kMaxDt];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = C > 1 ? (int)cluster_rank() : 0;
+    const bool lead = rank == 0;
+    const int nslots = P.prop == 1 ? kRkSlots : 2, SD = P.MD + 2;
+    double2 *const sl = reinterpret_cast<double2 *>(smem);
+    double2 *const yb = sl + (size_t)nslots * SD;  // [2][SD]
+    const Slots slots{sl, (size_t)SD};
+    const unsigned long long t_end = global_ns() + kSliceNs;
+    unsigned turn = blockIdx.x;
+    __shared__ Tally tally;
+    if (tid == 0) tally.reset();
+    auto sync = [&] {
+        if (C > 1) cluster_sync();
+        else __syncthreads();
+    };
+
+    while (true) {
+        const long long t0 = clock64();
+        // the lead takes a trajectory and tells the others: 0 none, 1 run
+        if (lead && warp == 0) {
+            GroupDesc gd{};
+            unsigned en;
+            const int n = take<1>(P, t_end, 0, Pick{0, 0}, turn, lane, gd, en);
+            en = __shfl_sync(0xffffffffu, en, 0);
+            const int tr = (int)(en >> 3), g = gd.group;
+            if (lane < C) {
+                if (C > 1) {
+                    st_cluster(map_rank(&s_go, lane), n);
+                    st_cluster(map_rank(&s_tr, lane), tr);
+                    st_cluster(map_rank(&s_group, lane), g);
+                    st_cluster(map_rank(&s_next, lane), (int)(en & 7u));
+                } else {
+                    s_go = n;
+                    s_tr = tr;
+                    s_group = g;
+                    s_next = (int)(en & 7u);
+                }
+            }
+        }
+        sync();
+        if (s_go <= 0) break;
+        const int tr = s_tr;
+        int g = s_group, in = s_next;
+        if (C > 1) __threadfence();  // the lead's acquire, for this CTA's reads of the trajectory
+        if (tid < (int)(sizeof(TrajState) / 16))
+            reinterpret_cast<uint4 *>(&s_st)[tid] = __ldcg(reinterpret_cast<const uint4 *>(&P.st[tr]) + tid);
+        for (int i = 0; i < nslots; i++) {
+            const double2 *src = slot_ptr(P, i, tr);
+            for (int k = tid; k < P.MD; k += blockDim.x) sl[i * SD + k] = __ldcg(src + k);
+        }
+        __syncthreads();
+        const int e = s_st.ens, nbd = P.nb * P.deep;
+        Ens E = global_ens(P, e);
+        if (nbd <= kMaxDt) {
+            if (tid < 32)
+                for (int i = tid; i < nbd; i += 32) s_dt[i] = E.dt[i];
+            E.dt = s_dt;
+        }
+        const int d = E.d, MD = 8 * ((d + 7) / 8), kp2 = (d + 1) / 2;
+        // the ensemble's matrices are equally far apart
+        const int g0 = E.g0;
+        const long long m0 = P.g_off[g0], mstep = P.g_off[g0 + 1] - m0;
+        const int row = rank * rows + tid;
+        const bool mine = tid < rows && row < d;
+        const double2 *mrow = P.mats + m0 + 2 * row;
+        int steps = 0, buf = 0, g2 = g;
+        long long t1 = clock64();
+        if (tid == 0) tally.setup += t1 - t0;
+        while (true) {
+            double2 *y = yb + buf * SD;
+            if (mine) {
+                const double2 v = row_matvec<kPre>(mrow + (g2 - g0) * mstep, sl + in * SD, kp2, 2 * (size_t)MD);
+                if (C > 1) {
+#pragma unroll
+                    for (int r = 0; r < C; r++) st_cluster(map_rank(y + row, r), v);
+                } else {
+                    y[row] = v;
+                }
+            }
+            sync();
+            const long long t2 = clock64();
+            if (warp == 0) {
+                unsigned entry;
+                const int next = column_epilogue(P, y, tr, s_st, lane, entry, E, slots, &s_st, lead);
+                if (lane == 0) {
+                    s_group = next;
+                    s_entry = entry;
+                }
+            }
+            __syncthreads();
+            if (tid == 0) tally.add(1, 1, t1, t1, t2, clock64());
+            t1 = clock64();
+            steps++;
+            buf ^= 1;
+            g2 = s_group;
+            in = (int)(s_entry & 7u);
+            if (g2 < 0) break;
+            if (steps % kStint == 0) {  // the lead's clock decides for all
+                if (lead && tid < C) {
+                    const int go = global_ns() < t_end ? 1 : 0;
+                    if (C > 1) st_cluster(map_rank(&s_go, tid), go);
+                    else s_go = go;
+                }
+                sync();
+                if (s_go == 0) break;
+            }
+        }
+        if (lead) {  // back to global memory, then to the queue of its next matrix (or done)
+            for (int i = 0; i < nslots; i++) {
+                double2 *dst = slot_ptr(P, i, tr);
+                for (int k = tid; k < d; k += blockDim.x) dst[k] = sl[i * SD + k];
+            }
+            if (tid < (int)(sizeof(TrajState) / 16))
+                reinterpret_cast<uint4 *>(&P.st[tr])[tid] = reinterpret_cast<const uint4 *>(&s_st)[tid];
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence();  // release
+                if (g2 >= 0) {
+                    const GroupDesc gd = load_desc(P.gd + g2);
+                    const unsigned pos = atomicAdd(&P.q[g2].tail, 1u);
+                    atomicAdd(&P.q[g2].avail, 1);
+                    unsigned *entry = P.ring + gd.roff + (pos & gd.rmask());
+                    bool put = false;
+                    for (long long i = 0; i < kWaitLimit && !put; i++) put = atomicCAS(entry, kFree, s_entry) == kFree;
+                    if (!put) {
+                        atomicAdd(&P.ctrl[4], 1);
+                        report_error(P, -1, ERR_TIMEOUT);
+                    }
+                } else {
+                    atomicSub(P.ctrl + kLive, 1);
+                }
+            }
+        }
+        sync();  // no CTA's shared memory is rewritten or left while another still uses it
+    }
+    if (C > 1) cluster_sync();
+    if (lead && tid == 0) tally.flush(P);
 }
 
 // Bucket trajectories for step 0 of a call.  mode 0: start of a run of P.target periods;
@@ -988,9 +1333,9 @@ __global__ void schedule_kernel(const Params P, int mode)
         if (!s.paused) return;
         s.paused = 0;
     }
-    const int g = group_of(P, s);
-    if (g >= 0) enqueue(P, P.cnt, P.lists, g, tr);
     P.st[tr] = s;
+    const int g = group_of(P, s);
+    if (g >= 0) enqueue(P, g, tr);
 }
 
 // Host-initiated observables of the current states (one warp per trajectory); the energy
@@ -1005,15 +1350,15 @@ __global__ void observe_kernel(const Params P, int dump, int is_start)
     TrajState s = P.st[tr];
     if (s.phase == PH_ERROR) return;
     const double2 *src = slot_ptr(P, s.cur, tr);
-    for (int k = lane; k < dim_of(P, s); k += 32) col[k] = src[k];
+    for (int k = lane; k < P.e_d[s.ens]; k += 32) col[k] = src[k];
     __syncwarp();
-    obs_prep(P, s, tr, col, lane, dump, is_start);
+    obs_prep(P, s, tr, global_ens(P, s.ens), global_slots(P, tr), col, lane, dump, is_start);
     if (lane == 0) {
         s.pc = 0;
         s.di = 0;
         s.phase = PH_OBS_E;
-        enqueue(P, P.cnt, P.lists, P.e_g0[s.ens] + P.gHE, tr);
         P.st[tr] = s;
+        enqueue(P, P.e_g0[s.ens] + P.gHE, tr);
     }
 }
 
@@ -1152,56 +1497,121 @@ __global__ void clear_records_kernel(const Params P)
 }
 
 // ---------------------------------------------------------------- host-side launchers
-size_t step_smem_bytes(int MD, int nc, int kb);
-
-template <int R4, int R2, int R1>
-static cudaError_t launch_step_t(const Params &P, int s, int grid, cudaStream_t st)
+// Lets a kernel take all the shared memory the current device gives a CTA, once per device (the same
+// value whoever asks, so engines on several threads do not disturb each other).
+template <class Kernel>
+static cudaError_t allow_smem(Kernel *kernel, std::atomic<unsigned long long> &done)
 {
-    static int attr_bytes = 0;
-    if (attr_bytes < P.step_smem) {
-        cudaError_t e =
-            cudaFuncSetAttribute(step_kernel<R4, R2, R1>, cudaFuncAttributeMaxDynamicSharedMemorySize, P.step_smem);
-        if (e != cudaSuccess) return e;
-        attr_bytes = P.step_smem;
-    }
-    step_kernel<R4, R2, R1><<<grid, kThreads, P.step_smem, st>>>(P, s);
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (e != cudaSuccess || (done.load() & bit)) return e;
+    cudaFuncAttributes a{};
+    e = cudaFuncGetAttributes(&a, kernel);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+    if (e == cudaSuccess) done.fetch_or(bit);
+    return e;
+}
+
+template <int NT, int R4, int R2, int R1>
+static cudaError_t launch_flow_t(const Params &P, int stop_live, int grid, cudaStream_t st)
+{
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e = allow_smem(flow_kernel<NT, R4, R2, R1>, done);
+    if (e != cudaSuccess) return e;
+    flow_kernel<NT, R4, R2, R1><<<grid, NT, P.step_smem, st>>>(P, stop_live);
     return cudaGetLastError();
 }
 
-cudaError_t launch_split_step(const Params &P, int s, int grid, cudaStream_t st);
-
-// Instantiation for the largest padded rows MD: up to 256 rows every sub-tile width may occur
-// (R4 = ceil(RB / 4)); up to 512 the 32-column sub-tiles belong to ensembles of at most 256 rows
-// (R4 = 8) and R2 = ceil(RB / 8); up to 1024 also R2 = 8 and R1 = ceil(RB / 16).
-cudaError_t launch_step(const Params &P, int s, int grid, cudaStream_t st)
+// Instantiation for the threads per CTA (nt) and the largest padded rows MD.  256 threads (two
+// CTAs per SM): 16-column sub-tiles have 4 warps per column block, 8-column ones 8.  512 threads:
+// up to 256 rows every sub-tile width may occur (R4 = ceil(RB / 4)); up to 512 the 32-column
+// sub-tiles belong to ensembles of at most 256 rows (R4 = 8) and R2 = ceil(RB / 8); up to 1024
+// also R2 = 8 and R1 = ceil(RB / 16).
+cudaError_t launch_flow(const Params &P, int nt, int stop_live, int grid, cudaStream_t st)
 {
-    if (P.split) return launch_split_step(P, s, grid, st);
     const int RB = P.MD / 8;
-    if (RB <= 32) {
+    if (nt == 256) {
         switch ((RB + 3) / 4) {
-        case 1: return launch_step_t<1, 1, 1>(P, s, grid, st);
-        case 2: return launch_step_t<2, 1, 1>(P, s, grid, st);
-        case 3: return launch_step_t<3, 2, 1>(P, s, grid, st);
-        case 4: return launch_step_t<4, 2, 1>(P, s, grid, st);
-        case 5: return launch_step_t<5, 3, 2>(P, s, grid, st);
-        case 6: return launch_step_t<6, 3, 2>(P, s, grid, st);
-        case 7: return launch_step_t<7, 4, 2>(P, s, grid, st);
-        default: return launch_step_t<8, 4, 2>(P, s, grid, st);
+        case 1: return launch_flow_t<256, 1, 1, 2>(P, stop_live, grid, st);
+        case 2: return launch_flow_t<256, 2, 1, 4>(P, stop_live, grid, st);
+        case 3: return launch_flow_t<256, 3, 2, 6>(P, stop_live, grid, st);
+        case 4: return launch_flow_t<256, 4, 2, 8>(P, stop_live, grid, st);
+        case 5: return launch_flow_t<256, 5, 3, 0>(P, stop_live, grid, st);
+        case 6: return launch_flow_t<256, 6, 3, 0>(P, stop_live, grid, st);
+        case 7: return launch_flow_t<256, 7, 4, 0>(P, stop_live, grid, st);
+        case 8: return launch_flow_t<256, 8, 4, 0>(P, stop_live, grid, st);
+        default: return cudaErrorInvalidValue;
         }
     }
+    if (RB <= 32) return launch_flow_t<512, 8, 4, 2>(P, stop_live, grid, st);
     if (RB <= 64) {
         switch ((RB + 7) / 8) {
-        case 5: return launch_step_t<8, 5, 3>(P, s, grid, st);
-        case 6: return launch_step_t<8, 6, 3>(P, s, grid, st);
-        case 7: return launch_step_t<8, 7, 4>(P, s, grid, st);
-        default: return launch_step_t<8, 8, 4>(P, s, grid, st);
+        case 5: return launch_flow_t<512, 8, 5, 3>(P, stop_live, grid, st);
+        case 6: return launch_flow_t<512, 8, 6, 3>(P, stop_live, grid, st);
+        case 7: return launch_flow_t<512, 8, 7, 4>(P, stop_live, grid, st);
+        default: return launch_flow_t<512, 8, 8, 4>(P, stop_live, grid, st);
         }
     }
     switch ((RB + 15) / 16) {
-    case 5: return launch_step_t<8, 8, 5>(P, s, grid, st);
-    case 6: return launch_step_t<8, 8, 6>(P, s, grid, st);
-    case 7: return launch_step_t<8, 8, 7>(P, s, grid, st);
-    case 8: return launch_step_t<8, 8, 8>(P, s, grid, st);
+    case 5: return launch_flow_t<512, 8, 8, 5>(P, stop_live, grid, st);
+    case 6: return launch_flow_t<512, 8, 8, 6>(P, stop_live, grid, st);
+    case 7: return launch_flow_t<512, 8, 8, 7>(P, stop_live, grid, st);
+    case 8: return launch_flow_t<512, 8, 8, 8>(P, stop_live, grid, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+size_t solo_smem_bytes(const Params &P)
+{
+    return (size_t)((P.prop == 1 ? kRkSlots : 2) + 2) * (P.MD + 2) * sizeof(double2);
+}
+
+// Rows per CTA when C CTAs share a matrix of at most d rows (whole 8-row blocks).
+static int solo_rows(int d, int C) { return 8 * ((d + 8 * C - 1) / (8 * C)); }
+
+template <int C, int kPre>
+static cudaError_t launch_solo_t(const Params &P, int workers, cudaStream_t st)
+{
+    const size_t smem = solo_smem_bytes(P);
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e = allow_smem(solo_kernel<C, kPre>, done);
+    if (e != cudaSuccess) return e;
+    const int rows = solo_rows(P.d, C);
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(workers * C);
+    lc.blockDim = dim3(32 * ((rows + 31) / 32));
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = C > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, solo_kernel<C, kPre>, P, rows);
+}
+
+// Eight k pairs in flight per thread where every CTA of the launch is resident with the registers
+// that takes (a lone CTA's matvec at d = 201: 110 cycles per k pair against 137), else four.
+template <int C>
+static cudaError_t launch_solo_c(const Params &P, int workers, cudaStream_t st)
+{
+    const int threads = 32 * ((solo_rows(P.d, C) + 31) / 32), per_sm = (workers * C + P.grid - 1) / P.grid;
+    return per_sm * threads * 256 <= 65536 ? launch_solo_t<C, 8>(P, workers, st) : launch_solo_t<C, 4>(P, workers, st);
+}
+
+// `workers` clusters of C CTAs (C a power of two up to 8, at least d / kSoloThreads).
+cudaError_t launch_solo(const Params &P, int C, int workers, cudaStream_t st)
+{
+    switch (C) {
+    case 1: return launch_solo_c<1>(P, workers, st);
+    case 2: return launch_solo_c<2>(P, workers, st);
+    case 4: return launch_solo_c<4>(P, workers, st);
+    case 8: return launch_solo_c<8>(P, workers, st);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -1213,34 +1623,37 @@ int pick_layout(int d, int *rows_per_block)
     return 8 * ((d + 7) / 8);
 }
 
-// Shared memory of the step kernel: nc staged columns of MD + 1 (odd stride) and kStages
-// propagator slabs of kb k rows.
+// Shared memory of the plain kernel: nc staged columns of MD + kColPad components (columns 32
+// bytes apart modulo the banks: conflict-free B operand reads) and two slabs of kb k rows (as
+// a ring of four half slabs where kb is a multiple of 4).
 size_t step_smem_bytes(int MD, int nc, int kb)
 {
-    return (size_t)(nc * (MD + 1) + kStages * kb * MD) * sizeof(double2);
+    return (size_t)(nc * (MD + kColPad) + 2 * kb * MD) * sizeof(double2);
 }
 
-// Static shared memory of the step kernel (the same for every instantiation).
-size_t step_static_smem()
+// Static shared memory of the plain kernel with nt threads (the same for every instantiation).
+size_t step_static_smem(int nt)
 {
     cudaFuncAttributes a{};
-    if (cudaFuncGetAttributes(&a, step_kernel<1, 1, 1>) != cudaSuccess) return 16384;
+    const cudaError_t e = nt == 256 ? cudaFuncGetAttributes(&a, flow_kernel<256, 1, 1, 2>)
+                                    : cudaFuncGetAttributes(&a, flow_kernel<512, 8, 4, 2>);
+    if (e != cudaSuccess) return 16384;
     return a.sharedSizeBytes;
 }
 
-// Widest sub-tile (32, 16 or 8 columns) whose staged columns leave room for slabs of at least
-// 8 k rows (at most 16, even) in `budget` bytes of dynamic shared memory, with at most 8 row
-// blocks per warp; failing that, the widest with 2-row slabs.  Returns false when none fits.
-bool pick_step_tiles(int MD, size_t budget, int *nc, int *kb)
+// Widest sub-tile (at most nc_max: 32, 16 or 8 columns) whose staged columns leave room for slabs
+// of at least 8 k rows (at most 16, even) in `budget` bytes of dynamic shared memory, with at most
+// 8 row blocks per warp; failing that, the widest with 2-row slabs.  Returns false when none fits.
+bool pick_step_tiles(int MD, size_t budget, int nt, int nc_max, int *nc, int *kb)
 {
     const int RB = MD / 8;
     for (int min_kb = 8; min_kb >= 2; min_kb -= 6) {
-        for (int c = kNC; c >= 8; c /= 2) {
-            const int W1 = 16 / (c / 8);
+        for (int c = nc_max; c >= 8; c /= 2) {
+            const int W1 = nt / 32 / (c / 8);  // warps per column block
             if ((RB + W1 - 1) / W1 > 8) continue;
-            const size_t bt = (size_t)c * (MD + 1) * sizeof(double2);
+            const size_t bt = (size_t)c * (MD + kColPad) * sizeof(double2);
             if (bt >= budget) continue;
-            int k = (int)((budget - bt) / ((size_t)kStages * MD * sizeof(double2)));
+            int k = (int)((budget - bt) / ((size_t)2 * MD * sizeof(double2)));
             k = std::min(k, kKB) & ~1;
             if (k < min_kb) continue;
             *nc = c;
@@ -1251,14 +1664,12 @@ bool pick_step_tiles(int MD, size_t budget, int *nc, int *kb)
     return false;
 }
 
-// The first micro-step after a host-side enqueue needs its plan (both forms).
+// The split form's first micro-step after a host-side enqueue needs its plan.
 cudaError_t launch_split_plan(const Params &P, cudaStream_t st);
 
 static cudaError_t launch_plan(const Params &P, cudaStream_t st)
 {
-    if (P.split) return launch_split_plan(P, st);
-    plan_kernel<<<1, 1024, 0, st>>>(P);
-    return cudaGetLastError();
+    return P.split ? launch_split_plan(P, st) : cudaGetLastError();
 }
 
 cudaError_t launch_schedule(const Params &P, int mode, cudaStream_t st)
@@ -1306,11 +1717,13 @@ __global__ void rk_schedule_kernel(const Params P)
     if (P.target > 0 && runs(P, tr)) {
         s.t = rk_step_time(P, s);
         rk_begin(s, P.rk_step, nrm, 0);
-        if (lane == 0) enqueue(P, P.cnt, P.lists, P.e_g0[s.ens], tr);
     } else {
         s.phase = PH_DONE;
     }
-    if (lane == 0) P.st[tr] = s;
+    if (lane == 0) {
+        P.st[tr] = s;
+        if (s.phase == PH_RK) enqueue(P, P.e_g0[s.ens], tr);
+    }
 }
 
 cudaError_t launch_rk_schedule(const Params &P, cudaStream_t st)

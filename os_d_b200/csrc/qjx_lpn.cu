@@ -12,7 +12,7 @@
 //
 // One CTA per pair.  The pair's work is a handful of d x d complex matvecs (characteristics)
 // plus one per bisection step of a renormalisation, thread per row, reading the FP64 matrices
-// in the engine's transposed layout mats[g][k][row] (coalesced across the CTA's threads, L2
+// in the engine's layout mats[g][k / 2][row][k % 2] (coalesced across the CTA's threads, L2
 // resident across CTAs); next to the period's micro-steps this is a small cost.
 //
 // Arithmetic: every operation is the one the CPU oracle (lpn_oracle.c) performs: the canonical
@@ -120,7 +120,7 @@ __device__ __forceinline__ void cta_matvec(const Params &P, const EnsCtx &E, int
     for (int r = threadIdx.x; r < d; r += blockDim.x) {
         double re = 0.0, im = 0.0;
         for (int k = 0; k < d; k++) {
-            const double2 m = mat[(size_t)k * MD + r];
+            const double2 m = mat[mat_at(k, r, MD)];
             const double2 v = x[k];
             re = __fma_rn(m.x, v.x, re);
             re = __fma_rn(-m.y, v.y, re);

@@ -183,9 +183,9 @@ __device__ bool recheck_column(const Params &P, int tr, unsigned char *smem, Tra
         rphase ^= 1u << q;
         const int k0 = sl * kb, kc = min(kb, kp - k0);
         if (ok && tid < dg) {
-            const double2 *Mq = slab + (size_t)q * kb * MDg + tid;
+            const double2 *Mq = slab + (size_t)q * kb * MDg;
             for (int kk = 0; kk < kc; kk++) {
-                const double2 m = Mq[(size_t)kk * MDg], v = xs[k0 + kk];
+                const double2 m = Mq[mat_at(kk, tid, MDg)], v = xs[k0 + kk];
                 re = __fma_rn(m.x, v.x, re);
                 re = __fma_rn(-m.y, v.y, re);
                 im = __fma_rn(m.x, v.y, im);
@@ -204,7 +204,8 @@ __device__ bool recheck_column(const Params &P, int tr, unsigned char *smem, Tra
     if (tid < dg) ys[tid] = make_double2(re, im);
     __syncthreads();
     if (warp == 0) {
-        const int g2 = column_epilogue(P, ys, tr, st, lane);
+        unsigned entry;
+        const int g2 = column_epilogue(P, ys, tr, st, lane, entry, global_ens(P, st.ens), global_slots(P, tr), &P.st[tr], true);
         if (g2 >= 0 && lane == 0) {
             const int pos = atomicAdd(&cnt_next[g2], 1);
             list_next[P.g_loff[g2] + pos] = tr;
@@ -582,6 +583,7 @@ __global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P,
                 break;
             }
             const long long t2 = clock64();
+            const Ens sys{d, e * P.Ge, P.e_dt + (size_t)e * P.nb * P.deep, P.e_rate + (size_t)e * P.nd};
             float *sacc = reinterpret_cast<float *>(smem);  // [RP][2 MDs + 1] FP32 accumulators
             const int SR = 2 * MDs + 1;
             for (int p0 = 0; p0 < rows; p0 += RP) {  // passes of RP trajectories
@@ -612,7 +614,9 @@ __global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P,
                     const float *row = sacc + (size_t)cc * SR;
                     for (int k = lane; k < MDs; k += 32) wcol[k] = make_double2((double)row[k], (double)row[MDs + k]);
                     __syncwarp();
-                    const int g2 = column_epilogue(P, wcol, s_tr[m], s_st[m], lane);
+                    unsigned entry;
+                    const int g2 = column_epilogue(P, wcol, s_tr[m], s_st[m], lane, entry, sys,
+                                                   global_slots(P, s_tr[m]), &P.st[s_tr[m]], true);
                     if (lane == 0) w_g2[warp][nm] = g2;
                     __syncwarp();
                 }
