@@ -1383,44 +1383,129 @@ __global__ void normalize_kernel(const Params P, double2 *hat)
     }
 }
 
-// one 16 x 16 tile of rho per block (256 threads), trajectories staged 32 at a time
-__global__ void __launch_bounds__(256) rho_kernel(const Params P, const double2 *hat, double2 *rho)
+constexpr int kRhoBlocks = 5;       // most 8 x 8 blocks of rho per CTA
+constexpr int kRhoT = 32;           // trajectories per stage
+constexpr int kRhoStages = 3;
+constexpr int kRhoStride = 12;      // components between trajectories of a staged block of 8 (192 bytes: the
+                                    // two trajectories of an MMA fall on different banks)
+
+size_t rho_smem_bytes(int per) { return (size_t)kRhoStages * (per + 2) * kRhoT * kRhoStride * sizeof(double2); }
+
+// rho_ij = (1/n) sum_t hat_t[i] conj(hat_t[j]) on the FP64 tensor core.  One warp per part (re or
+// im) of an 8 x 8 block: two trajectories are one MMA, A = [xr, xi] (re) or [xi, -xr] (im) of two
+// trajectories against B = [yr; yi], which is the canonical chain re += xr yr; re += xi yi;
+// im += xi yr; im -= xr yi with trajectories ascending, bit for bit.  The chain over n cannot be
+// split, so the work is spread over chains: a CTA takes `per` consecutive blocks (row-major), at
+// d = 201 676 blocks in 136 CTAs, 10 warps on each of 136 SMs at most 3 to a scheduler.
+// Bound: 3 chains x n / 2 MMAs of 16 cycles = 123 us at d = 201, n = 10^4 (the pipe's floor at a
+// perfect balance is 95 us); two fma chains per thread on 16 x 16 tiles before took 0.85 ms.
+__global__ void __launch_bounds__(64 * kRhoBlocks) rho_kernel(const Params P, const double2 *hat, double2 *rho, int per)
 {
-    __shared__ double2 a[32][16], b[32][16];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int i0 = blockIdx.y * 16, j0 = blockIdx.x * 16;
-    double re = 0.0, im = 0.0;
-    for (int c = 0; c < P.n; c += 32) {
-        for (int e = threadIdx.x; e < 32 * 16; e += 256) {
-            const int t = e >> 4, k = e & 15, tr = c + t;
-            double2 za = make_double2(0.0, 0.0), zb = za;
-            if (tr < P.n) {
-                if (i0 + k < P.d) za = hat[(size_t)tr * P.MD + i0 + k];
-                if (j0 + k < P.d) zb = hat[(size_t)tr * P.MD + j0 + k];
-            }
-            a[t][k] = za;
-            b[t][k] = zb;
-        }
-        __syncthreads();
-        const int m = min(32, P.n - c);
-        for (int t = 0; t < m; t++) {
-            const double2 x = a[t][ty], y = b[t][tx];
-            re = __fma_rn(x.x, y.x, re);
-            re = __fma_rn(x.y, y.y, re);
-            im = __fma_rn(x.y, y.x, im);
-            im = __fma_rn(-x.x, y.y, im);
-        }
-        __syncthreads();
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int RB = (P.d + 7) / 8, b0 = blockIdx.x * per, nb = min(per, RB * RB - b0);
+    const int part = warp & 1, mine = min(warp >> 1, nb - 1);  // (warps past the last block only load)
+    const int g = lane >> 2, t = lane & 3, th = t >> 1, todd = t & 1;
+    const int nst = (P.n + kRhoT - 1) / kRhoT;
+    // staged sets of 8 components per trajectory: 0 and 1 the row blocks of the run (two at most:
+    // per > 1 needs RB > 12), 2 + b the column block of its block b
+    const int ib0 = b0 / RB, sets = 2 + nb;
+    const bool two = (b0 + nb - 1) / RB > ib0;
+    auto at = [&](int it, int set) {
+        return reinterpret_cast<double2 *>(smem) + (size_t)((it % kRhoStages) * (per + 2) + set) * kRhoT * kRhoStride;
+    };
+    // a stage is sets x kRhoT x 8 components; this thread copies component tid % 8 of trajectories
+    // tid / 8 + 8 per i of every set (the addresses are worked out once: doing it in each stage took
+    // most of the kernel's time)
+    const int k = tid & 7, t0 = tid >> 3, tstep = blockDim.x >> 3;
+    int comp[kRhoBlocks + 2];
+#pragma unroll
+    for (int set = 0; set < kRhoBlocks + 2; set++) {
+        const int c = 8 * (set < 2 ? ib0 + set : (b0 + set - 2) % RB) + k;
+        comp[set] = (set < sets && (set != 1 || two)) ? (c < P.d ? c : -1) : -2;  // -1: zeros, -2: not staged
     }
-    const int i = i0 + ty, j = j0 + tx;
-    if (i < P.d && j < P.d)
-        rho[(size_t)i * P.d + j] = make_double2(__ddiv_rn(re, (double)P.n), __ddiv_rn(im, (double)P.n));
+    auto load = [&](int it) {
+        if (it < nst) {
+            double2 *dst = at(it, 0) + k;
+            for (int tt = t0; tt < kRhoT; tt += tstep) {
+                const int tr = it * kRhoT + tt;
+                const double2 *src = hat + (size_t)min(tr, P.n - 1) * P.MD;
+#pragma unroll
+                for (int set = 0; set < kRhoBlocks + 2; set++)
+                    if (comp[set] > -2)
+                        cp16(dst + (set * kRhoT + tt) * kRhoStride, src + max(comp[set], 0), comp[set] >= 0 && tr < P.n);
+            }
+        }
+        cp_commit();
+    };
+    const int blk = b0 + mine, aset = blk / RB - ib0, bset = 2 + mine;
+    double c0 = 0.0, c1 = 0.0;
+    for (int i = 0; i < kRhoStages - 1; i++) load(i);
+    for (int it = 0; it < nst; it++) {
+        cp_wait<kRhoStages - 2>();
+        __syncthreads();  // stage `it` has landed for every thread, and nobody reads the one refilled next
+        load(it + kRhoStages - 1);
+        const double *a = reinterpret_cast<const double *>(at(it, aset) + th * kRhoStride + g) + (part ? 1 - todd : todd);
+        const double *b = reinterpret_cast<const double *>(at(it, bset) + th * kRhoStride + g) + todd;
+#pragma unroll
+        for (int k = 0; k < kRhoT; k += 2) {
+            const double x = a[2 * k * kRhoStride];
+            dmma(c0, c1, (part && todd) ? neg(x) : x, b[2 * k * kRhoStride]);
+        }
+    }
+    if ((warp >> 1) >= nb) return;
+    const int i = 8 * (blk / RB) + g, j = 8 * (blk % RB) + 2 * t;
+    double *out = reinterpret_cast<double *>(rho) + part;
+    if (i < P.d && j < P.d) out[2 * ((size_t)i * P.d + j)] = __ddiv_rn(c0, (double)P.n);
+    if (i < P.d && j + 1 < P.d) out[2 * ((size_t)i * P.d + j + 1)] = __ddiv_rn(c1, (double)P.n);
 }
 
-__global__ void purity_kernel(const double2 *rho, int dd, double *out)
+constexpr int kPurityThreads = 1024, kPurityTile = 2 * kPurityThreads;
+
+// Canonical 32-lane squared norm of rho.  Its 32 chains of d^2 / 32 additions are one warp's; all
+// warps read rho and square it a tile ahead of them (one warp doing both spent its time on the loads).
+__global__ void __launch_bounds__(kPurityThreads) purity_kernel(const double2 *rho, int dd, double *out)
 {
-    const double s = warp_norm(rho, dd, threadIdx.x & 31);
-    if (threadIdx.x == 0) *out = s;
+    __shared__ double sq[2][kPurityTile];
+    const int tid = threadIdx.x, nt = (dd + kPurityTile - 1) / kPurityTile;
+    double2 v0 = make_double2(0.0, 0.0), v1 = v0;
+    auto fetch = [&](int it) {
+        const int i = it * kPurityTile + tid;
+        if (i < dd) v0 = rho[i];
+        if (i + kPurityThreads < dd) v1 = rho[i + kPurityThreads];
+    };
+    fetch(0);
+    double s = 0.0;
+    for (int it = 0; it < nt; it++) {
+        double *p = sq[it & 1];
+        p[tid] = __dadd_rn(__dmul_rn(v0.x, v0.x), __dmul_rn(v0.y, v0.y));
+        p[tid + kPurityThreads] = __dadd_rn(__dmul_rn(v1.x, v1.x), __dmul_rn(v1.y, v1.y));
+        fetch(it + 1);
+        __syncthreads();  // (the tile before last, whose buffer is written next, has been added)
+        if (tid < 32) {
+            const int m = min(kPurityTile, dd - it * kPurityTile);
+#pragma unroll 8
+            for (int e = tid; e < m; e += 32) s = __dadd_rn(s, p[e]);
+        }
+    }
+    if (tid < 32) s = warp_allsum(s);
+    if (tid == 0) *out = s;
+}
+
+// The current states of trajectories tr0 .. tr0 + count - 1, packed [count][d] (one warp each).
+__global__ void gather_states_kernel(const Params P, int tr0, int count, double2 *out)
+{
+    const int lane = threadIdx.x & 31, i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (i >= count) return;
+    const int tr = tr0 + i;
+    const double2 *src = slot_ptr(P, P.st[tr].cur, tr);
+    for (int k = lane; k < P.d; k += 32) out[(size_t)i * P.d + k] = src[k];
+}
+
+cudaError_t launch_gather_states(const Params &P, int tr0, int count, double2 *out, cudaStream_t st)
+{
+    gather_states_kernel<<<(count + 7) / 8, 256, 0, st>>>(P, tr0, count, out);
+    return cudaGetLastError();
 }
 
 __global__ void init_state_kernel(const Params P, int tr0, int tr1)
@@ -1695,9 +1780,14 @@ cudaError_t launch_observe(const Params &P, int dump, int is_start, cudaStream_t
 cudaError_t launch_purity(const Params &P, double2 *hat, double2 *rho, double *out, cudaStream_t st)
 {
     normalize_kernel<<<(P.n + 7) / 8, 256, 0, st>>>(P, hat);
-    const int tiles = (P.d + 15) / 16;
-    rho_kernel<<<dim3(tiles, tiles), 256, 0, st>>>(P, hat, rho);
-    purity_kernel<<<1, 32, 0, st>>>(rho, P.d * P.d, out);
+    const int RB = (P.d + 7) / 8, blocks = RB * RB;
+    // output blocks per CTA: all CTAs on the chip at once where there are few, at most kRhoBlocks
+    const int per = std::max(1, std::min(kRhoBlocks, (blocks + P.grid - 1) / P.grid));
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e = allow_smem(rho_kernel, done);
+    if (e != cudaSuccess) return e;
+    rho_kernel<<<(blocks + per - 1) / per, 64 * per, rho_smem_bytes(per), st>>>(P, hat, rho, per);
+    purity_kernel<<<1, kPurityThreads, 0, st>>>(rho, P.d * P.d, out);
     return cudaGetLastError();
 }
 
