@@ -21,6 +21,7 @@ constexpr int kColPad = 2;             // components between staged columns past
 constexpr int kMaxGroups = 256;        // distinct matrices in one engine
 constexpr int kMaxMD = 1024;           // d <= 1024 (plain form; the split form takes d <= 256)
 constexpr double kSplitNormSlack = 1e-4;  // split precision: tolerated norm excess over 1
+constexpr int kMaxTile = 128;             // split precision: most trajectories per tile (MMA M)
 constexpr int kMaxSplitStages = 8;        // split precision: deepest operand ring
 // plain kernel: a launch hands the device back after kSliceNs (engines of other streams get
 // their turn; the host launches again), and a CTA that finds no work for kIdleNs leaves
@@ -118,13 +119,13 @@ struct Params {
     double *gn;              // [n][nd] channel weights
     const double *g;         // [nd]
     const double *dt;        // [deep]
-    int *cnt;                // [3][G]  split form: bucket sizes of three micro-steps
-    int *lists;              // [2][ltot] split form: bucket lists of two
-    // plain form: one queue per group, a ring of entries (trajectory and input slot; kFree: empty)
+    int *cnt;                // [3][G]  lock-step: bucket sizes of three micro-steps
+    int *lists;              // [2][ltot] lock-step: bucket lists of two
+    // one queue per group (split form: and one for the FP64 rechecks), a ring of entries (trajectory and input slot; kFree: empty)
     // with counts of the entries taken and reserved so far
-    Queue *q;                // [G]
+    Queue *q;                // [G], split form [G + 1]
     unsigned int *ring;
-    const GroupDesc *gd;     // [G]
+    const GroupDesc *gd;     // as q
     // rng
     int rng_kind;
     unsigned long long seed;
@@ -207,9 +208,10 @@ struct Params {
     const long long *g_loff;          // [G] start of the group's bucket list (capacity: the
                                       // ensemble's trajectories); lists hold 2 x ltot entries
     long long ltot;
-    unsigned int *plan_sync;          // [1] CTAs finished in the current micro-step
-    unsigned int *gen;                // [1] split form: plans made (the grid barrier of a multi-step launch)
-    int *sdone;                       // [1] split form: micro-steps run since the host last cleared it
+    unsigned int *plan_sync;          // [1] CTAs finished in the current lock-step micro-step
+    int *sdone;                       // [1] split form: lock-step micro-steps run, or the longest chain
+    int *chain;                       // [n] split form: matvecs of each trajectory in this run
+    int flow;                         // queues (1) or lock-step lists (the split form with QJX_SPLIT_COOP=0)
 };
 
 // Lyapunov paired trajectories (task_id 7, LpnMult): [0, n/2) bases, n/2 + b the variation of b.

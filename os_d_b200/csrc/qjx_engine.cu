@@ -20,7 +20,8 @@ namespace qjx {
 cudaError_t launch_flow(const Params &P, int nt, int stop_live, int grid, cudaStream_t st);
 cudaError_t launch_solo(const Params &P, int C, int workers, cudaStream_t st);
 cudaError_t launch_split_step(const Params &P, int s, int grid, cudaStream_t st);
-cudaError_t launch_split_steps(const Params &P, int s0, int nsteps, int grid, cudaStream_t st);
+cudaError_t launch_split_flow(const Params &P, int grid, cudaStream_t st);
+cudaError_t launch_longest_chain(const Params &P, cudaStream_t st);
 int pick_layout(int d, int *rows_per_block);
 cudaError_t launch_dmma_peak(double *out, int blocks, int iters, cudaStream_t st);
 size_t step_smem_bytes(int MD, int nc, int kb);
@@ -79,7 +80,6 @@ struct qjx_engine {
     int *h_cnt = nullptr;   // pinned [G]
     int *h_ctrl = nullptr;  // pinned [16]: the control words [0, 8); split form: recheck counts [8, 11),
                             // micro-steps run [11], tiles of the next step [12]
-    bool split_coop = true;  // split form: batches of micro-steps as one cooperative launch
     std::vector<std::vector<double>> jt, jn, je;
     std::vector<std::vector<int>> jtype;
     qjx_stats stats{};
@@ -378,9 +378,9 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     h->grid = sms > 0 ? sms : 148;
-    // QJX_SPLIT_COOP=0: run the split form's micro-steps as one launch each (the path taken when a
-    // cooperative launch cannot make every CTA resident)
-    if (const char *v = getenv("QJX_SPLIT_COOP")) h->split_coop = v[0] != '0';
+    // QJX_SPLIT_COOP=0: the split form as lock-step micro-steps, one launch each
+    const char *coop = getenv("QJX_SPLIT_COOP");
+    h->P.flow = (c.precision == 0 || !coop || coop[0] != '0') ? 1 : 0;
     if (cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking); e != cudaSuccess)
         return bail_cuda(e, "cudaStreamCreateWithFlags");
     cudaEventCreate(&h->ev0);
@@ -571,11 +571,9 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
         // next to the input and product vectors
         P.rcnt = (int *)dalloc(h, 3 * sizeof(int));
         P.rlist = (int *)dalloc(h, (size_t)2 * n * sizeof(int));
-        P.gen = (unsigned int *)dalloc(h, sizeof(unsigned int));
         P.sdone = (int *)dalloc(h, sizeof(int));
-        if (!P.e_mds || !P.e_ks || !P.g_uoff || !P.splan || !P.rcnt || !P.rlist || !P.gen || !P.sdone)
+        if (!P.e_mds || !P.e_ks || !P.g_uoff || !P.splan || !P.rcnt || !P.rlist || !P.sdone)
             return bail(QJX_ERR_OOM);
-        cudaMemset(P.gen, 0, sizeof(unsigned int));
         cudaMemset(P.sdone, 0, sizeof(int));
         P.recheck_tol = c.split_recheck == 0.0 ? 1e-5 : (c.split_recheck < 0.0 ? 0.0 : c.split_recheck);
         const size_t ring = (size_t)P.sstages * split_stage_bytes(P.MDs);
@@ -604,27 +602,30 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     P.psi = (double2 *)dalloc(h, (size_t)psi_slots * n * MD * sizeof(double2));
     P.st = (TrajState *)dalloc(h, (size_t)n * sizeof(TrajState));
     P.gn = (double *)dalloc(h, (size_t)n * c.num_diss * sizeof(double));
-    if (c.precision == 1) {  // lock-step bucket lists
+    if (!P.flow) {  // lock-step bucket lists
         P.cnt = (int *)dalloc(h, (size_t)3 * G * sizeof(int));
         P.lists = (int *)dalloc(h, (size_t)2 * P.ltot * sizeof(int));
     } else {  // queues: a ring per group, a power of two long so that the positions may wrap
-        std::vector<GroupDesc> gd(G);
-        std::vector<Queue> q(G);
+        std::vector<GroupDesc> gd;
+        std::vector<Queue> q;
         long long roff = 0;
-        for (int e = 0; e < E; e++) {
+        auto add = [&](long long len, long long off, int nc, int kb, int dim, int e) {
             int rlog = 0;
-            while ((1ll << rlog) < ens[e].n) rlog++;
-            for (int l = 0; l < Ge; l++, roff += 1ll << rlog) {
-                gd[e * Ge + l] = GroupDesc{roff, g_off[e * Ge + l], (unsigned char)rlog, (unsigned char)e_nc[e],
-                                           (unsigned char)e_kb[e], 0, ens[e].d, e, e * Ge + l};
-                q[e * Ge + l] = Queue{0, 0, 0, e_nc[e]};
-            }
-        }
+            while ((1ll << rlog) < len) rlog++;
+            gd.push_back(GroupDesc{roff, off, (unsigned char)rlog, (unsigned char)nc, (unsigned char)kb, 0, dim, e, (int)gd.size()});
+            q.push_back(Queue{0, 0, 0, nc});
+            roff += 1ll << rlog;
+        };
+        for (int e = 0; e < E; e++)
+            for (int l = 0; l < Ge; l++)
+                add(ens[e].n, g_off[e * Ge + l], P.split ? kMaxTile : e_nc[e], e_kb[e], ens[e].d, e);
+        if (P.split) add(n, 0, 1, 0, 0, 0);  // FP64 rechecks
         h->ring_len = (size_t)roff;
         P.q = upload(h, q);
         P.ring = (unsigned int *)dalloc(h, h->ring_len * sizeof(unsigned int));
         P.gd = upload(h, gd);
     }
+    if (P.split && !(P.chain = (int *)dalloc(h, (size_t)n * sizeof(int)))) return bail(QJX_ERR_OOM);
     const size_t nd_ = (size_t)h->cfg.max_dumps * n;
     P.o_norm = (double *)dalloc(h, nd_ * sizeof(double));
     P.o_mean = (double *)dalloc(h, nd_ * sizeof(double));
@@ -641,7 +642,7 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     P.r_type = (int *)dalloc(h, rc * sizeof(int));
     P.ctrl = (int *)dalloc(h, 16 * sizeof(int));
     P.work = (long long *)dalloc(h, 4 * sizeof(long long));
-    if (!P.psi || !P.st || !P.gn || (P.split ? !P.cnt || !P.lists : !P.q || !P.ring || !P.gd) || !P.o_norm || !P.o_mean || !P.o_disp || !P.o_m2 ||
+    if (!P.psi || !P.st || !P.gn || (P.flow ? !P.q || !P.ring || !P.gd : !P.cnt || !P.lists) || !P.o_norm || !P.o_mean || !P.o_disp || !P.o_m2 ||
         !P.o_energy || !P.o_robs || !P.o_adr || !P.mean_start || !P.r_time || !P.r_norm || !P.r_eta || !P.r_type ||
         !P.ctrl || !P.work)
         return bail(QJX_ERR_OOM);
@@ -814,26 +815,28 @@ static cudaError_t clear_queues(qjx_engine *h)
 {
     Params &P = h->P;
     cudaError_t e = cudaMemsetAsync(P.ctrl, 0, sizeof(int) * 16, h->stream);
-    if (P.split) {
+    if (P.split && e == cudaSuccess) e = cudaMemsetAsync(P.chain, 0, sizeof(int) * P.n, h->stream);
+    if (!P.flow) {
         if (e == cudaSuccess) e = cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream);
     } else {
         if (e == cudaSuccess) // the counts, not the sub-tile width
-            e = cudaMemset2DAsync(P.q, sizeof(Queue), 0, offsetof(Queue, nc), P.G, h->stream);
+            e = cudaMemset2DAsync(P.q, sizeof(Queue), 0, offsetof(Queue, nc), P.G + (P.split ? 1 : 0), h->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(P.ring, 0xff, sizeof(unsigned int) * h->ring_len, h->stream);
     }
     return e;
 }
 
-// Trajectories paused on full record buffers: drains the records and queues them again (the split
-// form's lists start over at step 0).
+// Trajectories paused on full record buffers: drains the records and queues them again (lock-step
+// lists start over at step 0).
 static qjx_status resume_paused(qjx_engine *h)
 {
     Params &P = h->P;
     const qjx_status rs = drain_records(h);
     if (rs != QJX_OK) return rs;
     CK(cudaMemsetAsync(P.ctrl + 2, 0, sizeof(int), h->stream));
-    if (P.split) {
+    if (P.split) CK(cudaMemsetAsync(P.chain, 0, sizeof(int) * P.n, h->stream));
+    if (!P.flow) {
         CK(cudaMemsetAsync(P.cnt, 0, sizeof(int) * 3 * P.G, h->stream));
         CK(cudaMemsetAsync(P.rcnt, 0, 3 * sizeof(int), h->stream));
     }
@@ -854,15 +857,17 @@ static int solo_ctas(const qjx_engine *h, int live)
     return C;
 }
 
-// Plain form: one launch per time slice until no trajectory is left.  Up to solo_max trajectories run
-// one to a CTA or cluster, more share sub-tiles.
-static qjx_status run_flow(qjx_engine *h, FILE *bucket_log, int64_t *nlaunch)
+// One launch per time slice until no trajectory is left.  Plain form: up to solo_max trajectories run
+// one to a CTA or cluster, more share sub-tiles.  Split form: `steps` gets the longest trajectory's
+// matvecs (the micro-steps that lock-step would take).
+static qjx_status run_flow(qjx_engine *h, FILE *bucket_log, int64_t *steps, int64_t *nlaunch)
 {
     Params &P = h->P;
     int live = P.n;
     while (true) {
         CK(cudaEventRecord(h->eb0, h->stream));
-        if (live <= h->solo_max) CK(launch_solo(P, solo_ctas(h, live), live, h->stream));
+        if (P.split) CK(launch_split_flow(P, std::min(h->grid, live), h->stream));
+        else if (live <= h->solo_max) CK(launch_solo(P, solo_ctas(h, live), live, h->stream));
         else CK(launch_flow(P, h->flow_nt, h->solo_max, std::min(h->flow_grid, live), h->stream));
         CK(cudaEventRecord(h->eb1, h->stream));
         *nlaunch += 1;
@@ -881,6 +886,13 @@ static qjx_status run_flow(qjx_engine *h, FILE *bucket_log, int64_t *nlaunch)
         }
         live = h->h_ctrl[kLive];
         if (live > 0) continue;
+        if (P.split) {
+            CK(launch_longest_chain(P, h->stream));
+            CK(cudaMemcpyAsync(h->h_ctrl + 11, P.sdone, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaStreamSynchronize(h->stream));
+            *steps += h->h_ctrl[11];
+            *nlaunch += 1;
+        }
         if (h->h_ctrl[2] == 0) return QJX_OK;
         rs = resume_paused(h);
         if (rs != QJX_OK) return rs;
@@ -888,10 +900,10 @@ static qjx_status run_flow(qjx_engine *h, FILE *bucket_log, int64_t *nlaunch)
     }
 }
 
-// Split form: one cooperative launch runs up to 6 x batch lock-step micro-steps with grid barriers
-// between them (the buffers rotate with period 6).  Step 0 reads the buckets in cnt[0] / lists[0]
+// Split form in lock step: 6 x batch micro-steps between host polls, one launch each (an empty one
+// returns at once; the buffers rotate with period 6).  Step 0 reads the buckets in cnt[0] / lists[0]
 // that the schedule or observe kernel wrote.
-static qjx_status run_split(qjx_engine *h, int64_t *steps, int64_t *nlaunch)
+static qjx_status run_lockstep(qjx_engine *h, int64_t *steps, int64_t *nlaunch)
 {
     Params &P = h->P;
     int s0 = 0;  // index of the next micro-step
@@ -899,20 +911,8 @@ static qjx_status run_split(qjx_engine *h, int64_t *steps, int64_t *nlaunch)
     while (true) {
         CK(cudaEventRecord(h->eb0, h->stream));
         CK(cudaMemsetAsync(P.sdone, 0, sizeof(int), h->stream));
-        cudaError_t e = h->split_coop ? launch_split_steps(P, s0, 6 * batch, h->grid, h->stream)
-                                      : cudaErrorCooperativeLaunchTooLarge;
-        if (e == cudaErrorCooperativeLaunchTooLarge) {
-            // not every CTA can be resident (another context holds SMs): the same micro-steps
-            // as one launch each (an empty step returns at once)
-            cudaGetLastError();
-            h->split_coop = false;
-            e = cudaSuccess;
-            for (int k = 0; k < 6 * batch && e == cudaSuccess; k++) e = launch_split_step(P, s0 + k, h->grid, h->stream);
-            *nlaunch += 6 * batch;
-        } else {
-            *nlaunch += 1;
-        }
-        if (e != cudaSuccess) return cuda_fail(h, e, "launch_split_steps");
+        for (int k = 0; k < 6 * batch; k++) CK(launch_split_step(P, s0 + k, h->grid, h->stream));
+        *nlaunch += 6 * batch;
         CK(cudaEventRecord(h->eb1, h->stream));
         // the micro-steps run, the recheck counts and the next step's tiles
         CK(cudaMemcpyAsync(h->h_ctrl + 8, P.rcnt, 3 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -944,14 +944,14 @@ static qjx_status run_split(qjx_engine *h, int64_t *steps, int64_t *nlaunch)
 static qjx_status run_until_idle(qjx_engine *h)
 {
     Params &P = h->P;
-    // QJX_TRACE_BUCKETS=<file>: append the queue sizes seen at every host poll (plain form; profiling aid)
+    // QJX_TRACE_BUCKETS=<file>: append the queue sizes seen at every host poll (profiling aid)
     FILE *bucket_log = nullptr;
     if (const char *fn = getenv("QJX_TRACE_BUCKETS")) bucket_log = fopen(fn, "a");
     int64_t steps = 0, nlaunch = 0;
     long long work0[4] = {0, 0, 0, 0};
     cudaMemcpy(work0, P.work, 4 * sizeof(long long), cudaMemcpyDeviceToHost);
     cudaEventRecord(h->ev0, h->stream);
-    const qjx_status rs = P.split ? run_split(h, &steps, &nlaunch) : run_flow(h, bucket_log, &nlaunch);
+    const qjx_status rs = P.flow ? run_flow(h, bucket_log, &steps, &nlaunch) : run_lockstep(h, &steps, &nlaunch);
     if (bucket_log) fclose(bucket_log);
     cudaEventRecord(h->ev1, h->stream);
     cudaEventSynchronize(h->ev1);

@@ -23,8 +23,7 @@
 // FP64 has no tcgen05 kind, so the plain form's contraction runs on the FP64 tensor core
 // (mma.sync m8n8k4 f64), laid out so that every output keeps the oracle's k-ascending fma
 // chain (bit-identical results).  The split-precision form (qjx_split.cuh, included at the
-// end) runs lock-step micro-steps over the same buckets with bf16x3 products on the tcgen05 tensor
-// cores.
+// end) runs the same queues with bf16x3 products on the tcgen05 tensor cores.
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -129,11 +128,11 @@ __device__ __forceinline__ unsigned entry_of(int tr, const TrajState &s)
     return ((unsigned)tr << 3) | (unsigned)src_slot(s.phase, s.cur, s.rk_stage);
 }
 
-// Appends trajectory tr to bucket g before a run: the split form's lists of step 0, or the plain
-// form's queue (its entries past the tail are free).
+// Appends trajectory tr to bucket g before a run: to its queue (whose entries past the tail are
+// free), or the lock-step lists of step 0.
 __device__ __forceinline__ void enqueue(const Params &P, int g, int tr)
 {
-    if (P.split) {
+    if (!P.flow) {
         const int pos = atomicAdd(&P.cnt[g], 1);
         P.lists[P.g_loff[g] + pos] = tr;
     } else {
@@ -827,12 +826,12 @@ struct Pick {
 };
 
 // Looks the queues over (one warp, converged): a claim is at most NCM trajectories and an equal share
-// of the unfinished ones in whole 8-column blocks (NCM = 1: one trajectory).  Any queue that has the
-// share waiting will do (a different one for each CTA and attempt, so that claims spread), else the
-// fullest.  Queues are scanned 256 at a time from a place that differs by CTA, up to the first 256
-// with a share waiting.
+// of the unfinished ones in whole 8-column blocks, or `least` if that is more (NCM = 1: one
+// trajectory).  Any queue that has the share waiting will do (a different one for each CTA and
+// attempt, so that claims spread), else the fullest.  Queues are scanned 256 at a time from a place
+// that differs by CTA, up to the first 256 with a share waiting.
 template <int NCM>
-__device__ __forceinline__ Pick scan(const Params &P, int stop_live, unsigned &turn, int lane)
+__device__ __forceinline__ Pick scan(const Params &P, int stop_live, int least, unsigned &turn, int lane)
 {
     const int G = P.G, chunks = (G + 255) / 256;
     turn += 7u;
@@ -852,7 +851,7 @@ __device__ __forceinline__ Pick scan(const Params &P, int stop_live, unsigned &t
                 cap[i] = v.w;
             }
         }
-        share = min(NCM, 8 * ((live + 8 * (int)gridDim.x - 1) / (8 * (int)gridDim.x)));
+        share = min(NCM, max(least, 8 * ((live + 8 * (int)gridDim.x - 1) / (8 * (int)gridDim.x))));
         int b = 0, bi = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
@@ -874,34 +873,32 @@ __device__ __forceinline__ Pick scan(const Params &P, int stop_live, unsigned &t
     return pick;
 }
 
-// Takes trajectories from a queue (one warp, converged), from `pick` first if that has any: lane
-// i < n gets the i-th entry in `en`, gd the queue's descriptor.  Returns n, or 0: the call's work is
-// done, the slice is over, or nothing turned up for kIdleNs.  A claim is two atomics that cannot
-// fail (a claim by compare-and-swap of the head, before, was lost to another CTA four times in five
-// at d = 51): what the count of available entries grants, then as many positions.  What was written
-// about the trajectories before their entries is visible to this SM afterwards.
-template <int NCM>
-__device__ __forceinline__ int take(const Params &P, unsigned long long t_end, int stop_live, Pick pick, unsigned &turn,
-                                    int lane, GroupDesc &gd, unsigned &en)
+// A claim (one warp, converged): from `pick` first if that has any, else from what look() returns.
+// Returns how many trajectories it got, 0 when the call's work is done, the slice is over, or
+// nothing turned up for kIdleNs; gd is the queue's descriptor, pos the first entry's position.
+// A claim is two atomics that cannot fail (a claim by compare-and-swap of the head, before, was lost
+// to another CTA four times in five at d = 51): what the count of available entries grants, then as
+// many positions.
+template <int NCM, class Look>
+__device__ __forceinline__ int grant(const Params &P, unsigned long long t_end, const Look &look, Pick pick, int lane,
+                                     GroupDesc &gd, unsigned &pos)
 {
     // a queue that others have nearly emptied since it was looked at is passed over this many times:
     // a sub-tile of a few columns costs as much tensor time as a full block of eight
     constexpr int kTries = 2;
     unsigned long long t_idle = 0;
     int n = 0, tries = 0;
-    unsigned pos = 0;
-    en = kFree;
     while (true) {
-        if (pick.n == 0) pick = scan<NCM>(P, stop_live, turn, lane);
-        const unsigned long long now = global_ns();
+        if (pick.n == 0) pick = look();
+        const unsigned long long now = __shfl_sync(0xffffffffu, global_ns(), 0);
         if (pick.n < 0 || now >= t_end) return 0;
         if (pick.n > 0) {
             gd = load_desc(P.gd + pick.g);
             if (lane == 0) {
                 Queue *q = P.q + pick.g;
-                const int want = (pick.n > 16 && pick.n <= 24) ? 16 : pick.n;  // no sub-tile of 3 column blocks
-                n = max(0, min(want, atomicSub(&q->avail, want)));
-                if (n > 16 && n <= 24) n = 16;
+                auto whole = [](int m) { return NCM == 32 && m > 16 && m <= 24 ? 16 : m; };  // no 3 column blocks
+                const int want = whole(pick.n);
+                n = whole(max(0, min(want, atomicSub(&q->avail, want))));
                 if (4 * n < 3 * want && tries < kTries) n = 0;
                 if (n < want) atomicAdd(&q->avail, want - n);
                 if (n > 0) pos = atomicAdd(&q->head, (unsigned)n);
@@ -917,10 +914,27 @@ __device__ __forceinline__ int take(const Params &P, unsigned long long t_end, i
         __nanosleep(50);
     }
     pos = __shfl_sync(0xffffffffu, pos, 0);
-    if (lane < n) {
-        unsigned *entry = P.ring + gd.roff + ((pos + (unsigned)lane) & gd.rmask());
-        for (long long i = 0; i < kWaitLimit && en == kFree; i++) en = atomicExch(entry, kFree);
-    }
+    return n;
+}
+
+// The entry at a claimed position (kFree when it was never published: the bounded wait gave up).
+__device__ __forceinline__ unsigned take_entry(const Params &P, const GroupDesc &gd, unsigned pos)
+{
+    unsigned en = kFree;
+    unsigned *entry = P.ring + gd.roff + (pos & gd.rmask());
+    for (long long i = 0; i < kWaitLimit && en == kFree; i++) en = atomicExch(entry, kFree);
+    return en;
+}
+
+// A claim of up to NCM <= 32 trajectories with its entries: lane i < n gets the i-th in `en`.  What
+// was written about the trajectories before their entries is visible to this SM afterwards.
+template <int NCM>
+__device__ __forceinline__ int take(const Params &P, unsigned long long t_end, int stop_live, Pick pick, unsigned &turn,
+                                    int lane, GroupDesc &gd, unsigned &en)
+{
+    unsigned pos = 0;
+    const int n = grant<NCM>(P, t_end, [&] { return scan<NCM>(P, stop_live, 0, turn, lane); }, pick, lane, gd, pos);
+    en = lane < n ? take_entry(P, gd, pos + (unsigned)lane) : kFree;
     __threadfence();  // acquire
     if (__any_sync(0xffffffffu, lane < n && en == kFree)) {  // never published: report and stop
         if (lane == 0) {
@@ -932,28 +946,28 @@ __device__ __forceinline__ int take(const Params &P, unsigned long long t_end, i
     return n;
 }
 
-// Appends trajectories to their next queues (one warp, converged): lane i < n has the bucket g2 and
-// the entry `en` of one, -1 when it is finished, paused or failed.  Lanes with the same bucket find
-// each other, the lowest reserves the run.
-__device__ void append(const Params &P, int g2, unsigned en, int n, int lane)
+// Appends trajectories to their next queues (one warp, converged): lanes with `has` have the bucket
+// g2 and the entry `en` of one, -1 when it is finished, paused or failed.  Lanes with the same bucket
+// find each other, the lowest reserves the run.
+__device__ void append_lanes(const Params &P, bool has, int g2, unsigned en, int lane)
 {
     __threadfence();  // release: what the CTA wrote, before the entries
-    const unsigned m = __match_any_sync(0xffffffffu, g2);
+    const int key = has ? g2 : -2;
+    const unsigned m = __match_any_sync(0xffffffffu, key);
     const int leader = __ffs(m) - 1;
     GroupDesc gd{};
-    if (g2 >= 0) gd = load_desc(P.gd + g2);
+    if (key >= 0) gd = load_desc(P.gd + key);
     unsigned base = 0;
     if (lane == leader) {
-        if (g2 >= 0) {
-            base = atomicAdd(&P.q[g2].tail, (unsigned)__popc(m));
-            atomicAdd(&P.q[g2].avail, __popc(m));
-        } else {
-            const int gone = __popc(m) - (32 - n);  // lanes past n are in this set too
-            if (gone > 0) atomicSub(P.ctrl + kLive, gone);
+        if (key >= 0) {
+            base = atomicAdd(&P.q[key].tail, (unsigned)__popc(m));
+            atomicAdd(&P.q[key].avail, __popc(m));
+        } else if (key == -1) {
+            atomicSub(P.ctrl + kLive, __popc(m));
         }
     }
     base = __shfl_sync(0xffffffffu, base, leader);
-    bool put = g2 < 0;
+    bool put = key < 0;
     unsigned *entry = P.ring + gd.roff + ((base + (unsigned)__popc(m & ((1u << lane) - 1u))) & gd.rmask());
     for (long long i = 0; i < kWaitLimit && !put; i++) put = atomicCAS(entry, kFree, en) == kFree;
     if (!put) {
@@ -1025,7 +1039,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) flow_kernel(const Param
         const int nbd = P.nb * P.deep;
         const Ens sys{dg, s_gd.ens * P.Ge, nbd <= kMaxDt ? s_dt : P.e_dt + (size_t)s_gd.ens * nbd,
                     P.e_rate + (size_t)s_gd.ens * P.nd};
-        if (warp == 0) hint = scan<NCM>(P, stop_live, turn, lane);
+        if (warp == 0) hint = scan<NCM>(P, stop_live, 0, turn, lane);
         else if (nbd <= kMaxDt && tid >= 32 && tid < 32 + nbd) s_dt[tid - 32] = __ldg(P.e_dt + (size_t)s_gd.ens * nbd + tid - 32);
         const long long t1 = clock64();
         if constexpr (NT == 256) {
@@ -1052,7 +1066,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) flow_kernel(const Param
         __syncthreads();
         // warp 1 appends while warp 0 takes the next sub-tile (s_g2 and s_entry are rewritten after that
         // sub-tile's products)
-        if (warp == 1) append(P, lane < ncol ? s_g2[lane] : -1, lane < ncol ? s_entry[lane] : kFree, ncol, lane);
+        if (warp == 1) append_lanes(P, lane < ncol, lane < ncol ? s_g2[lane] : -1, lane < ncol ? s_entry[lane] : kFree, lane);
         if (tid == 0) tally.add(ncol, (ncb == 3) ? 4 : ncb, t0, t1, t2, clock64());
     }
     if (tid == 0) tally.flush(P);
@@ -1749,12 +1763,12 @@ bool pick_step_tiles(int MD, size_t budget, int nt, int nc_max, int *nc, int *kb
     return false;
 }
 
-// The split form's first micro-step after a host-side enqueue needs its plan.
+// The first lock-step micro-step after a host-side enqueue needs its plan.
 cudaError_t launch_split_plan(const Params &P, cudaStream_t st);
 
 static cudaError_t launch_plan(const Params &P, cudaStream_t st)
 {
-    return P.split ? launch_split_plan(P, st) : cudaGetLastError();
+    return P.flow ? cudaGetLastError() : launch_split_plan(P, st);
 }
 
 cudaError_t launch_schedule(const Params &P, int mode, cudaStream_t st)
@@ -1903,45 +1917,47 @@ cudaError_t launch_split_plan(const Params &P, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// Static shared memory of the split kernel.
+// Static shared memory of the split kernel (the same in both modes).
 size_t split_static_smem()
 {
-    cudaFuncAttributes a{};
-    if (cudaFuncGetAttributes(&a, split_step_kernel) != cudaSuccess) return 32768;
-    return a.sharedSizeBytes;
+    cudaFuncAttributes a{}, b{};
+    if (cudaFuncGetAttributes(&a, split_kernel<true>) != cudaSuccess ||
+        cudaFuncGetAttributes(&b, split_kernel<false>) != cudaSuccess)
+        return 32768;
+    return std::max(a.sharedSizeBytes, b.sharedSizeBytes);
 }
 
-static cudaError_t split_smem_attr(size_t smem)
+template <bool FLOW>
+static cudaError_t launch_split(const Params &P, int s, int grid, cudaStream_t st)
 {
-    static int attr_bytes = 0;
-    if (attr_bytes < (int)smem) {
-        cudaError_t e = cudaFuncSetAttribute(split_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr_bytes = (int)smem;
-    }
-    return cudaSuccess;
-}
-
-cudaError_t launch_split_step(const Params &P, int s, int grid, cudaStream_t st)
-{
-    const size_t smem = split_smem_bytes(P.MDs, P.MD, P.sstages);
-    cudaError_t e = split_smem_attr(smem);
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e = allow_smem(split_kernel<FLOW>, done);
     if (e != cudaSuccess) return e;
-    split_step_kernel<<<grid, kThreads, smem, st>>>(P, s, 1);
+    split_kernel<FLOW><<<grid, kThreads, split_smem_bytes(P.MDs, P.MD, P.sstages), st>>>(P, s);
     return cudaGetLastError();
 }
 
-// Micro-steps s0 .. s0 + nsteps - 1 in one launch (fewer when the work runs out first; the
-// count is left in P.sdone): a cooperative launch, so that every CTA is resident for the grid
-// barriers between the steps.
-cudaError_t launch_split_steps(const Params &P, int s0, int nsteps, int grid, cudaStream_t st)
+// One time slice of the split form, or its lock-step micro-step s.
+cudaError_t launch_split_flow(const Params &P, int grid, cudaStream_t st) { return launch_split<true>(P, 0, grid, st); }
+cudaError_t launch_split_step(const Params &P, int s, int grid, cudaStream_t st) { return launch_split<false>(P, s, grid, st); }
+
+// The most matvecs (rechecks included) of one trajectory since the counts were cleared, into P.sdone.
+__global__ void __launch_bounds__(1024) longest_chain_kernel(const Params P)
 {
-    const size_t smem = split_smem_bytes(P.MDs, P.MD, P.sstages);
-    cudaError_t e = split_smem_attr(smem);
-    if (e != cudaSuccess) return e;
-    Params Pc = P;
-    void *args[] = {&Pc, &s0, &nsteps};
-    return cudaLaunchCooperativeKernel((const void *)split_step_kernel, dim3(grid), dim3(kThreads), args, smem, st);
+    __shared__ int s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    int m = 0;
+    for (int i = threadIdx.x; i < P.n; i += 1024) m = max(m, P.chain[i]);
+    atomicMax(&s_max, m);
+    __syncthreads();
+    if (threadIdx.x == 0) *P.sdone = s_max;
+}
+
+cudaError_t launch_longest_chain(const Params &P, cudaStream_t st)
+{
+    longest_chain_kernel<<<1, 1024, 0, st>>>(P);
+    return cudaGetLastError();
 }
 
 }  // namespace qjx

@@ -1,7 +1,7 @@
 // qjx_split.cuh -- the split-precision micro-step on the tcgen05 tensor cores (precision 1).
 //
-// Same lock-step micro-steps, buckets and trajectory state machine as the FP64 plain form;
-// only the d x d complex matvec changes.  Roles are transposed against the FP64 kernel so that
+// Same queues, independent CTAs and trajectory state machine as the FP64 plain form; only the d x d
+// complex matvec changes.  Roles are transposed against the FP64 kernel so that
 // the trajectory, not the matrix row, is the MMA M dimension, and the complex product is four
 // real GEMMs sharing operands:
 //
@@ -37,12 +37,18 @@
 //   warps 14-15 load the tile's trajectory records meanwhile
 // then the FP32 accumulators of up to 64 trajectories at a time are staged in the idle ring by
 // the warps that own their TMEM lane quarters, and every warp runs its trajectories through the
-// epilogue and appends them to their next buckets.  A batched engine's ensembles each have their
-// own padded rows and k-steps; the tile plan of the next micro-step (rows per tile, first tile of
-// every bucket) is made by the last CTA to finish one.  One cooperative launch runs a batch of
-// micro-steps: between two of them every CTA waits at a grid barrier (an arrival counter, and a
-// generation number the planning CTA releases), and the operand ring, mbarriers and tensor
-// memory stay set up across them.
+// epilogue and appends them to their next queues.  A batched engine's ensembles each have their
+// own padded rows and k-steps.  A CTA takes an equal share of the unfinished trajectories from the
+// queue of one matrix (or one trajectory from the queue of FP64 rechecks, first), and keeps its
+// operand ring, mbarriers and tensor memory from tile to tile for a time slice.
+// (One cooperative launch of lock-step micro-steps with a grid barrier and a plan between them before
+// this: at d = 201 with 10^4 trajectories a CTA was busy 46 % of the time, the rest went on waiting
+// for the slowest tile and on the plan; 232 ms of kernel time for a period, now 197.  A tile, of 50
+// rows on average, now takes 15 k cycles to claim, the wait for work at the end of the period
+// included, 24 k of MMAs whatever its rows, and 23 k of epilogue.)
+// With QJX_SPLIT_COOP=0 the same tiles run as lock-step micro-steps, one launch each, over bucket
+// lists and a tile plan (rows per tile, first tile of every bucket) that the last CTA of a
+// micro-step makes for the next.
 
 constexpr int kAPlanes = 4;                  // A and B planes: Re hi, Re lo, Im hi, Im lo
 constexpr int kTileM = 128;                  // MMA M = TMEM lanes (a tile holds up to 128 trajectories)
@@ -50,19 +56,6 @@ constexpr int kMaxSStages = kMaxSplitStages;  // operand ring depth (runtime: th
 constexpr int kABytes = kTileM * 32;         // one plane of one k-step of A: 128 rows x 16 bf16
 constexpr int kTmemCols = 512;
 constexpr long long kSplitWait = 1ll << 20;  // bounded mbarrier polls (normal waits end within microseconds)
-constexpr long long kGridWait = 1ll << 24;   // bounded polls of the grid barrier (a micro-step is ~50 us)
-
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p)
-{
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned int *p, unsigned int v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 __device__ __forceinline__ uint64_t umma_desc_kmajor(uint32_t saddr)
 {
     return (uint64_t)((saddr >> 4) & 0x3FFFu)        // start address
@@ -148,10 +141,11 @@ __device__ __forceinline__ void split_pair(double2 v, uint32_t &hi, uint32_t &lo
 // FP64 recheck of one trajectory's step: y = M x with the plain form's arithmetic (per output the
 // k-ascending fma chain of the contract, k up to the even kp), the matrix streamed through the free
 // operand ring in slabs of kb k rows by TMA bulk copies (two buffers, mbarriers rbar[0..1]), then
-// the epilogue decides with the FP64 norm and the trajectory joins its next bucket.  Whole CTA;
-// returns false when a bounded wait gave up.
+// the epilogue decides with the FP64 norm and emit(lane, bucket, entry) sends the trajectory on (warp
+// 0).  Whole CTA; returns false when a bounded wait gave up.
+template <class Emit>
 __device__ bool recheck_column(const Params &P, int tr, unsigned char *smem, TrajState *st_s, uint64_t *rbar,
-                               uint32_t &rphase, int *cnt_next, int *list_next)
+                               uint32_t &rphase, const Emit &emit)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) load_state(st_s, &P.st[tr]);
@@ -206,10 +200,7 @@ __device__ bool recheck_column(const Params &P, int tr, unsigned char *smem, Tra
     if (warp == 0) {
         unsigned entry;
         const int g2 = column_epilogue(P, ys, tr, st, lane, entry, global_ens(P, st.ens), global_slots(P, tr), &P.st[tr], true);
-        if (g2 >= 0 && lane == 0) {
-            const int pos = atomicAdd(&cnt_next[g2], 1);
-            list_next[P.g_loff[g2] + pos] = tr;
-        }
+        emit(lane == 0, g2, entry);
     }
     fence_proxy_async();  // generic writes to the ring before later bulk copies into it
     __syncthreads();
@@ -354,18 +345,21 @@ size_t split_smem_bytes(int MDs, int MD, int stages)
     return ring > epi ? ring : epi;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P, int s0, int nsteps)
+// FLOW: tiles from the queues until the call's trajectories are done or the time slice is over (s0 is
+// not used); else the tiles of lock-step micro-step s0.
+template <bool FLOW>
+__global__ void __launch_bounds__(kThreads, 1) split_kernel(const Params P, int s0)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int S = P.sstages;
     const size_t stage_bytes = (size_t)kAPlanes * (kABytes + (size_t)P.MDs * 32);  // ring stride (largest MDs)
     __shared__ __align__(8) uint64_t fullA[kMaxSStages], fullB[kMaxSStages], empty[kMaxSStages], accf, rbar[2];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_tr[kTileM];
+    __shared__ int s_tr[kTileM];  // (FLOW: first the entries taken)
     __shared__ long long s_src[kTileM];
     __shared__ __align__(16) TrajState s_st[kTileM];
-    __shared__ int s_fail, s_last;
-    __shared__ unsigned int s_gen;
+    __shared__ int s_fail, s_n;  // s_n: columns taken (FLOW), or whether this CTA is the last of the micro-step
+    __shared__ int s_g;
     __shared__ int w_g2[kThreads / 32][kTileM / (kThreads / 32)];  // per warp: its trajectories' next buckets
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -404,32 +398,82 @@ __global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P,
     bool ok = true;
     long long tr_setup = 0, tr_mma = 0, tr_stage = 0, tr_epi = 0;
     const long long t_begin = clock64();
-    int steps_done = 0;
+    const unsigned long long t_end = FLOW ? global_ns() + kSliceNs : 0;
+    unsigned turn = blockIdx.x;
 
-    // micro-steps s0 .. s0 + nsteps - 1 (one, when launched per step); between two steps of one
-    // launch every CTA waits at a grid barrier whose last arrival plans the next step
-    for (int si = 0; si < nsteps; si++) {
-        const int s = s0 + si;
-        const int *cnt_cur = P.cnt + (s % 3) * G;
-        int *cnt_next = P.cnt + ((s + 1) % 3) * G;
-        const int *list_cur = P.lists + (size_t)(s & 1) * P.ltot;
-        int *list_next = P.lists + (size_t)((s + 1) & 1) * P.ltot;
-        const int *rlist_cur = P.rlist + (size_t)(s & 1) * P.n;
-        int *rlist_next = P.rlist + (size_t)((s + 1) & 1) * P.n;
-        int *rcnt_next = P.rcnt + (s + 1) % 3;
-        const int Rtot = __ldcg(P.rcnt + s % 3);  // FP64 rechecks of this micro-step
-        const int Rw = __ldcg(P.splan), T = __ldcg(P.splan + 1 + G);  // this step's plan (rows per tile, tiles)
-        const int R = Rw & 0xFFFF;
-        const bool heavy_fewer = (Rw >> 16) != 0;
-        if (T + Rtot == 0) break;  // nothing left in this call (every CTA reads the same plan)
-        if (blockIdx.x == 0) {
-            for (int i = tid; i < G; i += kThreads) P.cnt[((s + 2) % 3) * G + i] = 0;
-            if (tid == 0) P.rcnt[(s + 2) % 3] = 0;
+    // lock-step: this micro-step's lists and plan (rows per tile, tiles)
+    int *const cnt_next = FLOW ? nullptr : P.cnt + ((s0 + 1) % 3) * G;
+    int *const list_next = FLOW ? nullptr : P.lists + (size_t)((s0 + 1) & 1) * P.ltot;
+    int *const rlist_next = FLOW ? nullptr : P.rlist + (size_t)((s0 + 1) & 1) * P.n;
+    int *const rcnt_next = FLOW ? nullptr : P.rcnt + (s0 + 1) % 3;
+    const int Rtot = FLOW ? 0 : __ldcg(P.rcnt + s0 % 3);  // FP64 rechecks of this micro-step
+    const int Rw = FLOW ? 0 : __ldcg(P.splan), T = FLOW ? 0 : __ldcg(P.splan + 1 + G);
+    const bool some = FLOW || T + Rtot > 0;
+    // (an empty step too: the launches after it must not see the counts of three steps before)
+    if (!FLOW && blockIdx.x == 0) {
+        for (int i = tid; i < G; i += kThreads) P.cnt[((s0 + 2) % 3) * G + i] = 0;
+        if (tid == 0) P.rcnt[(s0 + 2) % 3] = 0;
+    }
+    // sends the trajectories of a warp's lanes with `has` on (converged): next bucket g2, queue entry en
+    auto emit = [&](bool has, int g2, unsigned en) {
+        if (FLOW) {
+            __syncwarp();
+            append_lanes(P, has, g2 == kRecheck ? G : g2, en, lane);
+            if (has) atomicAdd(&P.chain[en >> 3], 1);
+        } else if (has) {
+            if (g2 >= 0) {
+                const int pos = atomicAdd(&cnt_next[g2], 1);
+                list_next[P.g_loff[g2] + pos] = (int)(en >> 3);
+            } else if (g2 == kRecheck) {
+                rlist_next[atomicAdd(rcnt_next, 1)] = (int)(en >> 3);
+            }
         }
-
-        for (int t = blockIdx.x; t < T + Rtot && ok; t += gridDim.x) {
-            if (t >= T) {  // an FP64 recheck (the CTAs past the split tiles take these first)
-                if (!recheck_column(P, rlist_cur[t - T], smem, &s_st[0], rbar, rphase, cnt_next, list_next)) {
+    };
+    {
+        for (int t = blockIdx.x; ok && (FLOW || t < T + Rtot); t += gridDim.x) {
+            if (FLOW) {
+                const long long t0 = clock64();
+                if (warp == 0) {
+                    GroupDesc gd{};
+                    unsigned pos = 0;
+                    const int m = grant<kTileM>(
+                        P, t_end,
+                        [&] {
+                            Pick pick = scan<kTileM>(P, 0, P.min_rows, turn, lane);
+                            if (pick.n >= 0 && __ldcg(&P.q[G].avail) > 0) pick = Pick{1, G};  // FP64 rechecks first
+                            return pick;
+                        },
+                        Pick{0, 0}, lane, gd, pos);
+                    bool got = true;
+                    for (int i = lane; i < m; i += 32) {
+                        const unsigned en = take_entry(P, gd, pos + (unsigned)i);
+                        got = got && en != kFree;
+                        s_tr[i] = (int)en;
+                    }
+                    __threadfence();  // acquire
+                    if (!__all_sync(0xffffffffu, got) && lane == 0) s_fail = 1;
+                    if (lane == 0) {
+                        s_n = m;
+                        s_g = gd.group;
+                    }
+                }
+                __syncthreads();
+                if (s_fail) {
+                    ok = false;
+                    break;
+                }
+                if (s_n == 0) break;
+                if (s_g == G) {
+                    const int tr = (int)((unsigned)s_tr[0] >> 3);
+                    __syncthreads();
+                    if (!recheck_column(P, tr, smem, &s_st[0], rbar, rphase, emit)) ok = false;
+                    work += 1;
+                    nrechk += 1;
+                    continue;
+                }
+                tr_setup += clock64() - t0;
+            } else if (t >= T) {  // an FP64 recheck (the CTAs past the split tiles take these first)
+                if (!recheck_column(P, P.rlist[(size_t)(s0 & 1) * P.n + t - T], smem, &s_st[0], rbar, rphase, emit)) {
                     ok = false;
                     break;
                 }
@@ -438,22 +482,32 @@ __global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P,
                 continue;
             }
             const long long t0 = clock64();
-            const int g = split_tile_group(P, t, lane);  // every warp finds it (warp-uniform)
+            const int g = FLOW ? s_g : split_tile_group(P, t, lane);  // (every warp finds it)
             const int e = P.g_ens[g];
             const int d = P.e_d[e], MDs = P.e_mds[e], KS = P.e_ks[e], bbytes = MDs * 32;
-            const int Rg = group_rows(R, heavy_fewer && g - P.e_g0[e] >= P.nb * P.deep);
-            const int base = (t - __ldcg(P.splan + 1 + g)) * Rg;
-            const int rows = min(Rg, __ldcg(cnt_cur + g) - base);
-            if (tid < kTileM) {
-                if (tid < rows) {
-                    const int tr = list_cur[P.g_loff[g] + base + tid];
-                    const TrajState *sp = &P.st[tr];
-                    const int slot = src_slot(sp->phase, sp->cur, sp->rk_stage);
-                    s_tr[tid] = tr;
-                    s_src[tid] = ((long long)slot * n + tr) * P.MD;
-                } else {
-                    s_tr[tid] = -1;
-                    s_src[tid] = -1;
+            int rows = s_n;
+            if (FLOW) {
+                if (tid < kTileM) {
+                    const unsigned en = (unsigned)s_tr[tid];
+                    const int tr = (int)(en >> 3);
+                    s_tr[tid] = tid < rows ? tr : -1;
+                    s_src[tid] = tid < rows ? ((long long)(en & 7u) * n + tr) * P.MD : -1;
+                }
+            } else {
+                const int Rg = group_rows(Rw & 0xFFFF, (Rw >> 16) != 0 && g - P.e_g0[e] >= P.nb * P.deep);
+                const int base = (t - __ldcg(P.splan + 1 + g)) * Rg;
+                rows = min(Rg, __ldcg(P.cnt + (s0 % 3) * G + g) - base);
+                if (tid < kTileM) {
+                    if (tid < rows) {
+                        const int tr = P.lists[(size_t)(s0 & 1) * P.ltot + P.g_loff[g] + base + tid];
+                        const TrajState *sp = &P.st[tr];
+                        const int slot = src_slot(sp->phase, sp->cur, sp->rk_stage);
+                        s_tr[tid] = tr;
+                        s_src[tid] = ((long long)slot * n + tr) * P.MD;
+                    } else {
+                        s_tr[tid] = -1;
+                        s_src[tid] = -1;
+                    }
                 }
             }
             __syncthreads();
@@ -608,27 +662,24 @@ __global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P,
                 // every warp runs its trajectories (columns warp, warp + 16, ...) through the epilogue,
                 // then appends them to their next buckets with one atomic each, all in flight together
                 const int pn = min(RP, rows - p0);
-                int nm = 0;
+                int nm = 0, slots8 = 0;  // slots8: the queue entries' slots, three bits per trajectory
                 for (int cc = warp; cc < pn; cc += kThreads / 32, nm++) {
                     const int m = p0 + cc;
                     const float *row = sacc + (size_t)cc * SR;
                     for (int k = lane; k < MDs; k += 32) wcol[k] = make_double2((double)row[k], (double)row[MDs + k]);
                     __syncwarp();
                     unsigned entry;
-                    const int g2 = column_epilogue(P, wcol, s_tr[m], s_st[m], lane, entry, sys,
-                                                   global_slots(P, s_tr[m]), &P.st[s_tr[m]], true);
+                    const int g2 = column_epilogue(P, wcol, s_tr[m], s_st[m], lane, entry, sys, global_slots(P, s_tr[m]),
+                                                   &P.st[s_tr[m]], true);
                     if (lane == 0) w_g2[warp][nm] = g2;
+                    slots8 |= (int)(entry & 7u) << (3 * nm);
                     __syncwarp();
                 }
-                if (lane < nm) {
-                    const int g2 = w_g2[warp][lane];
-                    const int tr = s_tr[p0 + warp + (kThreads / 32) * lane];
-                    if (g2 >= 0) {
-                        const int pos = atomicAdd(&cnt_next[g2], 1);
-                        list_next[P.g_loff[g2] + pos] = tr;
-                    } else if (g2 == kRecheck) {
-                        rlist_next[atomicAdd(rcnt_next, 1)] = tr;
-                    }
+                {
+                    const bool has = lane < nm;
+                    const int g2 = has ? w_g2[warp][lane] : -1;
+                    const int tr = has ? s_tr[p0 + warp + (kThreads / 32) * lane] : 0;
+                    emit(has, g2, ((unsigned)tr << 3) | (unsigned)((slots8 >> (3 * (lane & 7))) & 7));
                 }
                 fence_proxy_async();  // generic writes to the ring before the next tile's bulk copies
                 __syncthreads();
@@ -640,39 +691,22 @@ __global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P,
             tr_mma += t2 - t1;
             tr_epi += t3 - t2;
         }
-
-        steps_done++;
-        if (!ok && tid == 0) atomicAdd(&P.ctrl[4], 1);  // every CTA stops after the barrier below
-        // the last CTA to finish plans the next micro-step from the buckets all CTAs filled; with a
-        // next step in this launch the others wait for that plan (bounded), then read it
+    }
+    if (!ok && tid == 0) atomicAdd(&P.ctrl[4], 1);
+    if (!FLOW && some) {
+        // the last CTA to finish plans the next micro-step from the buckets all CTAs filled
         __syncthreads();
         if (tid == 0) {
             __threadfence();
-            s_gen = ld_acquire_u32(P.gen);
-            s_last = atomicAdd(P.plan_sync, 1u) == gridDim.x - 1;
+            s_n = atomicAdd(P.plan_sync, 1u) == gridDim.x - 1;
         }
         __syncthreads();
-        const bool more = si + 1 < nsteps;
-        if (s_last) {
+        if (s_n) {
             __threadfence();
             split_plan(P, cnt_next, __ldcg(rcnt_next), gridDim.x);
-            if (tid == 0) {
-                *P.plan_sync = 0u;
-                __threadfence();
-                st_release_u32(P.gen, s_gen + 1u);
-            }
-        } else if (more && tid == 0) {
-            long long i = 0;
-            while (ld_acquire_u32(P.gen) == s_gen && i < kGridWait) i++;
-            if (i == kGridWait) {
-                atomicAdd(&P.ctrl[4], 1);
-                report_error(P, -1, ERR_TIMEOUT);
-            }
+            if (tid == 0) *P.plan_sync = 0u;
         }
-        __syncthreads();
-        __threadfence();
-        if (!more || !ok || __ldcg(P.ctrl + 4) != 0) break;
-    }  // micro-steps
+    }
 
     if (!ok) {
         // give the copies and MMAs still in flight time to land before the memory goes away
@@ -712,5 +746,5 @@ __global__ void __launch_bounds__(kThreads, 1) split_step_kernel(const Params P,
         tr[6] += tr_stage;
         tr[7] += work;
     }
-    if (blockIdx.x == 0 && tid == 0 && steps_done) atomicAdd(P.sdone, steps_done);
+    if (!FLOW && some && blockIdx.x == 0 && tid == 0) atomicAdd(P.sdone, 1);
 }
