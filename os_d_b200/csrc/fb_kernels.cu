@@ -297,9 +297,9 @@ __device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity)
 // acknowledged.  Two mbarriers and two arguments are enough: a CTA can send entries of stage s + 1
 // only after it has all of stage s, so after every CTA has finished reading the argument of stage s
 // (the one that stage s + 1 overwrites is that of stage s - 1).  One warp works out the next step's
-// drive values meanwhile.  Bound: the latency of a stage (gather, row sum, st.async, mbarrier), about
-// 0.5 us.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread its own
-// sine): 2.9 us a stage at N = 50.
+// drive values meanwhile.  Bound: the latency of a stage (gather, row sum, st.async, mbarrier),
+// 1.6 us at N = 50.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread
+// its own sine): 2.9 us.
 __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResParams P, int cs)
 {
     extern __shared__ __align__(16) unsigned char fsm[];
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
 // ---- grid form: systems too large for a cluster, on every SM
 // The rows of the system over all CTAs of one cooperative launch, the two arguments in global memory
 // (L2), a bounded grid barrier per stage.  Bound: the latency of a stage (L2 gather, row sum, barrier),
-// about 1.5 us; one launch per stage before this took 8 us.
+// 3.3 us at N = 100; one launch per stage before this took 8.2 us.
 constexpr int kGridThreads = 256;
 
 __global__ void __launch_bounds__(kGridThreads, 1) rk4_grid(const FbResParams P)

@@ -673,7 +673,7 @@ __device__ __forceinline__ void load_slab(const double2 *mat, double2 *Us, int s
 // together ahead of the MMAs.  With only two to four warps on a scheduler it is the instructions
 // between the MMAs that cost: a test of the row block around each MMA, a slab of two k pairs with its
 // barrier or mbarrier, a counter of warps per stage.  (A lone 8-column sub-tile of d = 201 took 56k
-// cycles with those, against 21k of tensor pipe.)
+// cycles with those, now 36k, against 21k of tensor pipe.)
 template <int N, int WPC, int NT>
 __device__ __forceinline__ void tile_rows(const double2 *mat, double2 *Bt, double2 *Us, int d, int kp, int KS, int MD,
                                           int S16, int cb, int sub, int lane)
@@ -989,7 +989,7 @@ __device__ void append_lanes(const Params &P, bool has, int g2, unsigned en, int
 // that column only.
 //
 // What bounds it: the FP64 tensor pipe (8 d^2 flop per column).  Two CTAs of 256 threads per SM
-// while both fit the shared memory (16-column sub-tiles, d <= ~240), so one CTA's scan, gather and
+// while both fit the shared memory (16-column sub-tiles, d <= 232), so one CTA's scan, gather and
 // epilogue overlap the other's products; one CTA of 512 threads (32, 16 or 8 columns) above that.
 // R4, R2, R1: row blocks per warp of the sub-tiles whose column blocks are shared by 4 warps, by
 // 8 and by 16 (512 threads) or 2 (256 threads, 32-column sub-tiles; 0: none wider than 16).
@@ -1399,7 +1399,8 @@ __global__ void normalize_kernel(const Params P, double2 *hat)
 
 constexpr int kRhoBlocks = 5;       // most 8 x 8 blocks of rho per CTA
 constexpr int kRhoT = 32;           // trajectories per stage
-constexpr int kRhoStages = 3;
+constexpr int kRhoLoaders = 128;   // threads that load
+constexpr int kRhoStages = 5;
 constexpr int kRhoStride = 12;      // components between trajectories of a staged block of 8 (192 bytes: the
                                     // two trajectories of an MMA fall on different banks)
 
@@ -1410,15 +1411,19 @@ size_t rho_smem_bytes(int per) { return (size_t)kRhoStages * (per + 2) * kRhoT *
 // trajectories against B = [yr; yi], which is the canonical chain re += xr yr; re += xi yi;
 // im += xi yr; im -= xr yi with trajectories ascending, bit for bit.  The chain over n cannot be
 // split, so the work is spread over chains: a CTA takes `per` consecutive blocks (row-major), at
-// d = 201 676 blocks in 136 CTAs, 10 warps on each of 136 SMs at most 3 to a scheduler.
-// Bound: 3 chains x n / 2 MMAs of 16 cycles = 123 us at d = 201, n = 10^4 (the pipe's floor at a
-// perfect balance is 95 us); two fma chains per thread on 16 x 16 tiles before took 0.85 ms.
-__global__ void __launch_bounds__(64 * kRhoBlocks) rho_kernel(const Params P, const double2 *hat, double2 *rho, int per)
+// d = 201 676 blocks in 136 CTAs, 10 warps on each of 136 SMs at most 3 to a scheduler.  Four more
+// warps load: with the MMA warps loading too, all of them put their copies before the MMAs of a
+// stage at the same time (275 us with three stages; loaders 255 us, and 246 us with five stages).
+// Bound: the MMA pipe would need 3 chains x n / 2 MMAs of 16 cycles = 123 us at d = 201, n = 10^4;
+// an MMA's two operand loads and the copies take about as many cycles of shared memory.  246 us; two
+// fma chains per thread on 16 x 16 tiles before: the purity took 1.01 ms in all, now 0.445 ms.
+__global__ void __launch_bounds__(64 * kRhoBlocks + kRhoLoaders) rho_kernel(const Params P, const double2 *hat, double2 *rho, int per)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int RB = (P.d + 7) / 8, b0 = blockIdx.x * per, nb = min(per, RB * RB - b0);
-    const int part = warp & 1, mine = min(warp >> 1, nb - 1);  // (warps past the last block only load)
+    const int part = warp & 1, mine = warp >> 1;
+    const bool loads = tid >= 64 * per, mma = mine < nb && !loads;
     const int g = lane >> 2, t = lane & 3, th = t >> 1, todd = t & 1;
     const int nst = (P.n + kRhoT - 1) / kRhoT;
     // staged sets of 8 components per trajectory: 0 and 1 the row blocks of the run (two at most:
@@ -1428,10 +1433,10 @@ __global__ void __launch_bounds__(64 * kRhoBlocks) rho_kernel(const Params P, co
     auto at = [&](int it, int set) {
         return reinterpret_cast<double2 *>(smem) + (size_t)((it % kRhoStages) * (per + 2) + set) * kRhoT * kRhoStride;
     };
-    // a stage is sets x kRhoT x 8 components; this thread copies component tid % 8 of trajectories
-    // tid / 8 + 8 per i of every set (the addresses are worked out once: doing it in each stage took
+    // a stage is sets x kRhoT x 8 components; a loading thread copies component tid % 8 of every
+    // 16th trajectory of every set (the addresses are worked out once: doing it in each stage took
     // most of the kernel's time)
-    const int k = tid & 7, t0 = tid >> 3, tstep = blockDim.x >> 3;
+    const int k = tid & 7, t0 = (tid - 64 * per) >> 3;
     int comp[kRhoBlocks + 2];
 #pragma unroll
     for (int set = 0; set < kRhoBlocks + 2; set++) {
@@ -1441,7 +1446,7 @@ __global__ void __launch_bounds__(64 * kRhoBlocks) rho_kernel(const Params P, co
     auto load = [&](int it) {
         if (it < nst) {
             double2 *dst = at(it, 0) + k;
-            for (int tt = t0; tt < kRhoT; tt += tstep) {
+            for (int tt = t0; tt < kRhoT; tt += kRhoLoaders / 8) {
                 const int tr = it * kRhoT + tt;
                 const double2 *src = hat + (size_t)min(tr, P.n - 1) * P.MD;
 #pragma unroll
@@ -1454,11 +1459,12 @@ __global__ void __launch_bounds__(64 * kRhoBlocks) rho_kernel(const Params P, co
     };
     const int blk = b0 + mine, aset = blk / RB - ib0, bset = 2 + mine;
     double c0 = 0.0, c1 = 0.0;
-    for (int i = 0; i < kRhoStages - 1; i++) load(i);
+    for (int i = 0; loads && i < kRhoStages - 1; i++) load(i);
     for (int it = 0; it < nst; it++) {
-        cp_wait<kRhoStages - 2>();
-        __syncthreads();  // stage `it` has landed for every thread, and nobody reads the one refilled next
-        load(it + kRhoStages - 1);
+        if (loads) cp_wait<kRhoStages - 2>();
+        __syncthreads();  // stage `it` has landed, and nobody reads the one refilled next
+        if (loads) load(it + kRhoStages - 1);
+        if (!mma) continue;
         const double *a = reinterpret_cast<const double *>(at(it, aset) + th * kRhoStride + g) + (part ? 1 - todd : todd);
         const double *b = reinterpret_cast<const double *>(at(it, bset) + th * kRhoStride + g) + todd;
 #pragma unroll
@@ -1467,7 +1473,7 @@ __global__ void __launch_bounds__(64 * kRhoBlocks) rho_kernel(const Params P, co
             dmma(c0, c1, (part && todd) ? neg(x) : x, b[2 * k * kRhoStride]);
         }
     }
-    if ((warp >> 1) >= nb) return;
+    if (!mma) return;
     const int i = 8 * (blk / RB) + g, j = 8 * (blk % RB) + 2 * t;
     double *out = reinterpret_cast<double *>(rho) + part;
     if (i < P.d && j < P.d) out[2 * ((size_t)i * P.d + j)] = __ddiv_rn(c0, (double)P.n);
@@ -1800,7 +1806,7 @@ cudaError_t launch_purity(const Params &P, double2 *hat, double2 *rho, double *o
     static std::atomic<unsigned long long> done{0};
     const cudaError_t e = allow_smem(rho_kernel, done);
     if (e != cudaSuccess) return e;
-    rho_kernel<<<(blocks + per - 1) / per, 64 * per, rho_smem_bytes(per), st>>>(P, hat, rho, per);
+    rho_kernel<<<(blocks + per - 1) / per, 64 * per + kRhoLoaders, rho_smem_bytes(per), st>>>(P, hat, rho, per);
     purity_kernel<<<1, kPurityThreads, 0, st>>>(rho, P.d * P.d, out);
     return cudaGetLastError();
 }
