@@ -700,7 +700,7 @@ def split_form(args, q, new_engine, timed_windows, snap, value, ens_plain, x_pla
         "same_jump_count_fraction_after_window": float(np.mean(per_period["split_jumps"] == per_period["plain_jumps"])),
         "horizon": hor,
         "recheck_curve": {"periods": HC, "window_start": "the timed window's checkpoint", "points": curve},
-        "roofline": {"bound": "tensor", "kernel": "qjx::split_step_kernel",
+        "roofline": {"bound": "tensor", "kernel": "qjx::split_kernel",
                      "achieved": exec_flops / kern_s / 1e12, "peak": bf16_peak, "unit": "TFLOP/s",
                      "frac": exec_flops / kern_s / 1e12 / bf16_peak,
                      "peak_source": "MEASURED_PEAKS.json bf16_tflops (cuBLAS bf16 burst)" if peaks else "fallback 1590",
@@ -779,7 +779,7 @@ def run_ours(args):
 
     def timed_windows(eng, snap, clocks=None):
         """K timed runs of the window, each from the checkpoint `snap`; device time of each run
-        (CUDA events around the micro-step launches), max over ranks."""
+        (CUDA events around the trajectory kernels), max over ranks."""
         st0 = eng.stats()
         barrier()
         if clocks:
@@ -847,7 +847,7 @@ def run_ours(args):
                 "algorithmic_flops_per_launch": flops / max(launches_step, 1),
                 "avg_launch_ms": kern_ms / max(launches_step, 1),
                 "matvecs_per_traj_period": matvecs / (n * P * args.steps)}
-    traffic_file = os.path.join(ROOT, "profiles", "step_kernel_traffic.json")
+    traffic_file = os.path.join(ROOT, "profiles", "flow_kernel_traffic.json")
     if os.path.exists(traffic_file):
         with open(traffic_file) as f:
             tf = json.load(f)

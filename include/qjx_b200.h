@@ -55,7 +55,7 @@ typedef enum {
 
 typedef struct qjx_engine qjx_engine;
 
-/* Tile shapes of the micro-step kernels.  All zero: the engine's rule, or the choice the autotuner
+/* Tile shapes of the trajectory kernels.  All zero: the engine's rule, or the choice the autotuner
  * (qjx_autotune) cached for this dimension and precision.  Tiles never change results: every
  * output keeps its own summation order whatever the tiling. */
 typedef struct {
@@ -93,10 +93,9 @@ typedef struct {
                           cores as bf16 hi/lo planes with FP32 accumulation (products hi*hi + hi*lo +
                           lo*hi), states, norms, thresholds, jump times and renormalisation stay
                           FP64.  Needs d <= 256.  QJX has no such mode
-                          (its zgemv is FP64).  A split engine runs a batch of micro-steps as one
-                          cooperative launch (one CTA per SM); when another context holds SMs it
-                          runs them one launch each, with the same results ($QJX_SPLIT_COOP=0
-                          selects that from the start). */
+                          (its zgemv is FP64).  $QJX_SPLIT_COOP=0 runs a split
+                          engine in lock-step micro-steps, one launch each, instead of from its
+                          queues, with the same results. */
     const double *branch_len; /* [num_branches] durations of the branches of a period (NULL: T / 2
                           each, the dimer's half periods); systems with unequal parts (the JCS kick
                           and free evolution, init_split_structure_jcs, core.cpp:10086-10124) give
@@ -104,20 +103,20 @@ typedef struct {
                           or 2 deep_num_steps. */
     double split_recheck; /* split form (precision 1): a norm test whose split-precision norm p lies
                           within split_recheck * p of the threshold is not decided; that step's
-                          matvec is computed again in FP64 (the plain form's arithmetic) in the next
-                          micro-step and decides.  0 selects 1e-5 (about 5x the measured split error
+                          matvec is computed again in FP64 (the plain form's arithmetic) and that
+                          decides.  0 selects 1e-5 (about 5x the measured split error
                           of the norm), a negative value turns the recheck off. */
     qjx_tiles tiles;   /* tile shapes (all 0: rule or autotuner cache) */
 } qjx_config;
 
 typedef struct {
-    int64_t micro_steps;     /* split form: lock-step micro-steps; plain form: sub-tiles (one matrix on 1 to 32
-                                trajectories) */
+    int64_t micro_steps;     /* split form: matvecs and rechecks of the longest trajectory (the micro-steps of
+                                lock-step); plain form: sub-tiles (one matrix on 1 to 32 trajectories) */
     int64_t matvecs;         /* complex d x d matvecs executed (trajectory-steps) */
     int64_t jumps;           /* jumps recorded */
     double kernel_ms;        /* device time of run/observe calls, first to last launch (CUDA events) */
     double last_call_ms;     /* device time of the last run/observe call */
-    double step_kernel_ms;   /* device time of the micro-step kernel batches alone (CUDA events) */
+    double step_kernel_ms;   /* device time of the trajectory kernel's launches alone (CUDA events) */
     int64_t launches;        /* kernels launched by the engine */
     int64_t mma_tiles;       /* split form: 128-row tcgen05 tiles (12 MMAs of 128 x MDs x 16 per k-step) */
     int64_t rechecks;        /* split form: norm tests taken again on an FP64 matvec */
@@ -151,8 +150,8 @@ typedef struct {
     const double *U, *L, *g, *HE, *R;
 } qjx_ensemble;
 /* Batched engine: n_ens ensembles of uneven Hilbert dimension (d <= 1024) advanced together by
- * the same persistent micro-step launches (every (ensemble, matrix) pair is a bucket of the
- * grouped GEMM; a sub-tile multiplies only its ensemble's d x d block).  cfg supplies what the
+ * the same persistent kernel (every (ensemble, matrix) pair has a queue of trajectories; a
+ * sub-tile multiplies only its ensemble's d x d block).  cfg supplies what the
  * ensembles share: deep, num_branches, num_diss, num_robs, record, rng_kind, rec_cap, keep_adr,
  * max_dumps, device, deep_num_steps, precision (1 needs every ensemble's d <= 256; each then has
  * its own bf16 planes, k-steps and padded rows); cfg's d, n_traj, T, seed and tr_base are
@@ -296,7 +295,7 @@ qjx_status qjx_lpn_get_last(qjx_engine *h, int *renormed, double *ratio, double 
 qjx_status qjx_checkpoint_size(qjx_engine *h, size_t *bytes);
 qjx_status qjx_checkpoint_save(qjx_engine *h, void *buf, size_t bytes);
 qjx_status qjx_checkpoint_load(qjx_engine *h, const void *buf, size_t bytes);
-/* Per-CTA trace of the micro-step kernel (profiling aid, off by default): enabling clears
+/* Per-CTA trace of the trajectory kernel (profiling aid, off by default): enabling clears
  * and starts accumulating, per persistent CTA, clock64 cycles {total, setup, (reserved),
  * MMA loop, epilogue} and counts {sub-tiles, 8-column blocks, columns}.  qjx_get_trace
  * copies [n_ctas][n_fields] int64 (out may be NULL to query the shape). */
@@ -420,9 +419,10 @@ qjx_status qjx_fb_create(int n, const int *gs_rowptr, const int *gs_col, const d
                          double T, int num_steps, int device, qjx_fb **out);
 /* Integrate n_periods periods of num_steps RK4 steps starting at period index period0.
  * When the system fits, one thread-block cluster (<= 16 CTAs) holds it in distributed shared
- * memory and runs a period per launch; otherwise one launch per RK stage. */
+ * memory and runs a period per launch; a larger one runs a period as one cooperative launch over all
+ * SMs, or as one launch per RK stage where its CTAs cannot all be resident. */
 qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods);
-/* Cluster size of the cluster-resident path (0: per-stage kernels). */
+/* Cluster size of the cluster-resident path (0: grid-wide or per-stage kernels). */
 qjx_status qjx_fb_info(qjx_fb *h, int *cluster_size);
 qjx_status qjx_fb_get(qjx_fb *h, double *x, double *last_period_ms);
 void qjx_fb_destroy(qjx_fb *h);

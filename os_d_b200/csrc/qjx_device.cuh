@@ -13,7 +13,7 @@
 
 namespace qjx {
 
-// ---- launch geometry of the micro-step kernel ----
+// ---- launch geometry of the trajectory kernels ----
 constexpr int kThreads = 512;          // 16 warps (split-form kernel)
 constexpr int kKB = 16;                // most k rows per propagator slab
 constexpr int kMaxDt = 64;             // split-level steps [nb][deep] a CTA keeps in shared memory
@@ -150,10 +150,10 @@ struct Params {
     double *r_time, *r_norm, *r_eta;
     int *r_type;
     // control: [0] error count, [1] first error trajectory, [2] paused count, [3] first error code,
-    //          [4] timeouts, [kLive] trajectories left (plain form)
+    //          [4] timeouts, [kLive] trajectories left (queues)
     int *ctrl;
     long long *work;         // trajectory-matvecs; split form: tiles, rechecks; [3] plain form: sub-tiles
-    // optional per-CTA trace, accumulated over micro-steps: [grid][kTraceFields] clock64 cycles
+    // optional per-CTA trace, accumulated over launches: [grid][kTraceFields] clock64 cycles
     // and counts (null: tracing off)
     long long *trace;
     // split-precision form: bf16 hi/lo planes of Re M and Im M of every matrix in tcgen05
@@ -166,12 +166,12 @@ struct Params {
     // in usplit
     const int *e_mds, *e_ks;
     const long long *g_uoff;
-    // tile plan of the next micro-step: [0] rows per tile, [1 + g] first tile of group g,
+    // tile plan of the next lock-step micro-step: [0] rows per tile, [1 + g] first tile of group g,
     // [1 + G] tiles in all; written by the last CTA of a micro-step (or split_plan_kernel)
     int *splan;
-    int grid;                     // CTAs of the micro-step kernels
+    int grid;                     // CTAs of the split kernel (SMs)
     // near-threshold FP64 rechecks of the split form: band (relative to the norm; 0: off), the
-    // recheck lists of the micro-steps ([3] counts, [2][n] trajectories) and the k rows of the
+    // recheck lists of lock-step ([3] counts, [2][n] trajectories) and the k rows of the
     // FP64 matrix slabs streamed through the operand ring
     double recheck_tol;
     int *rcnt;

@@ -1,5 +1,5 @@
 // qjx_engine.cu -- host side of the QJ trajectory engine: device memory, the loops over time slices
-// (plain form) and micro-step batches (split form), jump-record draining, and the C ABI declared in
+// of the trajectory kernels, jump-record draining, and the C ABI declared in
 // include/qjx_b200.h.
 #include <algorithm>
 #include <cmath>

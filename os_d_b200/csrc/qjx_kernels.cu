@@ -1413,7 +1413,8 @@ size_t rho_smem_bytes(int per) { return (size_t)kRhoStages * (per + 2) * kRhoT *
 // split, so the work is spread over chains: a CTA takes `per` consecutive blocks (row-major), at
 // d = 201 676 blocks in 136 CTAs, 10 warps on each of 136 SMs at most 3 to a scheduler.  Four more
 // warps load: with the MMA warps loading too, all of them put their copies before the MMAs of a
-// stage at the same time (275 us with three stages; loaders 255 us, and 246 us with five stages).
+// stage at the same time (ncu: 283 us, with the loaders 262; in a running program 255 us, and 246
+// with five stages instead of three).
 // Bound: the MMA pipe would need 3 chains x n / 2 MMAs of 16 cycles = 123 us at d = 201, n = 10^4;
 // an MMA's two operand loads and the copies take about as many cycles of shared memory.  246 us; two
 // fma chains per thread on 16 x 16 tiles before: the purity took 1.01 ms in all, now 0.445 ms.

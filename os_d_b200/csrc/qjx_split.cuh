@@ -1,4 +1,4 @@
-// qjx_split.cuh -- the split-precision micro-step on the tcgen05 tensor cores (precision 1).
+// qjx_split.cuh -- the split-precision form on the tcgen05 tensor cores (precision 1).
 //
 // Same queues, independent CTAs and trajectory state machine as the FP64 plain form; only the d x d
 // complex matvec changes.  Roles are transposed against the FP64 kernel so that
@@ -19,7 +19,7 @@
 // d = 201).  The accumulators are read back to FP64 and the FP64 epilogue of the plain form
 // runs unchanged (norm test, jump, renormalisation, observables), except that a norm within the
 // split error of the threshold is not decided: that trajectory's step is computed again as an
-// FP64 matvec (the plain form's arithmetic) by a CTA the split tiles leave free, which decides.
+// FP64 matvec (the plain form's arithmetic) by the next CTA that looks for work, which decides.
 //
 // Shared-memory operands use the K-major no-swizzle canonical layout: a core matrix is
 // 8 rows x 16 bytes (8 bf16 along K) stored contiguously; within one k-step (16 bf16 of K)
@@ -27,7 +27,7 @@
 // 8-row groups 256 bytes apart (stride byte offset).  The host writes B in exactly this
 // order, so one k-step of all four B planes is one contiguous TMA bulk copy.
 //
-// Per tile (one matrix, up to 128 trajectories of one bucket) a ring of S stages, one k-step of
+// Per tile (one matrix, up to 128 trajectories of one queue) a ring of S stages, one k-step of
 // A and B planes each:
 //   warps 0-3, 6-9, 10-13   three producer groups; group p converts the k-steps ks = p (mod 3):
 //               FP64 state -> bf16 planes of A (a warp-wide 256-bit load covers 8 rows x 128 bytes;
@@ -43,7 +43,7 @@
 // operand ring, mbarriers and tensor memory from tile to tile for a time slice.
 // (One cooperative launch of lock-step micro-steps with a grid barrier and a plan between them before
 // this: at d = 201 with 10^4 trajectories a CTA was busy 46 % of the time, the rest went on waiting
-// for the slowest tile and on the plan; 232 ms of kernel time for a period, now 197.  A tile, of 50
+// for the slowest tile and on the plan; 232 ms of kernel time for two periods, now 197.  A tile, of 50
 // rows on average, now takes 15 k cycles to claim, the wait for work at the end of the period
 // included, 24 k of MMAs whatever its rows, and 23 k of epilogue.)
 // With QJX_SPLIT_COOP=0 the same tiles run as lock-step micro-steps, one launch each, over bucket
