@@ -749,7 +749,7 @@ def run_ours(args):
         os.environ.setdefault("QJX_TILE_CACHE", os.path.join(tempfile.mkdtemp(), "tiles.txt"))
         tuned = {}
         for prec in (0, 1):
-            best, table = q.autotune(M["U"], M["L"], [1.0], M["HE"], T=M["T"], n_traj=2048, precision=prec,
+            best, table = q.autotune(M["U"], M["L"], [1.0], M["HE"], T=M["T"], n_traj=n, precision=prec,
                                      n_periods=1, device=local)
             tuned["split" if prec else "plain"] = {"best": best, "candidates_us_per_traj_period":
                                                    [[t, round(us, 4)] for t, us in table]}

@@ -863,10 +863,12 @@ __device__ __forceinline__ Pick scan(const Params &P, int stop_live, int least, 
         }
         const int m = __reduce_max_sync(0xffffffffu, b);
         if (m > pick.n) {
-            const unsigned who = __ballot_sync(0xffffffffu, b == m);
-            const int r = turn & 31;
-            pick.n = m;
-            pick.g = __shfl_sync(0xffffffffu, bi, (__ffs(__funnelshift_r(who, who, r)) - 1 + r) & 31);
+            // 128 rows: any lane's queue with half as many, so that CTAs spread over short queues, and more
+            // tries (18 ensembles of 1000, d 60 to 240: 174 ms a period; in lock-step 217)
+            const unsigned who = __ballot_sync(0xffffffffu, NCM == 128 ? 2 * b > m : b == m);
+            const int r = turn & 31, from = (__ffs(__funnelshift_r(who, who, r)) - 1 + r) & 31;
+            pick.n = __shfl_sync(0xffffffffu, b, from);
+            pick.g = __shfl_sync(0xffffffffu, bi, from);
         }
     }
     if (live <= stop_live) pick.n = -1;
@@ -885,7 +887,7 @@ __device__ __forceinline__ int grant(const Params &P, unsigned long long t_end, 
 {
     // a queue that others have nearly emptied since it was looked at is passed over this many times:
     // a sub-tile of a few columns costs as much tensor time as a full block of eight
-    constexpr int kTries = 2;
+    constexpr int kTries = NCM == 128 ? 8 : 2;
     unsigned long long t_idle = 0;
     int n = 0, tries = 0;
     while (true) {
