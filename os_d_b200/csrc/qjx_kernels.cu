@@ -1195,6 +1195,7 @@ __global__ void __launch_bounds__(kSoloThreads, kPre > 4 ? 1 : 2) solo_kernel(co
     unsigned turn = blockIdx.x;
     __shared__ Tally tally;
     if (tid == 0) tally.reset();
+    if (C > 1) cluster_sync();  // every CTA of the cluster has started: its shared memory may be written
     auto sync = [&] {
         if (C > 1) cluster_sync();
         else __syncthreads();
