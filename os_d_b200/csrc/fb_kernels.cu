@@ -296,8 +296,11 @@ __device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity)
 // all n entries have arrived, with no cluster barrier (two round trips) and no wait for stores to be
 // acknowledged.  Two mbarriers and two arguments are enough: a CTA can send entries of stage s + 1
 // only after it has all of stage s, so after every CTA has finished reading the argument of stage s
-// (the one that stage s + 1 overwrites is that of stage s - 1).  One warp works out the next step's
-// drive values meanwhile.  Bound: the latency of a stage (gather, row sum, st.async, mbarrier),
+// (the one that stage s + 1 overwrites is that of stage s - 1).  That holds for warps with rows, whose
+// entries the next stage needs, and for the two that arrive at the mbarrier; the others (about half
+// at N = 50) skip the stages: nothing would keep the cluster from getting two stages ahead of one, whose
+// mbarrier would then show the old parity again.  One warp works out the next step's drive values
+// meanwhile.  Bound: the latency of a stage (gather, row sum, st.async, mbarrier),
 // 1.6 us at N = 50.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread
 // its own sine): 2.9 us.
 __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResParams P, int cs)
@@ -325,9 +328,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
     }
     __syncthreads();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const bool works = warp == 0 || warp == nw - 1 || 32 * warp < r.S || nw - 1 - warp < r.L;
     bool ok = true;
     uint32_t it = 0;  // stages done
-    for (int s = 0; s < P.num_steps; s++) {
+    for (int s = 0; works && s < P.num_steps; s++) {
 #pragma unroll 1
         for (int stage = 1; stage <= 4; stage++, it++) {
             const double *arg = buf + (it & 1) * (size_t)(n + 1);
@@ -367,12 +371,13 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
                 ok = false;
                 atomicExch(P.fail, 1);
             }
+            __syncwarp();  // (no lane starts a stage while another still waits for the one before)
         }
     }
-    for (int i = tid; i < r.S + r.L; i += nt) P.x[P.perm[r.base + i]] = m.x[i];
-    // no CTA leaves while another's stores into it may be on their way
+    // every thread is past its last stage, so all stores into this CTA have arrived
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = tid; i < r.S + r.L; i += nt) P.x[P.perm[r.base + i]] = m.x[i];
 }
 
 // ---- grid form: systems too large for a cluster, on every SM
