@@ -420,7 +420,9 @@ qjx_status qjx_fb_create(int n, const int *gs_rowptr, const int *gs_col, const d
 /* Integrate n_periods periods of num_steps RK4 steps starting at period index period0.
  * When the system fits, one thread-block cluster (<= 16 CTAs) holds it in distributed shared
  * memory and runs a period per launch; a larger one runs a period as one cooperative launch over all
- * SMs, or as one launch per RK stage where its CTAs cannot all be resident. */
+ * SMs, or as one launch per RK stage where its CTAs cannot all be resident.  QJX_ERR_TIMEOUT: a bounded
+ * wait between the CTAs gave up ($QJX_FB_POLLS polls, 2^24 by default); x is what it was before the
+ * call, and the handle can be run again. */
 qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods);
 /* Cluster size of the cluster-resident path (0: grid-wide or per-stage kernels). */
 qjx_status qjx_fb_info(qjx_fb *h, int *cluster_size);

@@ -125,7 +125,7 @@ static cudaError_t queue_rk_stages(const FbParams &P, double T, int num_steps, i
 // lane holds one product, and a level of the tree that pairs a product with an absent lane's +0.0
 // changes nothing but a -0 into +0, which one addition at the end does for all.
 constexpr int kW = 20;
-constexpr long long kFbWait = 1ll << 24;  // polls of a wait before it gives up
+constexpr long long kFbWait = 1ll << 24;  // polls of a wait before it gives up (default of QJX_FB_POLLS)
 
 // Rows of one CTA: S short rows, then L long ones; row i of the CTA is entry base + i of the vectors.
 struct FbRows {
@@ -146,7 +146,8 @@ struct FbResParams {
     double *x;
     double *buf;                             // grid form: two arguments [2][n + 1]
     unsigned *arrived;                       // grid form: CTAs that have passed a stage
-    int *fail;                               // a wait that gave up
+    int *fail;                               // a wait that gave up (the launch's result is not valid then)
+    long long polls;                         // polls of a wait before it gives up
     int maxS, maxL, maxN;                    // strides of the per-CTA arrays
     double drv_ampl, drv_freq, drv_phase;
     int drv_type;
@@ -219,6 +220,14 @@ __device__ __forceinline__ FbSmem fb_carve(const FbResParams &P, unsigned char *
     return m;
 }
 
+// Whether a wait of this run has given up.
+__device__ __forceinline__ bool fb_failed(const FbResParams &P)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(P.fail) : "memory");
+    return v != 0;
+}
+
 // Loads a CTA's rows and the first step's drive (CTA-wide; the caller synchronises).
 __device__ __forceinline__ void fb_load_rows(const FbResParams &P, int cta, const FbRows &r, const FbSmem &m)
 {
@@ -275,9 +284,9 @@ __device__ __forceinline__ uint32_t fb_map(uint32_t addr, int rank)
     return a;
 }
 
-__device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity)
+__device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity, long long polls)
 {
-    for (long long i = 0; i < kFbWait; i++) {
+    for (long long i = 0; i < polls; i++) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -300,7 +309,9 @@ __device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity)
 // entries the next stage needs, and for the two that arrive at the mbarrier; the others (about half
 // at N = 50) skip the stages: nothing would keep the cluster from getting two stages ahead of one, whose
 // mbarrier would then show the old parity again.  One warp works out the next step's drive values
-// meanwhile.  Bound: the latency of a stage (gather, row sum, st.async, mbarrier),
+// meanwhile.  A thread whose wait gives up runs on to the end without waiting, sending or arriving (its
+// mbarriers may not take more than a stage brings), so every other wait ends too.
+// Bound: the latency of a stage (gather, row sum, st.async, mbarrier),
 // 1.6 us at N = 50.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread
 // its own sine): 2.9 us.
 __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResParams P, int cs)
@@ -309,6 +320,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
     __shared__ __align__(8) uint64_t bar[2];
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int n = P.n;
+    if (fb_failed(P)) return;  // (in an earlier period: the same for every CTA)
     int rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     double *buf = reinterpret_cast<double *>(fsm);  // [2][n + 1]
@@ -329,7 +341,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
     __syncthreads();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     const bool works = warp == 0 || warp == nw - 1 || 32 * warp < r.S || nw - 1 - warp < r.L;
-    bool ok = true;
+    int to = cs;      // CTAs that this thread sends to (0: its wait gave up)
     uint32_t it = 0;  // stages done
     for (int s = 0; works && s < P.num_steps; s++) {
 #pragma unroll 1
@@ -339,7 +351,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
             const uint32_t mb = bar0 + 8 * (it & 1);
             const double drv = m.drv[3 * (s & 1) + (stage == 1 ? 0 : (stage == 4 ? 2 : 1))];
             auto send = [&](int i, double v) {
-                for (int c = 0; c < cs; c++)
+                for (int c = 0; c < to; c++)
                     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
                                      fb_map(out + 8 * i, c)),
                                  "l"(__double_as_longlong(v)), "r"(fb_map(mb, c))
@@ -363,20 +375,25 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
             if (warp == nw - 1) {
                 if (stage == 1 && lane < 3) m.drv[3 * ((s + 1) & 1) + lane] = stage_drive(P, s + 1, lane);
                 __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mb) : "memory");
+                if (lane == 0 && to) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mb) : "memory");
             }
-            if (tid == 0)
+            if (tid == 0 && to)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(8 * n) : "memory");
-            if (ok && !fb_wait(mb, (it >> 1) & 1)) {  // (every CTA then runs on without waiting, to the end)
-                ok = false;
+            if (to && !fb_wait(mb, (it >> 1) & 1, P.polls)) {
+                to = 0;
                 atomicExch(P.fail, 1);
             }
             __syncwarp();  // (no lane starts a stage while another still waits for the one before)
         }
     }
-    // every thread is past its last stage, so all stores into this CTA have arrived
+    // every thread is past its last stage, so all stores into this CTA have arrived, unless a wait gave up:
+    // then they get 100 us to
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (fb_failed(P)) {
+        for (int i = 0; i < 100; i++) __nanosleep(1000);
+        return;
+    }
     for (int i = tid; i < r.S + r.L; i += nt) P.x[P.perm[r.base + i]] = m.x[i];
 }
 
@@ -392,6 +409,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) rk4_grid(const FbResParams P)
     __shared__ int s_ok;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int n = P.n, cta = blockIdx.x;
+    if (fb_failed(P)) return;  // (in an earlier period; in this one the other CTAs' waits give up too)
     const FbSmem m = fb_carve(P, fsm);
     int *ec = m.lp + 2 * P.maxL + 2;  // [kW][maxS]
     const FbRows r = P.rows[cta];
@@ -411,7 +429,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) rk4_grid(const FbResParams P)
             unsigned v;
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.arrived) : "memory");
-            } while ((int)(v - want) < 0 && ++i < kFbWait);
+            } while ((int)(v - want) < 0 && ++i < P.polls);
             if ((int)(v - want) < 0) {
                 s_ok = 0;
                 atomicExch(P.fail, 1);
@@ -465,6 +483,7 @@ struct qjx_fb {
     size_t smem = 0;
     fb::FbResParams R{};
     int *h_fail = nullptr;  // pinned
+    double *x0 = nullptr;   // x before the call, for a call in which a wait gives up
     int device = 0;
     double T = 0.0;
     int num_steps = 0;
@@ -602,8 +621,9 @@ static bool fb_upload_deal(qjx_fb *h, const FbSystem &y, const FbDeal &d, bool c
     R.perm = fb_upload(h, d.perm);
     R.x = h->P.x;
     R.fail = (int *)fb_alloc(h, sizeof(int));
+    h->x0 = (double *)fb_alloc(h, sizeof(double) * n);
     if (!R.rows || !R.ev || !(cluster ? (const void *)R.ec16 : R.ec32) || !R.lv || !R.lc || !R.lp || !R.ks || !R.qv || !R.qc ||
-        !R.perm || !R.fail || cudaMemset(R.fail, 0, sizeof(int)) != cudaSuccess ||
+        !R.perm || !R.fail || !h->x0 ||
         (!h->h_fail && cudaMallocHost(&h->h_fail, sizeof(int)) != cudaSuccess))
         return false;
     *h->h_fail = 0;
@@ -768,7 +788,8 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
     if (cudaSetDevice(h->device) != cudaSuccess) return QJX_ERR_CUDA;
     const fb::FbParams &P = h->P;
     cudaEventRecord(h->e0, h->stream);
-    if (h->cs || h->grid) {  // one launch per period
+    const bool resident = h->cs || h->grid;
+    if (resident) {  // one launch per period
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(h->cs ? h->cs : h->grid);
         lc.blockDim = dim3(h->cs ? fb::kClusterThreads : fb::kGridThreads);
@@ -786,8 +807,13 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
         }
         lc.attrs = at;
         lc.numAttrs = 1;
+        const size_t xbytes = sizeof(double) * P.n;
+        cudaMemsetAsync(h->R.fail, 0, sizeof(int), h->stream);
+        cudaMemcpyAsync(h->x0, P.x, xbytes, cudaMemcpyDeviceToDevice, h->stream);
+        const char *polls = std::getenv("QJX_FB_POLLS");
         for (int p = period0; p < period0 + n_periods; p++) {
             fb::FbResParams C = h->R;
+            C.polls = polls ? std::atoll(polls) : fb::kFbWait;
             C.period = p;
             if (!h->cs) cudaMemsetAsync(C.arrived, 0, sizeof(unsigned), h->stream);
             const cudaError_t e = h->cs ? cudaLaunchKernelEx(&lc, fb::rk4_cluster, C, h->cs)
@@ -811,7 +837,12 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, h->e0, h->e1);
     h->last_ms = ms;
-    if (h->h_fail && *h->h_fail) return QJX_ERR_TIMEOUT;
+    if (resident && *h->h_fail) {  // the states of before the call; the handle can be run again
+        if (cudaMemcpyAsync(P.x, h->x0, sizeof(double) * P.n, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess ||
+            cudaStreamSynchronize(h->stream) != cudaSuccess)
+            return QJX_ERR_CUDA;
+        return QJX_ERR_TIMEOUT;
+    }
     return QJX_OK;
 }
 
