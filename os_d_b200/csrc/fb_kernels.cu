@@ -640,6 +640,17 @@ static bool fb_upload_deal(qjx_fb *h, const FbSystem &y, const FbDeal &d, bool c
     return true;
 }
 
+// Lets a kernel take all the shared memory that the device gives a CTA.  The limit belongs to the kernel,
+// not to a handle: set to what one handle needs, a smaller handle's creation would take it from a larger.
+template <class Kernel>
+static bool fb_allow_smem(Kernel *kernel, int optin)
+{
+    cudaFuncAttributes a{};
+    return cudaFuncGetAttributes(&a, kernel) == cudaSuccess &&
+           cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes) ==
+               cudaSuccess;
+}
+
 // The cluster form: the smallest cluster (a power of two up to 16) with at most kClusterRows rows a
 // CTA, or 16, when its shared memory holds the system.
 static bool fb_setup_cluster(qjx_fb *h, const FbSystem &y)
@@ -655,7 +666,7 @@ static bool fb_setup_cluster(qjx_fb *h, const FbSystem &y)
         const size_t bytes = sizeof(double) * 2 * ((size_t)y.n + 1) + fb::fb_rows_bytes(d.maxS, d.maxL, d.maxN) +
                              sizeof(unsigned short) * fb::kW * d.maxS + 16;
         if (bytes + 1024 > (size_t)optin) continue;
-        if (cudaFuncSetAttribute(fb::rk4_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        if (!fb_allow_smem(fb::rk4_cluster, optin) ||
             (cs > 8 && cudaFuncSetAttribute(fb::rk4_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
             cudaGetLastError();
             continue;
@@ -696,7 +707,7 @@ static bool fb_setup_grid(qjx_fb *h, const FbSystem &y)
     fb_deal(y, sms, d);
     const size_t bytes = fb::fb_rows_bytes(d.maxS, d.maxL, d.maxN) + sizeof(int) * fb::kW * d.maxS + 16;
     if (bytes + 1024 > (size_t)optin ||
-        cudaFuncSetAttribute(fb::rk4_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        !fb_allow_smem(fb::rk4_grid, optin) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fb::rk4_grid, fb::kGridThreads, bytes) != cudaSuccess || per < 1) {
         cudaGetLastError();
         return false;
