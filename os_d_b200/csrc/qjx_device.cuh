@@ -211,6 +211,10 @@ struct Params {
     unsigned int *plan_sync;          // [1] CTAs finished in the current lock-step micro-step
     int *sdone;                       // [1] split form: lock-step micro-steps run, or the longest chain
     int *chain;                       // [n] split form: matvecs of each trajectory in this run
+    // sections in which the queues are looked over, 256 at most each: the queues of a block of sect_ens
+    // ensembles, or one of sect_parts parts of one ensemble's; and the trajectories left of each block
+    int sections, sect_ens, sect_parts;
+    int *left;                        // [sections / sect_parts]
     int flow;                         // queues (1) or lock-step lists (the split form with QJX_SPLIT_COOP=0)
 };
 

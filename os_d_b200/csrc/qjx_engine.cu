@@ -621,6 +621,10 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
                 add(ens[e].n, g_off[e * Ge + l], P.split ? kMaxTile : e_nc[e], e_kb[e], ens[e].d, e);
         if (P.split) add(n, 0, 1, 0, 0, 0);  // FP64 rechecks
         h->ring_len = (size_t)roff;
+        P.sect_ens = std::max(1, 256 / Ge);
+        P.sect_parts = (Ge + 255) / 256;
+        P.sections = (E + P.sect_ens - 1) / P.sect_ens * P.sect_parts;
+        P.left = (int *)dalloc(h, (size_t)(P.sections / P.sect_parts) * sizeof(int));
         P.q = upload(h, q);
         P.ring = (unsigned int *)dalloc(h, h->ring_len * sizeof(unsigned int));
         P.gd = upload(h, gd);
@@ -642,7 +646,7 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     P.r_type = (int *)dalloc(h, rc * sizeof(int));
     P.ctrl = (int *)dalloc(h, 16 * sizeof(int));
     P.work = (long long *)dalloc(h, 4 * sizeof(long long));
-    if (!P.psi || !P.st || !P.gn || (P.flow ? !P.q || !P.ring || !P.gd : !P.cnt || !P.lists) || !P.o_norm || !P.o_mean || !P.o_disp || !P.o_m2 ||
+    if (!P.psi || !P.st || !P.gn || (P.flow ? !P.q || !P.ring || !P.gd || !P.left : !P.cnt || !P.lists) || !P.o_norm || !P.o_mean || !P.o_disp || !P.o_m2 ||
         !P.o_energy || !P.o_robs || !P.o_adr || !P.mean_start || !P.r_time || !P.r_norm || !P.r_eta || !P.r_type ||
         !P.ctrl || !P.work)
         return bail(QJX_ERR_OOM);
@@ -822,6 +826,7 @@ static cudaError_t clear_queues(qjx_engine *h)
     } else {
         if (e == cudaSuccess) // the counts, not the sub-tile width
             e = cudaMemset2DAsync(P.q, sizeof(Queue), 0, offsetof(Queue, nc), P.G + (P.split ? 1 : 0), h->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(P.left, 0, sizeof(int) * (P.sections / P.sect_parts), h->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(P.ring, 0xff, sizeof(unsigned int) * h->ring_len, h->stream);
     }
     return e;

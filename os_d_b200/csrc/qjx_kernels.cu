@@ -140,6 +140,7 @@ __device__ __forceinline__ void enqueue(const Params &P, int g, int tr)
         P.ring[P.gd[g].roff + (pos & P.gd[g].rmask())] = entry_of(tr, P.st[tr]);
         atomicAdd(&P.q[g].avail, 1);
         atomicAdd(P.ctrl + kLive, 1);
+        atomicAdd(P.left + P.st[tr].ens / P.sect_ens, 1);
     }
 }
 
@@ -825,50 +826,82 @@ struct Pick {
     int n, g;
 };
 
-// Looks the queues over (one warp, converged): a claim is at most NCM trajectories and an equal share
-// of the unfinished ones in whole 8-column blocks, or `least` if that is more (NCM = 1: one
-// trajectory).  Any queue that has the share waiting will do (a different one for each CTA and
-// attempt, so that claims spread), else the fullest.  Queues are scanned 256 at a time from a place
-// that differs by CTA, up to the first 256 with a share waiting.
+// Looks over at most 256 queues, base to end - 1 (one warp, converged).  A claim is at most NCM trajectories
+// and an equal share of the `live` unfinished ones in whole 8-column blocks, or `least` if that is more
+// (NCM = 1: one trajectory).  Any queue that has the share waiting will do (a different one for each CTA
+// and attempt, so that claims spread), else the fullest; MANY: any with `goal` waiting and half of the
+// fullest's.  Leaves `pick` as it is when that has as many.
+template <int NCM, bool MANY>
+__device__ __forceinline__ void look_over(const Params &P, int base, int end, int live, int least, int goal, unsigned turn, int lane,
+                                          Pick &pick)
+{
+    int av[8], cap[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int gi = base + 32 * i + lane;
+        av[i] = cap[i] = 0;
+        if (gi < end) {
+            const int4 v = __ldcg(reinterpret_cast<const int4 *>(P.q) + gi);
+            av[i] = v.x;
+            cap[i] = v.w;
+        }
+    }
+    const int share = min(NCM, max(least, 8 * ((live + 8 * (int)gridDim.x - 1) / (8 * (int)gridDim.x))));
+    int b = 0, bi = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int a = min(av[i], min(share, cap[i]));
+        if (a > b) {
+            b = a;
+            bi = base + 32 * i + lane;
+        }
+    }
+    const int m = __reduce_max_sync(0xffffffffu, b);
+    if (m > pick.n) {
+        // 128 rows: any lane's queue with more than half as many, so that CTAs spread over short queues, and
+        // more tries (18 ensembles of 1000, d 60 to 240: 174 ms a period; in lock-step 217)
+        const unsigned who =
+            __ballot_sync(0xffffffffu, NCM == 128 ? 2 * b > m : (MANY ? b >= max(min(m, goal), (m + 1) / 2) : b == m));
+        const int r = turn & 31, from = (__ffs(__funnelshift_r(who, who, r)) - 1 + r) & 31;
+        pick.n = __shfl_sync(0xffffffffu, b, from);
+        pick.g = __shfl_sync(0xffffffffu, bi, from);
+    }
+}
+
+// The queue to take from: -1 when at most stop_live trajectories are left.  More than 256 queues are looked over
+// by sections (see Params), from one that differs by CTA.  Most queues of many ensembles never hold a
+// share, and CTAs that all look for the fullest take it from each other: the scan ends at the first
+// section with more waiting in one queue than in the mean queue, and sections whose ensembles are done are
+// passed over.  ms a period, looking for a share everywhere / now / in lock-step: 64 ensembles of 200 (d 21 to 121)
+// 216 / 52 / 206, in split precision 168 / 102 / 135; 128 of 30 (d 21 to 201) 434 / 90 / 431; 128 of 100
+// in split precision 383 / 136 / 205; 8 of 200 (d 51 to 401) 159 / 152 / 365.
 template <int NCM>
 __device__ __forceinline__ Pick scan(const Params &P, int stop_live, int least, unsigned &turn, int lane)
 {
-    const int G = P.G, chunks = (G + 255) / 256;
     turn += 7u;
     const int live = __ldcg(P.ctrl + kLive);
-    int share = NCM;
     Pick pick{0, 0};
-    for (int c = 0; c < chunks && pick.n < share; c++) {
-        const int base = 256 * (int)((c + turn) % (unsigned)chunks);
-        int av[8], cap[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int gi = base + 32 * i + lane;
-            av[i] = cap[i] = 0;
-            if (gi < G) {
-                const int4 v = __ldcg(reinterpret_cast<const int4 *>(P.q) + gi);
-                av[i] = v.x;
-                cap[i] = v.w;
+    if (P.sections == 1) {
+        look_over<NCM, false>(P, 0, P.G, live, least, 0, turn, lane, pick);
+    } else {
+        const int sections = P.sections, per = P.sect_ens * P.Ge, goal = min(NCM, live / P.G + 1);
+        int at = (int)(turn % (unsigned)sections);
+        for (int c = 0; c < sections && pick.n < goal;) {
+            if (P.sect_parts == 1) {  // the next section with trajectories left
+                const int s = at + lane;
+                const unsigned left =
+                    __ballot_sync(0xffffffffu, lane < sections - c && __ldcg(P.left + (s < sections ? s : s - sections)) > 0);
+                const int skip = left ? __ffs(left) - 1 : 32;
+                c += skip;
+                at += skip;
+                if (at >= sections) at -= sections;
+                if (!left) continue;
             }
-        }
-        share = min(NCM, max(least, 8 * ((live + 8 * (int)gridDim.x - 1) / (8 * (int)gridDim.x))));
-        int b = 0, bi = 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int a = min(av[i], min(share, cap[i]));
-            if (a > b) {
-                b = a;
-                bi = base + 32 * i + lane;
-            }
-        }
-        const int m = __reduce_max_sync(0xffffffffu, b);
-        if (m > pick.n) {
-            // 128 rows: any lane's queue with half as many, so that CTAs spread over short queues, and more
-            // tries (18 ensembles of 1000, d 60 to 240: 174 ms a period; in lock-step 217)
-            const unsigned who = __ballot_sync(0xffffffffu, NCM == 128 ? 2 * b > m : b == m);
-            const int r = turn & 31, from = (__ffs(__funnelshift_r(who, who, r)) - 1 + r) & 31;
-            pick.n = __shfl_sync(0xffffffffu, b, from);
-            pick.g = __shfl_sync(0xffffffffu, bi, from);
+            const int block = at / P.sect_parts;
+            look_over<NCM, true>(P, block * per + 256 * (at - block * P.sect_parts), min(P.G, (block + 1) * per), live, least, goal,
+                                 turn, lane, pick);
+            c++;
+            at = at + 1 < sections ? at + 1 : 0;
         }
     }
     if (live <= stop_live) pick.n = -1;
@@ -950,7 +983,7 @@ __device__ __forceinline__ int take(const Params &P, unsigned long long t_end, i
 
 // Appends trajectories to their next queues (one warp, converged): lanes with `has` have the bucket
 // g2 and the entry `en` of one, -1 when it is finished, paused or failed.  Lanes with the same bucket
-// find each other, the lowest reserves the run.
+// find each other, the lowest reserves the run.  All are of one ensemble.
 __device__ void append_lanes(const Params &P, bool has, int g2, unsigned en, int lane)
 {
     __threadfence();  // release: what the CTA wrote, before the entries
@@ -965,6 +998,7 @@ __device__ void append_lanes(const Params &P, bool has, int g2, unsigned en, int
             base = atomicAdd(&P.q[key].tail, (unsigned)__popc(m));
             atomicAdd(&P.q[key].avail, __popc(m));
         } else if (key == -1) {
+            atomicSub(P.left + P.st[en >> 3].ens / P.sect_ens, __popc(m));
             atomicSub(P.ctrl + kLive, __popc(m));
         }
     }
@@ -1314,6 +1348,7 @@ __global__ void __launch_bounds__(kSoloThreads, kPre > 4 ? 1 : 2) solo_kernel(co
                         report_error(P, -1, ERR_TIMEOUT);
                     }
                 } else {
+                    atomicSub(P.left + e / P.sect_ens, 1);
                     atomicSub(P.ctrl + kLive, 1);
                 }
             }
