@@ -23,6 +23,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -482,7 +483,6 @@ struct qjx_fb {
     int cs = 0, grid = 0;
     size_t smem = 0;
     fb::FbResParams R{};
-    int *h_fail = nullptr;  // pinned
     double *x0 = nullptr;   // x before the call, for a call in which a wait gives up
     int device = 0;
     double T = 0.0;
@@ -511,14 +511,6 @@ struct FbSystem {
     const double *ks;
 };
 
-template <class V>
-static V *fb_upload(qjx_fb *h, const std::vector<V> &v)
-{
-    V *p = (V *)fb_alloc(h, v.size() * sizeof(V));
-    if (p && !v.empty() && cudaMemcpy(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
-    return p;
-}
-
 // The rows dealt to `nc` CTAs and their shared-memory form: the rows of each nonzero count, in their
 // natural order (neighbours read neighbouring columns), cut into nc equal runs, so every CTA gets the
 // same mix.  Entries of the vectors are numbered CTA after CTA, short rows first.
@@ -531,23 +523,27 @@ struct FbDeal {
 static void fb_deal(const FbSystem &y, int nc, FbDeal &d)
 {
     const int n = y.n;
-    std::vector<int> order(n);
-    for (int i = 0; i < n; i++) order[i] = i;
     // a row's nonzeros; past kW (long) also when its drive has several
-    auto nnz = [&](int i) {
+    std::vector<int> nnz(n), order(n), first;
+    int most = 0;
+    for (int i = 0; i < n; i++) {
         const int g = y.gr[i + 1] - y.gr[i], q = y.qr[i + 1] - y.qr[i];
-        return q > 1 ? fb::kW + 1 + g + q : g;
-    };
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return nnz(a) < nnz(b); });
+        nnz[i] = q > 1 ? fb::kW + 1 + g + q : g;
+        most = std::max(most, nnz[i]);
+    }
+    first.assign(most + 2, 0);
+    for (int i = 0; i < n; i++) first[nnz[i] + 1]++;
+    for (int k = 0; k <= most; k++) first[k + 1] += first[k];
+    const std::vector<int> runs = first;  // rows of k nonzeros: order[runs[k]] .. order[runs[k + 1] - 1]
+    for (int i = 0; i < n; i++) order[first[nnz[i]]++] = i;
     std::vector<std::vector<int>> mine(nc);
+    for (auto &m : mine) m.reserve(n / nc + 64);
     int turn = 0;  // where the remainders of a count go next
-    for (int i = 0; i < n;) {
-        int j = i;
-        while (j < n && nnz(order[j]) == nnz(order[i])) j++;
+    for (int k = 0; k <= most; k++) {
+        const int i = runs[k], j = runs[k + 1];
         const int per = (j - i) / nc;
         for (int c = 0; c < nc; c++) mine[c].insert(mine[c].end(), order.begin() + i + c * per, order.begin() + i + (c + 1) * per);
-        for (int k = i + nc * per; k < j; k++, turn++) mine[turn % nc].push_back(order[k]);
-        i = j;
+        for (int l = i + nc * per; l < j; l++, turn++) mine[turn % nc].push_back(order[l]);
     }
     d = FbDeal();
     d.perm.reserve(n);
@@ -555,7 +551,7 @@ static void fb_deal(const FbSystem &y, int nc, FbDeal &d)
     for (int c = 0; c < nc; c++) {
         fb::FbRows r{(int)d.perm.size(), 0, 0, 0};
         for (int i : mine[c]) {  // ascending counts: the long rows are last
-            if (nnz(i) <= fb::kW) {
+            if (nnz[i] <= fb::kW) {
                 r.S++;
             } else {
                 r.L++;
@@ -572,61 +568,111 @@ static void fb_deal(const FbSystem &y, int nc, FbDeal &d)
     d.maxS = std::max(32, (d.maxS + 31) & ~31);
 }
 
+// One device allocation for several arrays: room() for each, then alloc(), then at().
+struct FbArena {
+    size_t bytes = 0;
+    unsigned char *dev = nullptr;
+    template <class V>
+    size_t room(size_t n)
+    {
+        const size_t at = bytes;
+        bytes += (n * sizeof(V) + 15) & ~(size_t)15;
+        return at;
+    }
+    bool alloc(qjx_fb *h) { return (dev = (unsigned char *)fb_alloc(h, bytes)) != nullptr; }
+    template <class V>
+    V *at(size_t off) const
+    {
+        return (V *)(dev + off);
+    }
+    template <class V>
+    V *put(size_t off, const V *v, size_t n) const
+    {
+        if (n) cudaMemcpy(dev + off, v, n * sizeof(V), cudaMemcpyHostToDevice);
+        return at<V>(off);
+    }
+};
+
 static bool fb_upload_deal(qjx_fb *h, const FbSystem &y, const FbDeal &d, bool cluster)
 {
     const int n = y.n, nc = (int)d.rows.size();
-    std::vector<double> ev((size_t)nc * fb::kW * d.maxS, 0.0), lv((size_t)nc * std::max(1, d.maxN), 0.0), ks(n), qv(n, 0.0);
-    std::vector<int> ec(ev.size(), n), lc(lv.size(), 0), lp((size_t)nc * (2 * d.maxL + 1), 0), qc(n, n);
+    const size_t nev = (size_t)nc * fb::kW * d.maxS, nlv = (size_t)nc * d.maxN, nlp = (size_t)nc * (2 * d.maxL + 1);
+    FbArena a;
+    const size_t orows = a.room<fb::FbRows>(nc), oev = a.room<double>(nev), olv = a.room<double>(nlv), oks = a.room<double>(n);
+    const size_t oqv = a.room<double>(n), olc = a.room<int>(nlv), olp = a.room<int>(nlp), oqc = a.room<int>(n);
+    const size_t operm = a.room<int>(n), oec = cluster ? a.room<unsigned short>(nev) : a.room<int>(nev);
+    const size_t filled = a.bytes;
+    const size_t ofail = a.room<int>(1), ox0 = a.room<double>(n), oarrived = a.room<unsigned>(1);
+    const size_t obuf = a.room<double>(cluster ? 0 : 2 * ((size_t)n + 1));
+    std::unique_ptr<unsigned char[]> host(new (std::nothrow) unsigned char[filled]);
+    if (!host || !a.alloc(h)) return false;
+    unsigned char *const at0 = host.get();
+    double *const ev = (double *)(at0 + oev), *const lv = (double *)(at0 + olv), *const ks = (double *)(at0 + oks);
+    double *const qv = (double *)(at0 + oqv);
+    int *const lc = (int *)(at0 + olc), *const lp = (int *)(at0 + olp), *const qc = (int *)(at0 + oqc);
+    std::memcpy(at0 + orows, d.rows.data(), nc * sizeof(fb::FbRows));
+    std::memcpy(at0 + operm, d.perm.data(), n * sizeof(int));
+    std::fill(ev, ev + nev, 0.0);
+    std::fill(lv, lv + nlv, 0.0);
+    std::fill(qv, qv + n, 0.0);
+    std::fill(lc, lc + nlv, n);
+    std::fill(lp, lp + nlp, 0);
+    std::fill(qc, qc + n, n);
+    if (cluster) std::fill((unsigned short *)(at0 + oec), (unsigned short *)(at0 + oec) + nev, (unsigned short)n);
+    else std::fill((int *)(at0 + oec), (int *)(at0 + oec) + nev, n);
     for (int c = 0; c < nc; c++) {
         const fb::FbRows &r = d.rows[c];
-        int at = 0;
-        for (int i = 0; i < r.S + r.L; i++) {
+        int *const start = lp + (size_t)c * (2 * d.maxL + 1);
+        double *const v = lv + (size_t)c * d.maxN;
+        int *const col = lc + (size_t)c * d.maxN;
+        for (int i = 0; i < r.S + r.L; i++) ks[r.base + i] = y.ks[d.perm[r.base + i]];
+        for (int i = 0; i < r.S; i++) {
             const int row = d.perm[r.base + i], b = y.gr[row], len = y.gr[row + 1] - b;
-            ks[r.base + i] = y.ks[row];
-            if (i < r.S) {
-                for (int l = 0; l < len; l++) {
-                    const size_t e = ((size_t)c * fb::kW + l) * d.maxS + i;
-                    ev[e] = y.gv[b + l];
-                    ec[e] = d.pos[y.gc[b + l]];
-                }
-                if (y.qr[row + 1] > y.qr[row]) {
-                    qv[r.base + i] = y.qv[y.qr[row]];
-                    qc[r.base + i] = d.pos[y.qc[y.qr[row]]];
-                }
-            } else {
-                auto put = [&](double v, int col) {
-                    lv[(size_t)c * d.maxN + at] = v;
-                    lc[(size_t)c * d.maxN + at++] = d.pos[col];
-                };
-                int *start = lp.data() + (size_t)c * (2 * d.maxL + 1) + 2 * (i - r.S);
-                for (int l = 0; l < len; l++) put(y.gv[b + l], y.gc[b + l]);
-                start[1] = at;
-                for (int l = y.qr[row]; l < y.qr[row + 1]; l++) put(y.qv[l], y.qc[l]);
-                start[2] = at;
+            for (int l = 0; l < len; l++) {
+                const size_t e = ((size_t)c * fb::kW + l) * d.maxS + i;
+                ev[e] = y.gv[b + l];
+                if (cluster) ((unsigned short *)(at0 + oec))[e] = (unsigned short)d.pos[y.gc[b + l]];
+                else ((int *)(at0 + oec))[e] = d.pos[y.gc[b + l]];
+            }
+            if (y.qr[row + 1] > y.qr[row]) {
+                qv[r.base + i] = y.qv[y.qr[row]];
+                qc[r.base + i] = d.pos[y.qc[y.qr[row]]];
             }
         }
+        // the nonzeros of long row i from `at` on
+        auto put = [&](int i, const int *rp, const int *ci, const double *val, int at) {
+            const int row = d.perm[r.base + r.S + i];
+            for (int l = rp[row]; l < rp[row + 1]; l++, at++) {
+                v[at] = val[l];
+                col[at] = d.pos[ci[l]];
+            }
+            return at;
+        };
+        int at = 0;
+        for (int j = 0; j < r.L; j++) {
+            start[2 * j + 1] = put(j, y.gr, y.gc, y.gv, at);
+            start[2 * j + 2] = at = put(j, y.qr, y.qc, y.qv, start[2 * j + 1]);
+        }
     }
+    if (cudaMemcpy(a.dev, at0, filled, cudaMemcpyHostToDevice) != cudaSuccess) return false;
     fb::FbResParams &R = h->R;
     R.n = n;
-    R.rows = fb_upload(h, d.rows);
-    R.ev = fb_upload(h, ev);
-    if (cluster) R.ec16 = fb_upload(h, std::vector<unsigned short>(ec.begin(), ec.end()));
-    else R.ec32 = fb_upload(h, ec);
-    R.lv = fb_upload(h, lv);
-    R.lc = fb_upload(h, lc);
-    R.lp = fb_upload(h, lp);
-    R.ks = fb_upload(h, ks);
-    R.qv = fb_upload(h, qv);
-    R.qc = fb_upload(h, qc);
-    R.perm = fb_upload(h, d.perm);
+    R.rows = a.at<fb::FbRows>(orows);
+    R.ev = a.at<double>(oev);
+    if (cluster) R.ec16 = a.at<unsigned short>(oec);
+    else R.ec32 = a.at<int>(oec);
+    R.lv = a.at<double>(olv);
+    R.lc = a.at<int>(olc);
+    R.lp = a.at<int>(olp);
+    R.ks = a.at<double>(oks);
+    R.qv = a.at<double>(oqv);
+    R.qc = a.at<int>(oqc);
+    R.perm = a.at<int>(operm);
     R.x = h->P.x;
-    R.fail = (int *)fb_alloc(h, sizeof(int));
-    h->x0 = (double *)fb_alloc(h, sizeof(double) * n);
-    if (!R.rows || !R.ev || !(cluster ? (const void *)R.ec16 : R.ec32) || !R.lv || !R.lc || !R.lp || !R.ks || !R.qv || !R.qc ||
-        !R.perm || !R.fail || !h->x0 ||
-        (!h->h_fail && cudaMallocHost(&h->h_fail, sizeof(int)) != cudaSuccess))
-        return false;
-    *h->h_fail = 0;
+    R.fail = a.at<int>(ofail);
+    h->x0 = a.at<double>(ox0);
+    R.arrived = a.at<unsigned>(oarrived);
+    R.buf = a.at<double>(obuf);
     R.maxS = d.maxS;
     R.maxL = d.maxL;
     R.maxN = d.maxN;
@@ -713,9 +759,6 @@ static bool fb_setup_grid(qjx_fb *h, const FbSystem &y)
         return false;
     }
     if (!fb_upload_deal(h, y, d, false)) return false;
-    h->R.buf = (double *)fb_alloc(h, sizeof(double) * 2 * ((size_t)y.n + 1));
-    h->R.arrived = (unsigned *)fb_alloc(h, sizeof(unsigned));
-    if (!h->R.buf || !h->R.arrived) return false;
     h->grid = sms;
     h->smem = bytes;
     return true;
@@ -742,51 +785,49 @@ extern "C" qjx_status qjx_fb_create(int n, const int *gs_rowptr, const int *gs_c
     cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     cudaEventCreate(&h->e0);
     cudaEventCreate(&h->e1);
-    const int gnz = gs_rowptr[n], qnz = qs_rowptr[n];
     fb::FbParams &P = h->P;
     P.n = n;
-    int *gr = (int *)fb_alloc(h, sizeof(int) * (n + 1)), *gc = (int *)fb_alloc(h, sizeof(int) * gnz);
-    int *qr = (int *)fb_alloc(h, sizeof(int) * (n + 1)), *qc = (int *)fb_alloc(h, sizeof(int) * qnz);
-    double *gv = (double *)fb_alloc(h, sizeof(double) * gnz), *qv = (double *)fb_alloc(h, sizeof(double) * qnz);
-    double *ks = (double *)fb_alloc(h, sizeof(double) * n);
-    P.x = (double *)fb_alloc(h, sizeof(double) * n);
-    P.va = (double *)fb_alloc(h, sizeof(double) * n);
-    P.vb = (double *)fb_alloc(h, sizeof(double) * n);
-    P.k1 = (double *)fb_alloc(h, sizeof(double) * n);
-    P.k2 = (double *)fb_alloc(h, sizeof(double) * n);
-    P.k3 = (double *)fb_alloc(h, sizeof(double) * n);
-    if (!gr || !gc || !qr || !qc || !gv || !qv || !ks || !P.x || !P.va || !P.vb || !P.k1 || !P.k2 || !P.k3) {
-        qjx_fb_destroy(h);
-        return QJX_ERR_OOM;
-    }
-    cudaMemcpy(gr, gs_rowptr, sizeof(int) * (n + 1), cudaMemcpyHostToDevice);
-    cudaMemcpy(gc, gs_col, sizeof(int) * gnz, cudaMemcpyHostToDevice);
-    cudaMemcpy(gv, gs_val, sizeof(double) * gnz, cudaMemcpyHostToDevice);
-    cudaMemcpy(qr, qs_rowptr, sizeof(int) * (n + 1), cudaMemcpyHostToDevice);
-    cudaMemcpy(qc, qs_col, sizeof(int) * qnz, cudaMemcpyHostToDevice);
-    cudaMemcpy(qv, qs_val, sizeof(double) * qnz, cudaMemcpyHostToDevice);
-    cudaMemcpy(ks, Ks, sizeof(double) * n, cudaMemcpyHostToDevice);
-    cudaMemcpy(P.x, x0, sizeof(double) * n, cudaMemcpyHostToDevice);
-    P.gr = gr;
-    P.gc = gc;
-    P.gv = gv;
-    P.qr = qr;
-    P.qc = qc;
-    P.qv = qv;
-    P.Ks = ks;
     P.drv_ampl = -drv_ampl;
     P.drv_freq = drv_freq;
     P.drv_phase = drv_phase;
     P.drv_type = drv_type;
+    P.x = (double *)fb_alloc(h, sizeof(double) * n);
+    if (!P.x) {
+        qjx_fb_destroy(h);
+        return QJX_ERR_OOM;
+    }
+    cudaMemcpy(P.x, x0, sizeof(double) * n, cudaMemcpyHostToDevice);
+    // resident forms; QJX_FB_PATH=stages forces the per-stage kernels
+    const char *path = std::getenv("QJX_FB_PATH");
+    const bool stages = path && std::string(path) == "stages";
+    const FbSystem sys{n, gs_rowptr, gs_col, gs_val, qs_rowptr, qs_col, qs_val, Ks};
+    if (stages || !fb_setup_cluster(h, sys)) {
+        // the stage kernels' system and vectors (for the grid form: where its CTAs cannot all be resident)
+        const size_t gnz = gs_rowptr[n], qnz = qs_rowptr[n];
+        FbArena a;
+        const size_t gr = a.room<int>(n + 1), gc = a.room<int>(gnz), gv = a.room<double>(gnz), qr = a.room<int>(n + 1);
+        const size_t qc = a.room<int>(qnz), qv = a.room<double>(qnz), ks = a.room<double>(n), v = a.room<double>(5 * (size_t)n);
+        if (!a.alloc(h)) {
+            qjx_fb_destroy(h);
+            return QJX_ERR_OOM;
+        }
+        P.gr = a.put(gr, gs_rowptr, n + 1);
+        P.gc = a.put(gc, gs_col, gnz);
+        P.gv = a.put(gv, gs_val, gnz);
+        P.qr = a.put(qr, qs_rowptr, n + 1);
+        P.qc = a.put(qc, qs_col, qnz);
+        P.qv = a.put(qv, qs_val, qnz);
+        P.Ks = a.put(ks, Ks, n);
+        P.va = a.at<double>(v);
+        P.vb = P.va + n;
+        P.k1 = P.vb + n;
+        P.k2 = P.k1 + n;
+        P.k3 = P.k2 + n;
+        if (!stages) fb_setup_grid(h, sys);
+    }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         qjx_fb_destroy(h);
         return QJX_ERR_CUDA;
-    }
-    // resident forms; QJX_FB_PATH=stages forces the per-stage kernels
-    const char *path = std::getenv("QJX_FB_PATH");
-    if (!(path && std::string(path) == "stages")) {
-        const FbSystem sys{n, gs_rowptr, gs_col, gs_val, qs_rowptr, qs_col, qs_val, Ks};
-        if (!fb_setup_cluster(h, sys)) fb_setup_grid(h, sys);
     }
     cudaGetLastError();
     *out = h;
@@ -839,7 +880,6 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
             }
             if (e != cudaSuccess) return QJX_ERR_CUDA;
         }
-        cudaMemcpyAsync(h->h_fail, h->R.fail, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
     } else if (fb::queue_rk_stages(P, h->T, h->num_steps, period0, n_periods, h->stream) != cudaSuccess) {
         return QJX_ERR_CUDA;
     }
@@ -848,7 +888,9 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, h->e0, h->e1);
     h->last_ms = ms;
-    if (resident && *h->h_fail) {  // the states of before the call; the handle can be run again
+    int failed = 0;
+    if (resident && cudaMemcpy(&failed, h->R.fail, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return QJX_ERR_CUDA;
+    if (failed) {  // the states of before the call; the handle can be run again
         if (cudaMemcpyAsync(P.x, h->x0, sizeof(double) * P.n, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess ||
             cudaStreamSynchronize(h->stream) != cudaSuccess)
             return QJX_ERR_CUDA;
@@ -940,7 +982,6 @@ extern "C" void qjx_fb_destroy(qjx_fb *h)
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void *p : h->allocs) cudaFree(p);
-    if (h->h_fail) cudaFreeHost(h->h_fail);
     if (h->e0) cudaEventDestroy(h->e0);
     if (h->e1) cudaEventDestroy(h->e1);
     if (h->stream) cudaStreamDestroy(h->stream);
