@@ -121,7 +121,8 @@ static cudaError_t queue_rk_stages(const FbParams &P, double T, int num_steps, i
 // Both resident forms keep each CTA's rows in shared memory for a whole launch (a period).  Short rows
 // (at most kW nonzeros and one of the drive, all but about N of the dimer's N^2) are held thread-per-row, nonzero l of
 // consecutive rows side by side (no bank conflicts), padded with a zero value and a column that holds
-// zero; long rows are done by a warp each.  Thread-per-row keeps the canonical order (lane partial
+// zero; long rows are done by a warp each, or (MANY) in slices of 32 rows, a thread each, where a CTA has more
+// of them than warps.  Thread-per-row keeps the canonical order (lane partial
 // sums over nonzeros l, l + 32, ..., then the butterfly tree): with at most kW <= 32 nonzeros each
 // lane holds one product, and a level of the tree that pairs a product with an absent lane's +0.0
 // changes nothing but a -0 into +0, which one addition at the end does for all.
@@ -139,8 +140,8 @@ struct FbResParams {
     const double *ev;                        // short rows: [kW][RS] values per CTA (RS = maxS)
     const unsigned short *ec16;              // and columns (entry numbers; n: the zero)
     const int *ec32;                         // the same for the grid form
-    const double *lv;                        // long rows: nonzeros, each row's of Gs, then of Qs
-    const int *lc, *lp;                      // columns, starts [CTA][2 maxL + 1]: Gs of row j at 2 j, Qs at 2 j + 1
+    const double *lv;                        // long rows: nonzeros, each row's (MANY: each slice's) of Gs, then of Qs
+    const int *lc, *lp;                      // columns, starts [CTA][2 maxL + 1]: Gs of row or slice j at 2 j, Qs at 2 j + 1
     const double *ks, *qv;                   // per entry: constant term; short rows: drive value (0: none)
     const int *qc;                           // and column (n: none)
     const int *perm;                         // entry -> row of the caller's vectors
@@ -178,6 +179,50 @@ __device__ __forceinline__ double long_row(const double *v, const int *c, int b,
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
     return s;
+}
+
+// Row sum of a long row by a thread: its nonzero l at v[32 l], a multiple of four of them (zero values of the zero
+// column past the row's).
+template <class Load>
+__device__ __forceinline__ double slice_row(const double *v, const int *c, int len, const Load &arg)
+{
+    double p[32];
+#pragma unroll
+    for (int l = 0; l < 32; l++) p[l] = 0.0;
+    for (int j = 0; j < len; j += 32) {
+#pragma unroll
+        for (int l = 0; l < 32; l += 4) {
+            if (j + l >= len) break;
+#pragma unroll
+            for (int i = l; i < l + 4; i++) p[i] = __fma_rn(v[32 * (j + i)], arg(c[32 * (j + i)]), p[i]);
+        }
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+        for (int l = 0; l < off; l++) p[l] = __dadd_rn(p[l], p[l + off]);
+    return p[0];
+}
+
+// The long rows of a CTA in a stage: emit(i, t1, t2) gets entry i and its two row sums, from one thread.
+template <bool MANY, class Load, class Emit>
+__device__ __forceinline__ void long_rows(const FbRows &r, const double *lv, const int *lc, const int *lp, int warp, int nw, int lane,
+                                          const Load &arg, const Emit &emit)
+{
+    if (MANY) {
+        for (int j = nw - 1 - warp; 32 * j < r.L; j += nw) {
+            const int g = lp[2 * j], q = lp[2 * j + 1], e = lp[2 * j + 2];
+            const double t1 = slice_row(lv + g + lane, lc + g + lane, (q - g) >> 5, arg);
+            const double t2 = slice_row(lv + q + lane, lc + q + lane, (e - q) >> 5, arg);
+            if (32 * j + lane < r.L) emit(r.S + 32 * j + lane, t1, t2);
+        }
+    } else {
+        for (int j = nw - 1 - warp; j < r.L; j += nw) {
+            const double t1 = long_row(lv, lc, lp[2 * j], lp[2 * j + 1], lane, arg);
+            const double t2 = long_row(lv, lc, lp[2 * j + 1], lp[2 * j + 2], lane, arg);
+            if (lane == 0) emit(r.S + j, t1, t2);
+        }
+    }
 }
 
 // drv of stage 1 (j = 0), 2 and 3 (j = 1) or 4 (j = 2) of step s (calcODE.cpp:84-94, 278-302)
@@ -315,6 +360,7 @@ __device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity, long long
 // Bound: the latency of a stage (gather, row sum, st.async, mbarrier),
 // 1.6 us at N = 50.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread
 // its own sine): 2.9 us.
+template <bool MANY>
 __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResParams P, int cs)
 {
     extern __shared__ __align__(16) unsigned char fsm[];
@@ -341,7 +387,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
     }
     __syncthreads();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    const bool works = warp == 0 || warp == nw - 1 || 32 * warp < r.S || nw - 1 - warp < r.L;
+    const bool works = warp == 0 || warp == nw - 1 || 32 * warp < r.S || (MANY ? 32 : 1) * (nw - 1 - warp) < r.L;
     int to = cs;      // CTAs that this thread sends to (0: its wait gave up)
     uint32_t it = 0;  // stages done
     for (int s = 0; works && s < P.num_steps; s++) {
@@ -366,13 +412,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
                 const double t1 = short_row(m.ev + i, P.maxS, x);
                 send(i, fb_finish(P, m, stage, i, t1, drive_sum(i), drv));
             }
-            for (int j = nw - 1 - warp; j < r.L; j += nw) {
-                const int i = r.S + j;
-                const auto load = [&](int c) { return arg[c]; };
-                const double t1 = long_row(m.lv, m.lc, m.lp[2 * j], m.lp[2 * j + 1], lane, load);
-                const double t2 = long_row(m.lv, m.lc, m.lp[2 * j + 1], m.lp[2 * j + 2], lane, load);
-                if (lane == 0) send(i, fb_finish(P, m, stage, i, t1, t2, drv));
-            }
+            long_rows<MANY>(r, m.lv, m.lc, m.lp, warp, nw, lane, [&](int c) { return arg[c]; },
+                            [&](int i, double t1, double t2) { send(i, fb_finish(P, m, stage, i, t1, t2, drv)); });
             if (warp == nw - 1) {
                 if (stage == 1 && lane < 3) m.drv[3 * ((s + 1) & 1) + lane] = stage_drive(P, s + 1, lane);
                 __syncwarp();
@@ -404,6 +445,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResPar
 // 3.3 us at N = 100; one launch per stage before this took 8.2 us.
 constexpr int kGridThreads = 256;
 
+template <bool MANY>
 __global__ void __launch_bounds__(kGridThreads, 1) rk4_grid(const FbResParams P)
 {
     extern __shared__ __align__(16) unsigned char fsm[];
@@ -459,13 +501,8 @@ __global__ void __launch_bounds__(kGridThreads, 1) rk4_grid(const FbResParams P)
                 const double t1 = short_row(m.ev + i, P.maxS, x);
                 __stcg(out + i, fb_finish(P, m, stage, i, t1, t2, drv));
             }
-            for (int j = nw - 1 - warp; j < r.L; j += nw) {
-                const int i = r.S + j;
-                const auto load = [&](int c) { return __ldcg(arg + c); };
-                const double t1 = long_row(m.lv, m.lc, m.lp[2 * j], m.lp[2 * j + 1], lane, load);
-                const double t2 = long_row(m.lv, m.lc, m.lp[2 * j + 1], m.lp[2 * j + 2], lane, load);
-                if (lane == 0) __stcg(out + i, fb_finish(P, m, stage, i, t1, t2, drv));
-            }
+            long_rows<MANY>(r, m.lv, m.lc, m.lp, warp, nw, lane, [&](int c) { return __ldcg(arg + c); },
+                            [&](int i, double t1, double t2) { __stcg(out + i, fb_finish(P, m, stage, i, t1, t2, drv)); });
             if (stage == 1 && warp == nw - 1 && lane < 3) m.drv[3 * ((s + 1) & 1) + lane] = stage_drive(P, s + 1, lane);
             q ^= 1;
             ok = sync();
@@ -481,6 +518,7 @@ struct qjx_fb {
     fb::FbParams P{};
     // resident forms: cs CTAs of one cluster, or `grid` CTAs of a cooperative launch (neither: stage kernels)
     int cs = 0, grid = 0;
+    bool many = false;  // long rows in slices
     size_t smem = 0;
     fb::FbResParams R{};
     double *x0 = nullptr;   // x before the call, for a call in which a wait gives up
@@ -518,9 +556,23 @@ struct FbDeal {
     std::vector<fb::FbRows> rows;
     std::vector<int> perm, pos;  // entry -> row, row -> entry
     int maxS = 0, maxL = 0, maxN = 0;
+    bool many = false;  // a CTA has more long rows than warps: slices of 32
 };
 
-static void fb_deal(const FbSystem &y, int nc, FbDeal &d)
+static int fb_pad4(int k) { return (k + 3) & ~3; }
+
+// Nonzeros of Gs and Qs (each a multiple of four) that slice j of a CTA's long rows holds per row.
+static void fb_slice(const FbSystem &y, const FbDeal &d, const fb::FbRows &r, int j, int &g, int &q)
+{
+    g = q = 0;
+    for (int i = 32 * j; i < std::min(r.L, 32 * j + 32); i++) {
+        const int row = d.perm[r.base + r.S + i];
+        g = std::max(g, fb_pad4(y.gr[row + 1] - y.gr[row]));
+        q = std::max(q, fb_pad4(y.qr[row + 1] - y.qr[row]));
+    }
+}
+
+static void fb_deal(const FbSystem &y, int nc, int warps, FbDeal &d)
 {
     const int n = y.n;
     // a row's nonzeros; past kW (long) also when its drive has several
@@ -563,6 +615,20 @@ static void fb_deal(const FbSystem &y, int nc, FbDeal &d)
         d.rows.push_back(r);
         d.maxS = std::max(d.maxS, r.S);
         d.maxL = std::max(d.maxL, r.L);
+    }
+    // Where the line lies: a warp takes about 1.1 us per long row, one after the other, a slice about as long as
+    // one or two of them (2600 rows of 25 nonzeros in a cluster, us a stage: 11.8 by warps, 2.1 in slices, 2.9 before
+    // both as CSR rows between cluster barriers; 40,000 of 40 in the grid form: 42.7, 7.6, stage kernels 16.9).
+    d.many = d.maxL > warps;
+    for (fb::FbRows &r : d.rows) {
+        if (d.many) {
+            r.ln = 0;
+            for (int j = 0; 32 * j < r.L; j++) {
+                int g, q;
+                fb_slice(y, d, r, j, g, q);
+                r.ln += 32 * (g + q);
+            }
+        }
         d.maxN = std::max(d.maxN, r.ln);
     }
     d.maxS = std::max(32, (d.maxS + 31) & ~31);
@@ -639,19 +705,30 @@ static bool fb_upload_deal(qjx_fb *h, const FbSystem &y, const FbDeal &d, bool c
                 qc[r.base + i] = d.pos[y.qc[y.qr[row]]];
             }
         }
-        // the nonzeros of long row i from `at` on
-        auto put = [&](int i, const int *rp, const int *ci, const double *val, int at) {
+        // the nonzeros of long row i from `at` on, `step` apart
+        auto put = [&](int i, const int *rp, const int *ci, const double *val, int at, int step) {
             const int row = d.perm[r.base + r.S + i];
-            for (int l = rp[row]; l < rp[row + 1]; l++, at++) {
+            for (int l = rp[row]; l < rp[row + 1]; l++, at += step) {
                 v[at] = val[l];
                 col[at] = d.pos[ci[l]];
             }
             return at;
         };
         int at = 0;
-        for (int j = 0; j < r.L; j++) {
-            start[2 * j + 1] = put(j, y.gr, y.gc, y.gv, at);
-            start[2 * j + 2] = at = put(j, y.qr, y.qc, y.qv, start[2 * j + 1]);
+        for (int j = 0; d.many && 32 * j < r.L; j++) {
+            int g, q;
+            fb_slice(y, d, r, j, g, q);
+            start[2 * j + 1] = at + 32 * g;
+            start[2 * j + 2] = at + 32 * (g + q);
+            for (int i = 32 * j; i < std::min(r.L, 32 * j + 32); i++) {
+                put(i, y.gr, y.gc, y.gv, at + i - 32 * j, 32);
+                put(i, y.qr, y.qc, y.qv, start[2 * j + 1] + i - 32 * j, 32);
+            }
+            at = start[2 * j + 2];
+        }
+        for (int j = 0; !d.many && j < r.L; j++) {
+            start[2 * j + 1] = put(j, y.gr, y.gc, y.gv, at, 1);
+            start[2 * j + 2] = at = put(j, y.qr, y.qc, y.qv, start[2 * j + 1], 1);
         }
     }
     if (cudaMemcpy(a.dev, at0, filled, cudaMemcpyHostToDevice) != cudaSuccess) return false;
@@ -683,6 +760,7 @@ static bool fb_upload_deal(qjx_fb *h, const FbSystem &y, const FbDeal &d, bool c
     R.T = h->T;
     R.h = h->T / double(h->num_steps);
     R.num_steps = h->num_steps;
+    h->many = d.many;
     return true;
 }
 
@@ -708,12 +786,13 @@ static bool fb_setup_cluster(qjx_fb *h, const FbSystem &y)
     while (cs < fb::kMaxCluster && (y.n + cs - 1) / cs > fb::kClusterRows) cs *= 2;
     for (; cs <= fb::kMaxCluster; cs *= 2) {
         FbDeal d;
-        fb_deal(y, cs, d);
+        fb_deal(y, cs, fb::kClusterThreads / 32, d);
+        auto *const kernel = d.many ? fb::rk4_cluster<true> : fb::rk4_cluster<false>;
         const size_t bytes = sizeof(double) * 2 * ((size_t)y.n + 1) + fb::fb_rows_bytes(d.maxS, d.maxL, d.maxN) +
                              sizeof(unsigned short) * fb::kW * d.maxS + 16;
         if (bytes + 1024 > (size_t)optin) continue;
-        if (!fb_allow_smem(fb::rk4_cluster, optin) ||
-            (cs > 8 && cudaFuncSetAttribute(fb::rk4_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+        if (!fb_allow_smem(kernel, optin) ||
+            (cs > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
             cudaGetLastError();
             continue;
         }
@@ -729,7 +808,7 @@ static bool fb_setup_cluster(qjx_fb *h, const FbSystem &y)
         lc.attrs = at;
         lc.numAttrs = 1;
         int nclusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&nclusters, fb::rk4_cluster, &lc) != cudaSuccess || nclusters < 1) {
+        if (cudaOccupancyMaxActiveClusters(&nclusters, kernel, &lc) != cudaSuccess || nclusters < 1) {
             cudaGetLastError();
             continue;
         }
@@ -750,11 +829,12 @@ static bool fb_setup_grid(qjx_fb *h, const FbSystem &y)
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
     if (!coop || sms < 1) return false;
     FbDeal d;
-    fb_deal(y, sms, d);
+    fb_deal(y, sms, fb::kGridThreads / 32, d);
+    auto *const kernel = d.many ? fb::rk4_grid<true> : fb::rk4_grid<false>;
     const size_t bytes = fb::fb_rows_bytes(d.maxS, d.maxL, d.maxN) + sizeof(int) * fb::kW * d.maxS + 16;
     if (bytes + 1024 > (size_t)optin ||
-        !fb_allow_smem(fb::rk4_grid, optin) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fb::rk4_grid, fb::kGridThreads, bytes) != cudaSuccess || per < 1) {
+        !fb_allow_smem(kernel, optin) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, fb::kGridThreads, bytes) != cudaSuccess || per < 1) {
         cudaGetLastError();
         return false;
     }
@@ -868,8 +948,9 @@ extern "C" qjx_status qjx_fb_run(qjx_fb *h, int period0, int n_periods)
             C.polls = polls ? std::atoll(polls) : fb::kFbWait;
             C.period = p;
             if (!h->cs) cudaMemsetAsync(C.arrived, 0, sizeof(unsigned), h->stream);
-            const cudaError_t e = h->cs ? cudaLaunchKernelEx(&lc, fb::rk4_cluster, C, h->cs)
-                                        : cudaLaunchKernelEx(&lc, fb::rk4_grid, C);
+            const cudaError_t e =
+                h->cs ? cudaLaunchKernelEx(&lc, h->many ? fb::rk4_cluster<true> : fb::rk4_cluster<false>, C, h->cs)
+                      : cudaLaunchKernelEx(&lc, h->many ? fb::rk4_grid<true> : fb::rk4_grid<false>, C);
             if (e == cudaErrorCooperativeLaunchTooLarge && !h->cs) {
                 // not every CTA can be resident (another context holds SMs): the stage kernels
                 cudaGetLastError();
