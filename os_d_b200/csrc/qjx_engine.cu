@@ -53,6 +53,9 @@ struct NvtxRange {
 using namespace qjx;
 
 constexpr size_t kPackBytes = 16 << 20;  // states packed at a time by qjx_get_states
+// qjx_get_states: both slots in one copy up to this many bytes (us a call there / packed on the device: 0.8 KB 34 / 43,
+// 33 KB 44 / 49, 49 KB 53 / 51, 133 KB 78 / 61)
+constexpr size_t kSmallStates = 40 << 10;
 
 struct qjx_engine {
     qjx_config cfg{};
@@ -1305,7 +1308,14 @@ extern "C" qjx_status qjx_get_states(qjx_engine *h, double *psi, double *t, doub
     const Params &P = h->P;
     std::vector<TrajState> st(P.n);
     CK(cudaMemcpy(st.data(), P.st, P.n * sizeof(TrajState), cudaMemcpyDeviceToHost));
-    if (psi) {
+    const size_t both = (size_t)2 * P.n * P.MD;  // components of two slots
+    if (psi && both * sizeof(double2) <= kSmallStates) {
+        // few: both slots in one copy, the current rows picked here
+        std::vector<double2> all(both);
+        CK(cudaMemcpy(all.data(), P.psi, both * sizeof(double2), cudaMemcpyDeviceToHost));
+        for (int i = 0; i < P.n; i++)
+            memcpy(psi + (size_t)2 * i * P.d, all.data() + ((size_t)st[i].cur * P.n + i) * P.MD, (size_t)P.d * sizeof(double2));
+    } else if (psi) {
         // packed on the device, a chunk at a time, and copied straight into the caller's rows (both slots
         // through a host vector before: 38 ms for 10^4 trajectories of d = 201)
         const size_t row = (size_t)P.d * sizeof(double2);
