@@ -248,6 +248,12 @@ static T *upload(qjx_engine *h, const std::vector<T> &v)
     return p;
 }
 
+// States that qjx_get_states packs at a time.
+static int pack_rows(const Params &P)
+{
+    return (int)std::min<size_t>(P.n, std::max<size_t>(1, kPackBytes / ((size_t)P.d * sizeof(double2))));
+}
+
 // ---------------------------------------------------------------- tile shapes
 // Whether a plain-form shape (columns per sub-tile, k rows per slab) is valid for padded rows MD: at
 // most 8 row blocks per warp of a 512-thread CTA, and columns and two slabs within kTileSmem bytes.
@@ -1018,6 +1024,10 @@ extern "C" qjx_status qjx_create_slots(const qjx_config *cfg, int n_slots, int d
         *out = nullptr;
         return QJX_ERR_OOM;
     }
+    // the buffer that packs states for the host, here so that a pool's memory is known when it is admitted
+    // (without it they are read back row by row)
+    h->d_pack = (double2 *)dalloc(h, pack_rows(h->P) * (size_t)h->P.d * sizeof(double2));
+    if (!h->d_pack) cudaGetLastError();
     cudaMemset(h->d_active, 0, (size_t)h->P.n);
     h->P.active = h->d_active;
     h->states_set = true;
@@ -1319,7 +1329,7 @@ extern "C" qjx_status qjx_get_states(qjx_engine *h, double *psi, double *t, doub
         // packed on the device, a chunk at a time, and copied straight into the caller's rows (both slots
         // through a host vector before: 38 ms for 10^4 trajectories of d = 201)
         const size_t row = (size_t)P.d * sizeof(double2);
-        const int chunk = (int)std::min<size_t>(P.n, std::max<size_t>(1, kPackBytes / row));
+        const int chunk = pack_rows(P);
         if (!h->d_pack) h->d_pack = (double2 *)dalloc(h, chunk * row);
         if (!h->d_pack) {  // no memory for it: a row at a time
             cudaGetLastError();

@@ -63,7 +63,8 @@ def size_class(d, n_traj):
 def pool_footprint(n_slots, d_cap, n_cap, deep, rec_cap=16, num_branches=2):
     """Device bytes of a serving engine of n_slots slots of (d_cap, n_cap) with one dump, no random
     observables and jump buffers of rec_cap records: matrices, two state slots, per-trajectory
-    records and queues (create_engine's allocations; checked against qjx_engine_bytes)."""
+    records, queues and the buffer that packs states for the host, 16 MB at most (the allocations of
+    create_engine and qjx_create_slots; checked against qjx_engine_bytes)."""
     md, kp = 8 * ((d_cap + 7) // 8), (d_cap + 1) & ~1
     ge = num_branches * deep + 2
     n, G = n_slots * n_cap, n_slots * ge
@@ -71,7 +72,8 @@ def pool_footprint(n_slots, d_cap, n_cap, deep, rec_cap=16, num_branches=2):
     psi = 2 * n * md * 16
     per_traj = 144 + 8 + 6 * 8 + 16 + 8 * d_cap + rec_cap * 28 + 1
     rings = G * (1 << (n_cap - 1).bit_length()) * 4  # a queue per matrix, a power of two long
-    return mats + psi + n * per_traj + rings + 48 * G + (1 << 20)
+    pack = min(n, max(1, (16 << 20) // (16 * d_cap))) * 16 * d_cap
+    return mats + psi + n * per_traj + rings + pack + 48 * G + (1 << 20)
 
 
 class _Pool:
