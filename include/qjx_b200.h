@@ -220,8 +220,9 @@ qjx_status qjx_get_stats(qjx_engine *h, qjx_stats *stats);
 /* The project's tile autotuner (no counterpart in the reference, which has no tiles): times the
  * candidate tile shapes of cfg->precision (plain: sub-tile columns x slab rows; split: ring depth x
  * fewest rows per tile) on scratch engines of cfg with the given operators (cfg->n_traj
- * trajectories from |0>, one untimed period, then n_periods timed periods of device time) and
- * returns the fastest in *best.  cand / us (capacity *n_cand; NULL to skip) receive every
+ * trajectories from |0>, one untimed period, then n_periods timed periods of device time, the plain form in
+ * sub-tiles to the last trajectory) and returns the fastest in *best.  With too few trajectories to fill
+ * the rule's sub-tiles on every SM only shapes of that width are timed.  cand / us (capacity *n_cand; NULL to skip) receive every
  * candidate and its device microseconds per trajectory-period; *n_cand the count.  The winner is
  * stored under (precision, d) in the tile cache file: $QJX_TILE_CACHE, else
  * $HOME/.cache/qjx_b200/tiles.txt; engines created later with all-zero cfg->tiles use it. */

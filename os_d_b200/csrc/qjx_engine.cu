@@ -280,6 +280,24 @@ static bool tiles_fit(int MD, size_t budget, int nt, int nc, int *kb)
     return step_smem_bytes(MD, nc, *kb) <= budget;
 }
 
+// Dynamic shared memory of a CTA of nt threads of the plain kernel: all that the device gives, or half of an SM's (256).
+static size_t flow_budget(int device, int nt)
+{
+    int optin = 0, per_sm = 0, reserved = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+    cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
+    return (size_t)std::max(0, (nt == 512 ? optin : per_sm / 2 - reserved) - (int)step_static_smem(nt));
+}
+
+// The rule's shape for padded rows MD in an engine whose largest ensemble has MDmax: two CTAs of 256 threads per SM
+// take at least 16 columns and slabs of 6 k rows.
+static bool rule_tiles(int MD, int MDmax, size_t budget, int nt, qjx_tiles *t)
+{
+    return pick_step_tiles(MD, budget, nt, std::min(max_columns(MD, nt), max_columns(MDmax, nt)), &t->nc, &t->kb) &&
+           (nt == 512 || (t->nc >= 16 && t->kb >= 6));
+}
+
 // The autotuner's cache: text lines "precision d nc kb stages rows us" (later lines win), in
 // $QJX_TILE_CACHE or $HOME/.cache/qjx_b200/tiles.txt.
 static std::string tile_cache_path()
@@ -404,18 +422,12 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     Params &P = h->P;
     std::vector<int> e_nc(E), e_kb(E);
     {  // plain kernel tiling of every ensemble within the shared memory
-        int optin = 0, per_sm = 0, reserved = 0;
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device);
-        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c.device);
-        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, c.device);
         // two CTAs of 256 threads per SM when every ensemble's sub-tiles fit half of the SM's shared
         // memory (16 columns and slabs of at least 6 k rows, d <= 232, or explicit or autotuned shapes
         // of at most 16 columns), so that one CTA's scan, staging and epilogue overlap the other's
         // products; else one CTA of 512
-        const size_t whole = (size_t)std::max(0, optin - (int)step_static_smem(512));
         for (const int nt : {256, 512}) {
-            const size_t budget =
-                nt == 512 ? whole : (size_t)std::max(0, per_sm / 2 - reserved - (int)step_static_smem(256));
+            const size_t budget = flow_budget(c.device, nt);
             size_t smem = 0;
             bool fits = nt == 512 || MD <= 256;
             for (int e = 0; e < E && fits; e++) {
@@ -428,8 +440,7 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
                 } else if (tile_cache_get(0, ens[e].d, &ct) && tiles_valid(MDe, ct.nc, ct.kb)) {
                     fits = ct.nc <= max_columns(MD, nt) && tiles_fit(MDe, budget, nt, ct.nc, &ct.kb);  // the autotuner's choice for this dimension
                 } else {
-                    fits = pick_step_tiles(MDe, budget, nt, std::min(max_columns(MDe, nt), max_columns(MD, nt)), &ct.nc, &ct.kb) &&
-                           (nt == 512 || (ct.nc >= 16 && ct.kb >= 6));
+                    fits = rule_tiles(MDe, MD, budget, nt, &ct);
                 }
                 e_nc[e] = ct.nc;
                 e_kb[e] = ct.kb;
@@ -1742,8 +1753,20 @@ extern "C" qjx_status qjx_autotune(const qjx_config *cfg, const double *U, const
         for (int st : {2, 3, 4, 6, 8})
             for (int rows : {8, 32, 64, 128}) list.push_back(qjx_tiles{0, 0, st, rows});
     } else {
+        // Widths are compared only with trajectories enough that every CTA's share fills the rule's width: with
+        // fewer, all widths run the same claims (2048 trajectories of d = 201: 8 columns by 2 % of noise, and
+        // an engine of 10^4 that then took 8 for 16 ran 38,700 trajectory-periods/s, not 46,000)
+        if (cudaSetDevice(cfg->device) != cudaSuccess) return QJX_ERR_CUDA;
+        const int MD = 8 * ((d + 7) / 8);
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device);
+        qjx_tiles rule{};
+        const bool two = MD <= 256 && rule_tiles(MD, MD, flow_budget(cfg->device, 256), 256, &rule);
+        if (!two && !rule_tiles(MD, MD, flow_budget(cfg->device, 512), 512, &rule)) return QJX_ERR_UNSUPPORTED;
+        const long long share = 8 * ((n + 8ll * sms * (two ? 2 : 1) - 1) / (8ll * sms * (two ? 2 : 1)));
         for (int nc : {32, 16, 8})
-            for (int kb : {16, 12, 8, 4}) list.push_back(qjx_tiles{nc, kb, 0, 0});
+            for (int kb : {16, 12, 8, 4})
+                if (nc == rule.nc || share >= rule.nc) list.push_back(qjx_tiles{nc, kb, 0, 0});
     }
     std::vector<double> psi((size_t)n * d * 2, 0.0);
     for (int i = 0; i < n; i++) psi[(size_t)i * d * 2] = 1.0;  // |0>
@@ -1758,6 +1781,7 @@ extern "C" qjx_status qjx_autotune(const qjx_config *cfg, const double *U, const
         c.max_dumps = 1;
         qjx_engine *h = nullptr;
         if (create_engine(&c, U, L, g, HE, nullptr, 2, &h) != QJX_OK) continue;  // the shape does not fit
+        h->solo_max = 0;  // sub-tiles to the last trajectory: a trajectory of its own CTA has no shape
         double t_us = -1.0;
         if (qjx_set_states(h, psi.data()) == QJX_OK && qjx_init_thresholds(h) == QJX_OK &&
             qjx_run_periods(h, 1, 0, nullptr, 0, 0) == QJX_OK) {
