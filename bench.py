@@ -225,8 +225,8 @@ def fbasis_bench(args, local):
                        f"Gs nnz {Gs.nnz}, Qs nnz {Qs.nnz}",
            "metric": "periods/s", "value": 1e3 / per, "ms_per_period": per, "us_per_rk4_step": 1e3 * per / steps,
            "kernel": "fb::rk4_cluster" if cs else "fb::rk4_grid", "cluster_size": cs,
-           "roofline": {"bound": "shared memory / cluster barrier latency (operands resident in the cluster's shared "
-                                 "memory, no HBM traffic after the first load)",
+           "roofline": {"bound": "latency of a stage: gather, row sum, st.async to every CTA, mbarrier (operands resident "
+                                 "in the cluster's shared memory, no HBM traffic after the first load)",
                         "achieved": achieved, "unit": "GB/s", "peak": smem_peak,
                         "peak_source": "shared-memory bandwidth of the cluster's SMs, 128 B/clk at 1965 MHz",
                         "frac": achieved / smem_peak, "algorithmic_bytes_per_rk4_step": step_bytes},
@@ -833,7 +833,7 @@ def run_ours(args):
 
     # roofline of the dominant kernel (flow_kernel, grouped FP64 complex GEMM + fused epilogue)
     matvecs = st1["matvecs"] - st0["matvecs"]
-    launches_step = st1["launches"] - st0["launches"]
+    launches_step = st1["launches"] - st0["launches"] - args.steps  # time slices (each step's run call schedules once)
     kern_ms = st1["step_kernel_ms"] - st0["step_kernel_ms"]
     flops = 8.0 * d * d * matvecs
     achieved = flops / (kern_ms * 1e-3) / 1e12

@@ -297,9 +297,9 @@ qjx_status qjx_checkpoint_size(qjx_engine *h, size_t *bytes);
 qjx_status qjx_checkpoint_save(qjx_engine *h, void *buf, size_t bytes);
 qjx_status qjx_checkpoint_load(qjx_engine *h, const void *buf, size_t bytes);
 /* Per-CTA trace of the trajectory kernel (profiling aid, off by default): enabling clears
- * and starts accumulating, per persistent CTA, clock64 cycles {total, setup, (reserved),
- * MMA loop, epilogue} and counts {sub-tiles, 8-column blocks, columns}.  qjx_get_trace
- * copies [n_ctas][n_fields] int64 (out may be NULL to query the shape). */
+ * and starts accumulating, per persistent CTA, clock64 cycles {total, setup, claim (plain form),
+ * product, epilogue} and counts {sub-tiles or tiles, 8-column blocks (split form: cycles of reading the
+ * accumulators back), columns}.  qjx_get_trace copies [n_ctas][n_fields] int64 (out may be NULL to query the shape). */
 qjx_status qjx_set_trace(qjx_engine *h, int enable);
 qjx_status qjx_get_trace(qjx_engine *h, int64_t *out, int *n_ctas, int *n_fields);
 /* Measured FP64 throughput of the device in TFLOP/s (2 flops per FMA): an FFMA-chain

@@ -18,13 +18,15 @@ constexpr int kThreads = 512;          // 16 warps (split-form kernel)
 constexpr int kKB = 16;                // most k rows per propagator slab
 constexpr int kMaxDt = 64;             // split-level steps [nb][deep] a CTA keeps in shared memory
 constexpr int kColPad = 2;             // components between staged columns past the padded rows
-constexpr int kMaxGroups = 256;        // distinct matrices in one engine
 constexpr int kMaxMD = 1024;           // d <= 1024 (plain form; the split form takes d <= 256)
 constexpr double kSplitNormSlack = 1e-4;  // split precision: tolerated norm excess over 1
 constexpr int kMaxTile = 128;             // split precision: most trajectories per tile (MMA M)
 constexpr int kMaxSplitStages = 8;        // split precision: deepest operand ring
-// plain kernel: a launch hands the device back after kSliceNs (engines of other streams get
-// their turn; the host launches again), and a CTA that finds no work for kIdleNs leaves
+// a CTA of the trajectory kernels leaves after kSliceNs, so that a launch hands the device back (engines of
+// other streams get their turn; the host launches again), or when it finds no work for kIdleNs.  A launch of
+// more one-trajectory CTAs than are resident lasts a slice per wave, because the later CTAs begin theirs
+// when the first leave (10^5 trajectories of d = 4: 13 ms; launching only the resident ones costs 11 to 20 % at
+// d <= 31, where every slice then ends with CTAs waiting for the last)
 constexpr unsigned long long kSliceNs = 4000000, kIdleNs = 200000;
 constexpr unsigned kFree = 0xffffffffu;  // an empty queue entry
 constexpr int kSoloThreads = 256;      // most threads (rows) per CTA of the one-trajectory kernel
@@ -239,8 +241,8 @@ struct LpnParams {
     double spec_div;                                                  // MBL: spec = robs slot 0 / W
     const int *words;                                                 // MBL: [d] basis words
 };
-// trace fields: total, setup (bucket scan + gather), operand wait, MMA loop, epilogue,
-// sub-tiles, 8-column blocks, columns
+// trace fields: total, setup (claim and staging), claim (plain form), product, epilogue, sub-tiles or tiles,
+// 8-column blocks (split form: cycles of reading the accumulators back), columns
 constexpr int kTraceFields = 8;
 
 // ---------------------------------------------------------------- Philox4x32-10

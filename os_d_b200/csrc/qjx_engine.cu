@@ -369,8 +369,7 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     const long long Gl = (long long)E * Ge;
     if (dmax > kMaxMD || Gl > (1 << 24) || ntot > (1 << 30)) return QJX_ERR_UNSUPPORTED;
     if (c.precision != 0 && c.precision != 1) return QJX_ERR_INVALID_ARG;
-    // the split kernel's N = MDs <= 256 and its shared-memory bucket tables hold one ensemble of
-    // at most kMaxGroups matrices
+    // the split kernel's N = MDs <= 256 (two accumulators of MDs columns in tensor memory)
     if (c.precision == 1 && dmax > 256) return QJX_ERR_UNSUPPORTED;
     const int G = (int)Gl;
     const int n = (int)ntot;
@@ -535,7 +534,9 @@ static qjx_status create_engine(const qjx_config *cfg, const std::vector<EnsDesc
     // one dimension (ms a period there / one trajectory per CTA throughout / sub-tiles to the last 100): d = 31:
     // 10^4 (10.2 / 10.2 / 11.1), d = 51: 3000 (14.5 / 18.1 / 16.3), d = 101: 500 to 1300 (21.3 / 33.9 /
     // 24.3), d = 201: 350 to 600 (68.5 / 78.3 / 74.7), d = 401: all of 300 (236 / 236 / 269); d^2 is the
-    // trajectories' mean in a batch.
+    // trajectories' mean in a batch.  Beyond that the constant decides; one trajectory per cluster throughout / to the
+    // last 100 / sub-tiles throughout: d = 601, 240: 275 / 259 / 344, d = 801, 240: 505 / 522 / 811, d = 1001, 250: 839 /
+    // 1435 / 2288, d = 501, 80: 82 / 82 / 292.
     double d2 = 0.0;
     for (const EnsDesc &x : ens) d2 += (double)x.n * x.d * x.d;
     h->solo_max = 250 + (int)(6.5e6 / (d2 / n));

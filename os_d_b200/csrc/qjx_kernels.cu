@@ -15,8 +15,8 @@
 // and no plan:
 //   * a sub-tile is one matrix x 8, 16 or 32 trajectory columns, full height (all d rows), so the
 //     column norm needed by the jump test stays inside the CTA;
-//   * the gathered state columns and the propagator K-slabs are copied to shared memory with cp.async
-//     through a ring of stages, so the tensor pipe is fed while the next slabs stream from L2;
+//   * the gathered state columns and the propagator K-slabs are copied to shared memory with cp.async,
+//     two slabs in turn, so the tensor pipe is fed while the next slab streams from L2;
 //   * the epilogue is the whole trajectory state machine: norm test, descend / accept,
 //     jump record, renormalisation, channel choice, threshold redraw, time bookkeeping,
 //     period and dump accounting and the observables.
@@ -196,7 +196,7 @@ __device__ __forceinline__ double adr_of(double2 v, double inv)
 
 // Observables of the state held in `col` (calc_chars_std[_start], core.cpp:665-725) and
 // the normalised state psi / sqrt(norm) written to the spare slot for the energy and
-// random-observable micro-steps.  Warp-cooperative; every lane computes the sequential
+// random-observable matvecs.  Warp-cooperative; every lane computes the sequential
 // sums identically.
 __device__ void obs_prep(const Params &P, const TrajState &s, int tr, const Ens &sys, const Slots &slots, const double2 *col, int lane,
                          int dump, int is_start)
@@ -1391,7 +1391,7 @@ __global__ void schedule_kernel(const Params P, int mode)
 }
 
 // Host-initiated observables of the current states (one warp per trajectory); the energy
-// and random-observable matvecs follow as micro-steps.
+// and random-observable matvecs follow from the queues.
 __global__ void observe_kernel(const Params P, int dump, int is_start)
 {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1740,7 +1740,9 @@ static cudaError_t launch_solo_t(const Params &P, int workers, cudaStream_t st)
 }
 
 // Eight k pairs in flight per thread where every CTA of the launch is resident with the registers
-// that takes (a lone CTA's matvec at d = 201: 110 cycles per k pair against 137), else four.
+// that takes (a lone CTA's matvec at d = 201: 110 cycles per k pair against 137), else four.  (Four with two
+// CTAs per SM leave 128 registers: with C > 1 the compiler spills about 24 of them, 400 bytes of stores and 456 of
+// loads per thread, with C = 1 two.)
 template <int C>
 static cudaError_t launch_solo_c(const Params &P, int workers, cudaStream_t st)
 {
@@ -1768,8 +1770,7 @@ int pick_layout(int d, int *rows_per_block)
 }
 
 // Shared memory of the plain kernel: nc staged columns of MD + kColPad components (columns 32
-// bytes apart modulo the banks: conflict-free B operand reads) and two slabs of kb k rows (as
-// a ring of four half slabs where kb is a multiple of 4).
+// bytes apart modulo the banks: conflict-free B operand reads) and two slabs of kb k rows.
 size_t step_smem_bytes(int MD, int nc, int kb)
 {
     return (size_t)(nc * (MD + kColPad) + 2 * kb * MD) * sizeof(double2);

@@ -13,7 +13,7 @@
 // One CTA per pair.  The pair's work is a handful of d x d complex matvecs (characteristics)
 // plus one per bisection step of a renormalisation, thread per row, reading the FP64 matrices
 // in the engine's layout mats[g][k / 2][row][k % 2] (coalesced across the CTA's threads, L2
-// resident across CTAs); next to the period's micro-steps this is a small cost.
+// resident across CTAs); next to the period's matvecs this is a small cost.
 //
 // Arithmetic: every operation is the one the CPU oracle (lpn_oracle.c) performs: the canonical
 // 32-lane sums of warp 0, k-ascending fma matvecs, and lpn_exp10 / lpn_log written out below

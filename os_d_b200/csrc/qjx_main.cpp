@@ -399,7 +399,7 @@ void run_lpn_mult(qjx_engine *h, const RunParam &rp, const ConfigParam &cp, cons
 
     qjx_stats st{};
     qjx_get_stats(h, &st);
-    std::cout << "micro-steps: " << st.micro_steps << ", matvecs: " << st.matvecs
+    std::cout << "sub-tiles: " << st.micro_steps << ", matvecs: " << st.matvecs
               << ", device time (ms): " << st.kernel_ms << std::endl;
 }
 
@@ -967,7 +967,7 @@ int main(int argc, char **argv)
 
         qjx_stats st{};
         qjx_get_stats(h, &st);
-        std::cout << "micro-steps: " << st.micro_steps << ", matvecs: " << st.matvecs
+        std::cout << "sub-tiles: " << st.micro_steps << ", matvecs: " << st.matvecs
                   << ", device time (ms): " << st.kernel_ms << std::endl;
         qjx_destroy(h);
     } catch (const std::exception &e) {

@@ -327,8 +327,8 @@ class Engine:
         self._chk(N.lib().qjx_set_trace(self.h, int(enable)), "qjx_set_trace")
 
     def trace(self):
-        """Per-CTA accumulated trace: columns total, setup, reserved, loop, epilogue cycles,
-        sub-tiles, 8-column blocks, columns."""
+        """Per-CTA accumulated trace: columns total, setup, claim, product, epilogue cycles, sub-tiles (split
+        form: tiles), 8-column blocks, columns."""
         nc, nf = C.c_int(), C.c_int()
         self._chk(N.lib().qjx_get_trace(self.h, None, C.byref(nc), C.byref(nf)), "qjx_get_trace")
         out = np.zeros((nc.value, nf.value), np.int64)
