@@ -391,7 +391,7 @@ class FBasis:
         N.check(N.lib().qjx_fb_run(self.h, period0, n_periods), what="qjx_fb_run")
 
     def cluster_size(self):
-        """CTAs of the cluster-resident RK4 path (0: per-stage kernels)."""
+        """CTAs of the cluster-resident RK4 path (0: grid-wide or per-stage kernels)."""
         cs = C.c_int()
         N.check(N.lib().qjx_fb_info(self.h, C.byref(cs)), what="qjx_fb_info")
         return cs.value
