@@ -358,7 +358,7 @@ __device__ __forceinline__ bool fb_wait(uint32_t bar, uint32_t parity, long long
 // meanwhile.  A thread whose wait gives up runs on to the end without waiting, sending or arriving (its
 // mbarriers may not take more than a stage brings), so every other wait ends too.
 // Bound: the latency of a stage (gather, row sum, st.async, mbarrier),
-// 1.6 us at N = 50.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread
+// 1.5 us at N = 50.  Before (cluster barriers, thread-per-row CSR with a 32-lane pass, every thread
 // its own sine): 2.9 us.
 template <bool MANY>
 __global__ void __launch_bounds__(kClusterThreads, 1) rk4_cluster(const FbResParams P, int cs)
